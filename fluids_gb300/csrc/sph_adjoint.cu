@@ -355,7 +355,7 @@ int adj_step(sph_adj* a, const float4* x, const float4* v, const float4* u, floa
     lb.aux = aux;
     lb.scenes = ctx->b.scenes;
     lb.flags = a->flags;
-    sph::launch_lists_density_remap(s, c, lb, ms, bs);
+    sph::launch_lists_density_remap(s, c, lb, ms, bs, ctx->num_sms);
     Bufs fb{};
     fb.pos_s = const_cast<float4*>(x);
     fb.vel_s = const_cast<float4*>(v);

@@ -513,7 +513,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
     if (x->p.method == SPH_WCSPH) {
         const bool lists = x->p.neighbor_mode == SPH_NEIGH_LIST;
         if (lists) {
-            sph::launch_lists_density(s, c, b, bs);
+            sph::launch_lists_density(s, c, b, bs, x->num_sms);
             mark(x, "k_lists_density");
         } else {
             sph::launch_wc_density(s, c, b, false, bs);
@@ -556,7 +556,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
     } else {
         if (!c.compat && !c.batched) {
             /* the lists and the initial density in one pass */
-            sph::launch_lists_density_pci(s, c, b, bs);
+            sph::launch_lists_density_pci(s, c, b, bs, x->num_sms);
             mark(x, "k_lists_density");
         } else {
             sph::launch_neigh_lists(s, c, b.pos_s, b.tab, b.bpos_s, b.btab, b.nlist, b.nlen, b.sblist, b.sblen, bs,

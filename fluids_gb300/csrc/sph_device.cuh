@@ -571,6 +571,10 @@ __device__ __forceinline__ float signf(float x) {
     return x;
 }
 __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf(x * x + y * y + z * z); }
+/* aux record of a particle: (p/rho^2, 1/rho, rho, p) */
+__device__ __forceinline__ float4 make_aux(float d, float p) {
+    return make_float4(p / (d * d), 1.0f / d, d, p);
+}
 
 
 }  // namespace sph

@@ -133,10 +133,15 @@ void launch_wc_forces(cudaStream_t s, const Const& c, const Bufs& b, bool lists,
 void launch_wc_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_aux(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 /* PHYSICS PCISPH: the neighbour lists and compute_initial_density in one pass */
-void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs);
-void launch_lists_density(cudaStream_t s, const Const& c, const Bufs& b, int bs);
+void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms);
+void launch_lists_density(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms);
 /* the list builder writing rows, entries and densities in id order (remap = sorted -> id) */
-void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap, int bs);
+void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap, int bs,
+                                int num_sms);
+
+/* sph_lists.cu: the same passes for small scenes, several lanes per particle; false (nothing
+ * launched) for contexts they do not take */
+bool launch_lists_split(cudaStream_t s, const Const& c, const Bufs& b, bool pci, const int32_t* remap, int num_sms);
 
 /* sph_pcisph.cu */
 void launch_pci_init_density(cudaStream_t s, const Const& c, const Bufs& b, int bs);

@@ -22,10 +22,6 @@
 
 namespace sph {
 
-__device__ __forceinline__ float4 make_aux(float d, float p) {
-    return make_float4(p / (d * d), 1.0f / d, d, p);
-}
-
 /* W_DEFAULT(r_norm, support_radius) of compute_density_pressure (wcsph.cl:61-62,70-71):
  * PHYSICS (h^2 - r^2)^3; COMPAT the kernel text's (h^2 - r)^3, or with the Monaghan kernels
  * w_monaghan(r, h). */
@@ -465,21 +461,25 @@ static void lists_density_launch(cudaStream_t s, const Const& c, const Bufs& b, 
                                                                 next, nullptr, nullptr, b.bnear, b.noff, b.prho);
 }
 
-void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
+void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
     if (c.n <= 0) return;
+    if (launch_lists_split(s, c, b, true, nullptr, num_sms)) return;
     k_lists_density<false, false, false, true><<<nblk(c.n, bs), bs, 0, s>>>(
         c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
         b.aux, b.scenes, b.tiles, nullptr, nullptr, nullptr, b.bnear, b.noff, b.prho);
 }
-void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap, int bs) {
+void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap, int bs,
+                                int num_sms) {
     if (c.n <= 0) return;
+    if (launch_lists_split(s, c, b, false, remap, num_sms)) return;
     k_lists_density<false, false, true><<<nblk(c.n, bs), bs, 0, s>>>(
         c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
         b.aux, b.scenes, b.tiles, nullptr, remap, b.flags);
 }
 
-void launch_lists_density(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
+void launch_lists_density(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
     if (c.n <= 0) return;
+    if (launch_lists_split(s, c, b, false, nullptr, num_sms)) return;
     if (c.compat) lists_density_launch<true, false>(s, c, b, bs);
     else if (c.batched) lists_density_launch<false, true>(s, c, b, bs);
     else lists_density_launch<false, false>(s, c, b, bs);
