@@ -372,7 +372,7 @@ int adj_step(sph_adj* a, const float4* x, const float4* v, const float4* u, floa
     fb.ids = a->ids;
     fb.scenes = ctx->b.scenes;
     fb.flags = a->flags;
-    sph::launch_wc_forces(s, c, fb, true, true, true, bs);
+    sph::launch_wc_forces(s, c, fb, true, true, true, bs, ctx->num_sms);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return afail(a, SPH_E_CUDA, std::string("adjoint forward launch: ") + cudaGetErrorString(e));
     return SPH_OK;

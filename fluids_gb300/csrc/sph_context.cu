@@ -391,11 +391,11 @@ int run_stage_impl(sph_ctx* x, int stage) {
         break;
     case SPH_S_NORMALS:
         sph::launch_aux(s, c, b, bs);   /* the density field may have been set from outside */
-        sph::launch_normals(s, c, b, uses_lists(x), bs);
+        sph::launch_normals(s, c, b, uses_lists(x), bs, x->num_sms);
         break;
     case SPH_S_WC_ACCEL:
         sph::launch_aux(s, c, b, bs);
-        sph::launch_wc_forces(s, c, b, x->p.neighbor_mode == SPH_NEIGH_LIST, false, true, bs);
+        sph::launch_wc_forces(s, c, b, x->p.neighbor_mode == SPH_NEIGH_LIST, false, true, bs, x->num_sms);
         break;
     case SPH_S_WC_INTEGRATE:
         sph::launch_wc_integrate(s, c, b, bs);
@@ -404,7 +404,7 @@ int run_stage_impl(sph_ctx* x, int stage) {
         sph::launch_pci_init_density(s, c, b, bs);
         break;
     case SPH_S_PCI_INIT_FORCES:
-        sph::launch_pci_init_forces(s, c, b, bs);
+        sph::launch_pci_init_forces(s, c, b, bs, x->num_sms);
         break;
     case SPH_S_PCI_LOOP: {
         cudaMemsetAsync(b.pci_maxerr, 0, sizeof(float) * x->max_iter_slots, s);
@@ -522,7 +522,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
         gather_vel();
         const bool pack = lists && c.sigma != 0.f;
         if (c.sigma != 0.f) {
-            sph::launch_normals(s, c, b, lists, bs, pack, lists);   /* k_lists_density wrote prho */
+            sph::launch_normals(s, c, b, lists, bs, x->num_sms, pack, lists);   /* k_lists_density wrote prho */
             mark(x, "k_normals");
         }
         if (x->any_massive) {
@@ -541,7 +541,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
                 sph::Const ck = c;
                 ck.block0 = b0;
                 ck.blocks = b1 - b0;
-                sph::launch_wc_forces(s, ck, b, lists, true, false, bs, pack);
+                sph::launch_wc_forces(s, ck, b, lists, true, false, bs, x->num_sms, pack);
                 const size_t i0 = (size_t)b0 * bs, i1 = std::min((size_t)b1 * bs, (size_t)x->N);
                 cudaEventRecord(x->ev_chunk[k], s);
                 cudaStreamWaitEvent(x->copy_stream, x->ev_chunk[k], 0);
@@ -550,7 +550,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
             cudaEventRecord(x->ev_copy, x->copy_stream);
             cudaStreamWaitEvent(s, x->ev_copy, 0);
         } else {
-            sph::launch_wc_forces(s, c, b, lists, true, false, bs, pack);
+            sph::launch_wc_forces(s, c, b, lists, true, false, bs, x->num_sms, pack);
         }
         mark(x, "k_wc_forces");
     } else {
@@ -570,10 +570,10 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
          * (velocity, normal, 1/rho) that the force pass reads */
         const bool pack = c.sigma != 0.f;
         if (pack) {
-            sph::launch_normals(s, c, b, true, bs, true, !c.compat && !c.batched);   /* after k_lists_density_pci */
+            sph::launch_normals(s, c, b, true, bs, x->num_sms, true, !c.compat && !c.batched);   /* after k_lists_density_pci */
             mark(x, "k_normals");
         }
-        sph::launch_pci_init_forces(s, c, b, bs, pack);
+        sph::launch_pci_init_forces(s, c, b, bs, x->num_sms, pack);
         mark(x, "k_pci_init_forces");
         cudaMemsetAsync(b.pci_maxerr, 0, sizeof(float) * x->max_iter_slots, s);
         cudaMemsetAsync(b.barrier, 0, 4 * sizeof(unsigned), s);

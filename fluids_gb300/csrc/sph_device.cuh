@@ -43,6 +43,7 @@ struct Const {
     int tile_blocks;     /* batched: CTAs of a persistent launch over the tiles */
     int block0, blocks;  /* single-scene passes launched in parts: blocks [block0, block0 + blocks)
                             of the whole pass (0, 0: the whole pass in one launch) */
+    int first, last;     /* the particles [first, last) of a launch with several lanes a particle */
 };
 
 /* One scene of a batched context: its grid (origin, dimensions, offset of its cells in the
@@ -90,10 +91,16 @@ struct SceneTile {
  * constants are read once, at a warp-uniform address, for its 32 particles (one per lane),
  * instead of being looked up per particle.  f must not use warp-collective operations (a
  * tile's lanes beyond its count are idle). */
-template <bool BATCH, class F>
+/* W > 1 (single scene): W adjacent threads per particle, all of them running f(c, 0, i) to its
+ * end (it sums over them); threads past the last particle run it for the last one, which f
+ * tells by lane_of_particle. */
+template <bool BATCH, int W = 1, class F>
 __device__ __forceinline__ void for_each_particle(const Const& c0, const SceneTile* __restrict__ tiles,
                                                   const SceneDev* __restrict__ scenes, unsigned* next, F&& f) {
-    if constexpr (BATCH) {
+    if constexpr (W > 1) {
+        const int i = c0.first + ((int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x) / W;
+        f(c0, 0LL, i < c0.last ? i : c0.last - 1);
+    } else if constexpr (BATCH) {
         __shared__ int s_chunk;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
 #pragma unroll 1
@@ -117,6 +124,13 @@ __device__ __forceinline__ void for_each_particle(const Const& c0, const SceneTi
         const int i = (c0.block0 + (int)blockIdx.x) * (int)blockDim.x + (int)threadIdx.x;
         if (i < c0.n) f(c0, 0LL, i);
     }
+}
+
+/* This thread's place among the W of its particle, W for a thread past the last particle. */
+template <int W>
+__device__ __forceinline__ int lane_of_particle(const Const& c) {
+    const int t = (int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x;
+    return c.first + t / W < c.last ? t & (W - 1) : W;
 }
 
 /* Compile-time choice: single-scene kernels (BATCH = false) use the parameter's grid and
@@ -468,6 +482,45 @@ __device__ __forceinline__ void list_neighbors(int i, int n, const int* __restri
         const float4 pj = __ldg(&npos[j]);
         f(j, pj, __fsub_rn(px, pj.x), __fsub_rn(py, pj.y), __fsub_rn(pz, pj.z));
     }
+}
+
+/* Lanes per particle of the list walks: the most of 8, 4 and 2 that half of the GPU's threads
+ * hold, else 1.  Measured on GB300 (normals + forces of a step, with the launch gaps, us; 1, 2,
+ * 4 and 8 lanes): 2,197 particles 33, 25, 19, 17; 9,261 35, 25, 20, 18; 32,768 36, 25, 25, 29;
+ * 64,000 36, 31, 33, 37; 125,000 45, 45, 47, 55. */
+inline int walk_lanes(int n, int num_sms) {
+    for (int w = 8; w > 1; w /= 2)
+        if ((long long)n * w <= 1024LL * num_sms) return w;
+    return 1;
+}
+/* The list of particle i shared by W lanes (small scenes, where one thread's walk is all
+ * latency): lane w visits entries w, w + W, ...; four entries and their positions are loaded
+ * before their visits.  A lane's last batch may visit the particle itself (distance 0) in
+ * place of entries past the end. */
+template <int W, class F>
+__device__ __forceinline__ void list_neighbors_split(int i, int n, const int* __restrict__ list, int len, int w,
+                                                     int self, const float4* __restrict__ npos, float px, float py,
+                                                     float pz, F&& f) {
+    constexpr int U = 4;
+#pragma unroll 1
+    for (int k = w; k < len; k += U * W) {
+        int j[U];
+        float4 q[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = k + u * W < len ? __ldg(&list[i + (size_t)(k + u * W) * n]) : self;
+#pragma unroll
+        for (int u = 0; u < U; ++u) q[u] = __ldg(&npos[j[u]]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            f(j[u], q[u], __fsub_rn(px, q[u].x), __fsub_rn(py, q[u].y), __fsub_rn(pz, q[u].z));
+    }
+}
+/* The sum of v over the W lanes of a particle, in all of them. */
+template <int W>
+__device__ __forceinline__ float sum_lanes(float v) {
+#pragma unroll
+    for (int d = W / 2; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d, W);
+    return v;
 }
 
 /* Neighbour source: either the cell scan or the materialised list, same order. */

@@ -126,10 +126,10 @@ void launch_wc_density(cudaStream_t s, const Const& c, const Bufs& b, bool lists
  * velocity, aux and normal); only the fused step uses it */
 /* prho: the step's list + density pass wrote b.prho, which the walk then reads for both the
  * neighbour's position and its density */
-void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, bool pack = false,
+void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack = false,
                     bool prho = false);
 void launch_wc_forces(cudaStream_t s, const Const& c, const Bufs& b, bool lists, bool fuse_integrate,
-                      bool write_acc, int bs, bool pack = false);
+                      bool write_acc, int bs, int num_sms, bool pack = false);
 void launch_wc_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_aux(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 /* PHYSICS PCISPH: the neighbour lists and compute_initial_density in one pass */
@@ -145,7 +145,7 @@ bool launch_lists_split(cudaStream_t s, const Const& c, const Bufs& b, bool pci,
 
 /* sph_pcisph.cu */
 void launch_pci_init_density(cudaStream_t s, const Const& c, const Bufs& b, int bs);
-void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, bool pack = false);
+void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms, bool pack = false);
 int pci_loop_blocks(int num_sms, int bs);
 cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter, int blocks,
                             int bs, bool fuse_integrate);

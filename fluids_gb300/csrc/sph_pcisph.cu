@@ -322,19 +322,20 @@ __global__ void __launch_bounds__(256) k_pci_init_density(Const c, Bufs b) {
 #ifndef SPH_PCI_INIT_PIPE
 #define SPH_PCI_INIT_PIPE 1
 #endif
-template <bool PACK, bool MON = false>
+/* W > 1 (small scenes, PACK): W lanes a particle (list_neighbors_split), their sums added. */
+template <bool PACK, bool MON = false, int W = 1>
 __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    b.f_press[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (W == 1 && t >= c.n) return;
+    const int w = W > 1 ? (t / W < c.n ? t & (W - 1) : W) : 0;
+    const int i = W > 1 ? min(t / W, c.n - 1) : t;
+    if (w == 0) b.f_press[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 pi = __ldg(&b.pos_s[i]), vi = __ldg(&b.vel_s[i]), ni = __ldg(&b.normal[i]);
     const float di = __ldg(&b.density[i]);
     const float H = c.h_def;
     const float two_rho0 = 2.0f * c.rho0_def;
     float vx = 0.f, vy = 0.f, vz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f, ox = 0.f, oy = 0.f, oz = 0.f;
-    list_neighbors<SPH_PCI_INIT_U, SPH_PCI_INIT_PIPE, SPH_PCI_INIT_PIPE>(i, c.n, b.nlist, __ldg(&b.nlen[i]), b.pos_s,
-                                                                       pi.x, pi.y, pi.z,
-                   [&](int j, float4, float dx, float dy, float dz) {
+    auto pair = [&](int j, float4, float dx, float dy, float dz) {
                        float4 vj, nj;
                        float rn, inv, w, K;
                        const float r2 = dx * dx + dy * dy + dz * dz;
@@ -366,13 +367,27 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
                        ox += ((dx * inv) * sk) * K;
                        oy += ((dy * inv) * sk) * K;
                        oz += ((dz * inv) * sk) * K;
-                   });
+                   };
+    if constexpr (W > 1) {
+        /* a lane's last batch may visit the particle itself, whose every term is zero */
+        list_neighbors_split<W>(i, c.n, b.nlist, w < W ? __ldg(&b.nlen[i]) : 0, w, i, b.pos_s, pi.x, pi.y, pi.z, pair);
+    } else {
+        list_neighbors<SPH_PCI_INIT_U, SPH_PCI_INIT_PIPE, SPH_PCI_INIT_PIPE>(i, c.n, b.nlist, __ldg(&b.nlen[i]),
+                                                                           b.pos_s, pi.x, pi.y, pi.z, pair);
+    }
     const float md = c.mass_def;
     const float vsc = (c.mu * (md * md)) * (c.visc_lapl / di);
     const float csc = md * c.st_main;
     const float tsc = (-c.sigma) * md;
-    b.f_other[i] = make_float4(vx * vsc + tsc * (ux + ox * csc), vy * vsc + tsc * (uy + oy * csc),
-                               vz * vsc + tsc * (uz + oz * csc), 0.f);
+    float fx = vx * vsc + tsc * (ux + ox * csc), fy = vy * vsc + tsc * (uy + oy * csc),
+          fz = vz * vsc + tsc * (uz + oz * csc);
+    if constexpr (W > 1) {
+        fx = sum_lanes<W>(fx);
+        fy = sum_lanes<W>(fy);
+        fz = sum_lanes<W>(fz);
+        if (w != 0) return;
+    }
+    b.f_other[i] = make_float4(fx, fy, fz, 0.f);
 }
 
 /* 5 blocks/SM (at most 51 registers, a few bytes of spill): 6.7 ms per 4M-particle step vs
@@ -483,8 +498,15 @@ void launch_pci_init_density(cudaStream_t s, const Const& c, const Bufs& b, int 
     if (c.compat) k_pci_init_density<true><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
     else k_pci_init_density<false><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
 }
-void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, bool pack) {
+void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms, bool pack) {
     if (c.n <= 0) return;
+    if (pack && !c.compat) {
+        switch (walk_lanes(c.n, num_sms)) {
+        case 8: k_pci_init_forces<true, false, 8><<<nblk(8 * c.n, 256), 256, 0, s>>>(c, b); return;
+        case 4: k_pci_init_forces<true, false, 4><<<nblk(4 * c.n, 256), 256, 0, s>>>(c, b); return;
+        case 2: k_pci_init_forces<true, false, 2><<<nblk(2 * c.n, 256), 256, 0, s>>>(c, b); return;
+        }
+    }
     if (c.monaghan) {
         if (pack) k_pci_init_forces<true, true><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
         else k_pci_init_forces<false, true><<<nblk(c.n, bs), bs, 0, s>>>(c, b);

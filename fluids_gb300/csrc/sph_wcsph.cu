@@ -186,22 +186,20 @@ __global__ void __launch_bounds__(256) k_aux(int n, const float* __restrict__ de
 #endif
 /* MON: compute_normals with the Monaghan kernels, GRAD_W_DEFAULT(r, r.r, h) / rho_j
  * (normals.cl:66; the kernel text passes r^2 where the function takes |r|). */
-template <bool LIST, bool EXACT, bool BATCH, bool MON = false, bool PRHO = false>
+template <bool LIST, bool EXACT, bool BATCH, bool MON = false, bool PRHO = false, int W = 1>
 __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl0, const float4* __restrict__ aux,
                                                  const float* __restrict__ dens, float4* __restrict__ normal,
                                                  const SceneDev* __restrict__ scenes,
                                                  const SceneTile* __restrict__ tiles, unsigned* next,
                                                  const float4* __restrict__ vel_s = nullptr,
                                                  float4* __restrict__ nrec = nullptr) {
-  for_each_particle<BATCH>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
+  for_each_particle<BATCH, W>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
     Neigh<LIST, EXACT> fl = fl0;
     fl.tab += base;
     const float4 pi = __ldg(&fl.npos[i]);
     const float H = c.h_def, HH = H * H;
     float nx = 0.f, ny = 0.f, nz = 0.f;
-    /* two entries deep with the next two loaded during the visits */
-    fl.template visit<true, SPH_NORMALS_WALK, SPH_NORMALS_PRED != 0>(c, i, pi.x, pi.y, pi.z,
-                                                                     [&](int j, float4 q, float dx, float dy, float dz) {
+    auto pair = [&](int j, float4 q, float dx, float dy, float dz) {
         /* 1/rho_j: PRHO, from the w of the neighbour record the walk loaded with its position
          * (npos = prho); otherwise from the dense density array (8 particles per 32-byte
          * sector instead of 2 for aux; the pass is bound by L1 throughput); __frcp_rn is the
@@ -221,7 +219,18 @@ __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl
             ny += dy * k;
             nz += dz * k;
         }
-    });
+    };
+    if constexpr (W > 1) {
+        const int w = lane_of_particle<W>(c);
+        list_neighbors_split<W>(i, c.n, fl.list, w < W ? __ldg(&fl.len[i]) : 0, w, i, fl.npos, pi.x, pi.y, pi.z, pair);
+        nx = sum_lanes<W>(nx);
+        ny = sum_lanes<W>(ny);
+        nz = sum_lanes<W>(nz);
+        if (w != 0) return;
+    } else {
+        /* two entries deep with the next two loaded during the visits */
+        fl.template visit<true, SPH_NORMALS_WALK, SPH_NORMALS_PRED != 0>(c, i, pi.x, pi.y, pi.z, pair);
+    }
     const float k = (c.poly6_grad * c.mass_def) * H;
     const float4 nv = make_float4(nx * k, ny * k, nz * k, 0.f);
     normal[i] = nv;
@@ -280,9 +289,10 @@ __device__ __forceinline__ void wc_integrate_one(const Const& c, float4 p, float
  * normal and 1/rho come from nrec as two adjacent float4 (one 32-byte sector) instead of
  * three separate loads; rho_j = 1/(1/rho_j) enters only the symmetrised surface-tension
  * factor 2 rho0 / (rho_i + rho_j) = 2 rho0 R_j / (rho_i R_j + 1). */
-template <bool COMPAT, bool LIST, bool FUSE, bool WRITE_ACC, bool ST, bool BATCH, bool PACK = false>
+template <bool COMPAT, bool LIST, bool FUSE, bool WRITE_ACC, bool ST, bool BATCH, bool PACK = false, int W = 1>
 __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const c0, Neigh<LIST, COMPAT> fl0, Neigh<LIST, COMPAT> bl0, Bufs b) {
-  for_each_particle<BATCH>(c0, b.tiles, b.scenes, b.tile_next + 3, [&](const Const& c, long long base, int i) {
+  for_each_particle<BATCH, W>(c0, b.tiles, b.scenes, b.tile_next + 3, [&](const Const& c, long long base, int i) {
+    const int w = W > 1 ? lane_of_particle<W>(c) : 0;
     Neigh<LIST, COMPAT> fl = fl0, bl = bl0;
     fl.tab += base;
     bl.tab += base;
@@ -295,7 +305,7 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
     auto boundary_pairs = [&]() {
         if (c.nb <= 0) return;
         const float c2 = 2.0f * C * sg;
-        bl.visit(c, i, pi.x, pi.y, pi.z, [&](int j, float4, float dx, float dy, float dz) {
+        auto pair = [&](int j, float4, float dx, float dy, float dz) {
             const float r2 = dx * dx + dy * dy + dz * dz;
             const float irn = rsqrtf(r2);
             const float w = h - r2 * irn;
@@ -303,7 +313,17 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
             bax += dx * k;
             bay += dy * k;
             baz += dz * k;
-        });
+        };
+        if constexpr (W > 1) {
+            const int len = w < W ? __ldg(&bl.len[i]) : 0;
+            for (int k = w; k < len; k += W) {
+                const int j = __ldg(&bl.list[i + (size_t)k * c.n]);
+                const float4 q = __ldg(&bl.npos[j]);
+                pair(j, q, __fsub_rn(pi.x, q.x), __fsub_rn(pi.y, q.y), __fsub_rn(pi.z, q.z));
+            }
+        } else {
+            bl.visit(c, i, pi.x, pi.y, pi.z, pair);
+        }
     };
     if (BATCH) boundary_pairs();
     float4 ni = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -311,11 +331,7 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
     float pax = 0.f, pay = 0.f, paz = 0.f, vax = 0.f, vay = 0.f, vaz = 0.f;
     float cux = 0.f, cuy = 0.f, cuz = 0.f, cox = 0.f, coy = 0.f, coz = 0.f;
     const float rmin2 = c.rmin2_wc, two_rho0 = 2.0f * c.rho0;
-    /* the list walk SPH_FORCES_WALK (four) entries deep with the next entries loaded during
-     * the visits and a predicated last batch, single-scene; the batched kernel walks two deep
-     * with a serial tail (measured faster there) */
-    fl.template visit<true, BATCH ? 2 : SPH_FORCES_WALK, !BATCH>(c, i, pi.x, pi.y, pi.z,
-                                                                 [&](int j, float4, float dx, float dy, float dz) {
+    auto pair = [&](int j, float4, float dx, float dy, float dz) {
         const float r2 = dx * dx + dy * dy + dz * dz;
         /* loaded ahead of the guard so that the list loop can issue them early */
         float4 aj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -353,7 +369,14 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
                 coz += dz * ck;
             }
         }
-    });
+    };
+    if constexpr (W > 1)
+        list_neighbors_split<W>(i, c.n, fl.list, w < W ? __ldg(&fl.len[i]) : 0, w, i, fl.npos, pi.x, pi.y, pi.z, pair);
+    else
+        /* the list walk SPH_FORCES_WALK (four) entries deep with the next entries loaded during
+         * the visits and a predicated last batch, single-scene; the batched kernel walks two
+         * deep with a serial tail (measured faster there) */
+        fl.template visit<true, BATCH ? 2 : SPH_FORCES_WALK, !BATCH>(c, i, pi.x, pi.y, pi.z, pair);
     /* single scene: the boundary pairs after the fluid pairs, so that their sums are not live
      * during the fluid walk (each term keeps its own accumulator, so the result is the same);
      * the batched kernel measured faster with them first (2.46 vs 2.59 ms per batched step) */
@@ -363,7 +386,14 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
     const float vs = COMPAT ? (c.visc_lapl * c.mu) : (c.visc_lapl * c.mu) * (m * ai.y);
     vax *= vs; vay *= vs; vaz *= vs;
     float ax = pax + vax + bax, ay = c.g + pay + vay + bay, az = paz + vaz + baz;
-    if (ST) {
+    if constexpr (W > 1) {
+        /* each lane's share of every term, then their sum */
+        const float cs = COMPAT ? c.st_main : c.st_main * m, ns = ST ? -c.sigma : 0.f;
+        ax = sum_lanes<W>(((ns * (cux + cox * cs) + pax) + vax) + bax);
+        ay = c.g + sum_lanes<W>(((ns * (cuy + coy * cs) + pay) + vay) + bay);
+        az = sum_lanes<W>(((ns * (cuz + coz * cs) + paz) + vaz) + baz);
+        if (w != 0) return;
+    } else if (ST) {
         const float cs = COMPAT ? c.st_main : c.st_main * m;
         const float ns = -c.sigma;
         ax = (((ns * (cux + cox * cs)) + pax) + vax) + bax;
@@ -490,8 +520,31 @@ void launch_aux(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
     k_aux<<<nblk(c.n, bs), bs, 0, s>>>(c.n, b.density, b.pressure, b.aux);
 }
 
-void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, bool pack, bool prho) {
+/* The walks of the fused step of a single scene take several lanes a particle in small scenes
+ * (walk_lanes); their sums then add by lane instead of in list order. */
+static int split_walk(const Const& c, int num_sms) { return c.batched || c.compat ? 1 : walk_lanes(c.n, num_sms); }
+
+template <int W>
+static void normals_split(cudaStream_t s, const Const& c0, const Bufs& b, float4* nrec) {
+    Const c = c0;
+    c.first = 0;
+    c.last = c.n;
+    auto fl = fluid_src<true, true>(b);
+    fl.npos = b.prho;
+    k_normals<true, true, false, false, true, W><<<nblk(c.n * W, 256), 256, 0, s>>>(
+        c, fl, b.aux, b.density, b.normal, b.scenes, b.tiles, nullptr, b.vel_s, nrec);
+}
+
+void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack, bool prho) {
     if (c.n <= 0) return;
+    if (prho && lists) {
+        float4* rec = pack ? b.nrec : nullptr;
+        switch (split_walk(c, num_sms)) {
+        case 8: normals_split<8>(s, c, b, rec); return;
+        case 4: normals_split<4>(s, c, b, rec); return;
+        case 2: normals_split<2>(s, c, b, rec); return;
+        }
+    }
     const int g = nblk(c.n, bs), gt = grid_for<true>(c, bs);
     float4* nrec = pack ? b.nrec : nullptr;
     unsigned* next = tile_counter(s, b, 2, c.batched != 0);
@@ -534,14 +587,36 @@ void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, i
     }
 }
 
+template <int W>
+static void forces_split(cudaStream_t s, const Const& c0, const Bufs& b, int bs, bool st) {
+    Const c = c0;
+    c.first = c0.block0 * bs;   /* a part of the pass covers the particles of its blocks of bs */
+    c.last = c0.blocks > 0 && (c0.block0 + c0.blocks) * bs < c.n ? (c0.block0 + c0.blocks) * bs : c.n;
+    auto fs = fluid_src<true, false>(b);
+    auto bsrc = bnd_src<true, false>(b);
+    const int g = nblk((c.last - c.first) * W, 256);
+    if (st) k_wc_forces<false, true, true, false, true, false, true, W><<<g, 256, 0, s>>>(c, fs, bsrc, b);
+    else k_wc_forces<false, true, true, false, false, false, false, W><<<g, 256, 0, s>>>(c, fs, bsrc, b);
+}
+
 template <bool COMPAT, bool LIST, bool BATCH>
 static void forces_launch(cudaStream_t s, const Const& c, const Bufs& b, bool fuse, bool write_acc, int bs,
-                          bool pack) {
+                          int num_sms, bool pack) {
     const int g = grid_for<BATCH>(c, bs);
     tile_counter(s, b, 3, BATCH);
     const bool st = c.sigma != 0.f;
     auto fs = fluid_src<LIST, COMPAT>(b);
     auto bsrc = bnd_src<LIST, COMPAT>(b);
+    if constexpr (LIST && !COMPAT && !BATCH) {
+        /* the fused step's pass, without the acceleration field */
+        if (fuse && !write_acc && pack == st) {
+            switch (split_walk(c, num_sms)) {
+            case 8: forces_split<8>(s, c, b, bs, st); return;
+            case 4: forces_split<4>(s, c, b, bs, st); return;
+            case 2: forces_split<2>(s, c, b, bs, st); return;
+            }
+        }
+    }
     if constexpr (LIST) {
         if (pack && st && fuse && !write_acc) {
             k_wc_forces<COMPAT, LIST, true, false, true, BATCH, true><<<g, bs, 0, s>>>(c, fs, bsrc, b);
@@ -560,22 +635,22 @@ static void forces_launch(cudaStream_t s, const Const& c, const Bufs& b, bool fu
 
 template <bool COMPAT, bool LIST>
 static void forces_dispatch(cudaStream_t s, const Const& c, const Bufs& b, bool fuse, bool write_acc, int bs,
-                            bool pack) {
+                            int num_sms, bool pack) {
     if constexpr (!COMPAT) {
-        if (c.batched) { forces_launch<false, LIST, true>(s, c, b, fuse, write_acc, bs, pack); return; }
+        if (c.batched) { forces_launch<false, LIST, true>(s, c, b, fuse, write_acc, bs, num_sms, pack); return; }
     }
-    forces_launch<COMPAT, LIST, false>(s, c, b, fuse, write_acc, bs, pack);
+    forces_launch<COMPAT, LIST, false>(s, c, b, fuse, write_acc, bs, num_sms, pack);
 }
 
 void launch_wc_forces(cudaStream_t s, const Const& c, const Bufs& b, bool lists, bool fuse_integrate,
-                      bool write_acc, int bs, bool pack) {
+                      bool write_acc, int bs, int num_sms, bool pack) {
     if (c.n <= 0) return;
     if (c.compat) {
-        if (lists) forces_dispatch<true, true>(s, c, b, fuse_integrate, write_acc, bs, pack);
-        else forces_dispatch<true, false>(s, c, b, fuse_integrate, write_acc, bs, pack);
+        if (lists) forces_dispatch<true, true>(s, c, b, fuse_integrate, write_acc, bs, num_sms, pack);
+        else forces_dispatch<true, false>(s, c, b, fuse_integrate, write_acc, bs, num_sms, pack);
     } else {
-        if (lists) forces_dispatch<false, true>(s, c, b, fuse_integrate, write_acc, bs, pack);
-        else forces_dispatch<false, false>(s, c, b, fuse_integrate, write_acc, bs, pack);
+        if (lists) forces_dispatch<false, true>(s, c, b, fuse_integrate, write_acc, bs, num_sms, pack);
+        else forces_dispatch<false, false>(s, c, b, fuse_integrate, write_acc, bs, num_sms, pack);
     }
 }
 
