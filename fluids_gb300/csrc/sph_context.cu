@@ -1705,12 +1705,13 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
         g_sort.device = dev;
         size_t ncap = (size_t)n;
         size_t wsb = sph::sort_workspace_bytes(n, 32);
-        if (cudaMalloc(&g_sort.ws, wsb) != cudaSuccess || cudaMalloc(&g_sort.kalt, 4 * ncap) != cudaSuccess ||
-            cudaMalloc(&g_sort.valt, 4 * ncap) != cudaSuccess || cudaMalloc(&g_sort.flags, 16) != cudaSuccess) {
+        if (cudaMalloc(&g_sort.ws, wsb) != cudaSuccess || cudaMalloc(&g_sort.kalt, 8 * ncap) != cudaSuccess ||
+            cudaMalloc(&g_sort.valt, 8 * ncap) != cudaSuccess || cudaMalloc(&g_sort.flags, 16) != cudaSuccess) {
             cudaGetLastError();
             return fail(nullptr, SPH_E_NOMEM, "sph_sort_pairs: scratch allocation failed");
         }
         cudaMemset(g_sort.flags, 0, 16);
+        cudaMemset(g_sort.ws, 0, wsb);   /* the sort's grid barrier starts at zero */
         if (cudaEventCreateWithFlags(&g_sort.done, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
             g_sort.done = nullptr;
@@ -1727,12 +1728,17 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
     cudaStreamIsCapturing(s, &cap);
     const bool order = g_sort.done && cap == cudaStreamCaptureStatusNone;
     if (order) cudaStreamWaitEvent(s, g_sort.done, 0);
-    uint32_t* kr;
-    int32_t* vr;
-    sph::sort_pairs(s, d_keys, d_vals, g_sort.kalt, g_sort.valt, n, key_bits, g_sort.ws, g_sort.flags, sms, &kr, &vr);
-    if (kr != d_keys) {
-        cudaMemcpyAsync(d_keys, kr, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(d_vals, vr, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
+    /* the last pass writes the caller's arrays; three passes go through both copies, a single
+     * one through a copy and back */
+    const int passes = sph::sort_passes(key_bits);
+    uint32_t *ka = g_sort.kalt, *kb = ka + g_sort.n_cap;
+    int32_t *va = g_sort.valt, *vb = va + g_sort.n_cap;
+    sph::SortBufs sb{d_keys, d_vals, {ka, d_keys, ka, d_keys}, {va, d_vals, va, d_vals}};
+    if (passes == 3) sb = sph::SortBufs{d_keys, d_vals, {ka, kb, d_keys, nullptr}, {va, vb, d_vals, nullptr}};
+    sph::sort_pairs_passes(s, sb, n, nullptr, key_bits, g_sort.ws, g_sort.flags, sms);
+    if (passes == 1) {
+        cudaMemcpyAsync(d_keys, ka, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
+        cudaMemcpyAsync(d_vals, va, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
     }
     if (order) cudaEventRecord(g_sort.done, s);
     cudaError_t e = cudaGetLastError();

@@ -144,6 +144,42 @@ __device__ __forceinline__ long long scene_setup_t(Const& c, const SceneDev* sce
 constexpr unsigned kFlagNan = 1u, kFlagEscaped = 2u, kFlagTimeout = 4u, kFlagOverflow = 8u,
                    kFlagNonconverged = 16u;
 
+constexpr long long kBarrierSpinLimit = 1LL << 24;
+
+/* Grid-wide barrier: bar[0] = arrivals, bar[1] = generation.  Returns false on timeout.
+ * extra > 0 (an injected stall) waits for arrivals that never come, so every CTA's bounded
+ * wait runs out. */
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned* flags, unsigned extra) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        volatile unsigned* vgen = bar + 1;
+        const unsigned gen = *vgen;
+        __threadfence();
+        const unsigned arrived = atomicAdd(bar, 1u);
+        int ok = 1;
+        if (arrived == gridDim.x - 1 + extra) {
+            atomicExch(bar, 0u);
+            __threadfence();
+            atomicAdd(bar + 1, 1u);
+        } else {
+            long long spins = 0;
+            while (*vgen == gen) {
+                if (++spins > kBarrierSpinLimit) {
+                    atomicOr(flags, kFlagTimeout);
+                    ok = 0;
+                    break;
+                }
+                __nanosleep(64);
+            }
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
 /* ---- IEEE helpers that the compiler may not contract into FMAs ---------------------- */
 __device__ __forceinline__ float r2_exact(float dx, float dy, float dz) {
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));

@@ -67,6 +67,16 @@ struct Bufs {
 /* sph_sort.cu */
 int sort_passes(int key_bits);
 size_t sort_workspace_bytes(int n, int key_bits);
+struct SortBufs {
+    const uint32_t* kin;
+    const int32_t* vin;   /* null: the identity */
+    uint32_t* k[4];       /* pass p's output (not its input) */
+    int32_t* v[4];
+};
+void sort_launches(cudaStream_t s, const SortBufs& b, int n, int passes, uint32_t* hist, unsigned* flags,
+                   const unsigned* gate, int hblocks, int sblocks);
+void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned* gate, int key_bits, void* ws,
+                       unsigned* flags, int num_sms);
 void sort_pairs(cudaStream_t s, uint32_t* k0, int32_t* v0, uint32_t* k1, int32_t* v1, int n, int key_bits,
                 void* ws, unsigned* flags, int num_sms, uint32_t** kres, int32_t** vres);
 /* The stable sort of keys[0, n) (values: the indices) into kout / vout, computed as an update

@@ -506,6 +506,8 @@ static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigne
             return sph_ctx_fail(x, SPH_E_NOMEM, "render: particle order buffers");
         }
         x->render_sort_bytes = nsort;
+        /* the sort workspace starts at zero */
+        cudaMemsetAsync(x->render_sort, 0, sph::sort_workspace_bytes(x->N, 16), x->stream);
     }
     if (x->render_pixels < npix) {
         cudaStreamSynchronize(x->stream);
@@ -528,11 +530,11 @@ static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigne
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
     sph::k_splat_clear<<<(unsigned)((npix + bs - 1) / bs), bs, 0, s>>>(npix, key);
-    uint32_t* okeys = reinterpret_cast<uint32_t*>(x->render_sort);
+    void* ws = x->render_sort;   /* first, so that it stays in place when the particle count changes */
+    uint32_t* okeys = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + sph::sort_workspace_bytes(n, 16));
     int32_t* order = reinterpret_cast<int32_t*>(okeys + n);
     uint32_t* okeys_alt = reinterpret_cast<uint32_t*>(order + n);
     int32_t* order_alt = reinterpret_cast<int32_t*>(okeys_alt + n);
-    void* ws = order_alt + n;
     sph::k_depth_order<<<(n + bs - 1) / bs, bs, 0, s>>>(v, n, x->b.pos, okeys, order);
     uint32_t* ks;
     int32_t* so;

@@ -7,9 +7,9 @@
  *
  * Algorithm (Adinets & Merrill, "Onesweep", 2022):
  *   1. k_sort_hist: one read of the keys builds the 256-bin histogram of every 8-bit digit
- *      pass at once (warp match_any aggregation into shared counters).
+ *      pass at once (aggregated per warp and digit into shared counters).
  *   2. per pass, k_onesweep: each CTA takes the next tile id from an atomic counter (so
- *      tiles are scheduled in order), ranks its kTile keys stably (warp match_any per
+ *      tiles are scheduled in order), ranks its kTile keys stably (ballots per
  *      32-key round, per-warp digit counters), publishes its per-digit counts, and looks
  *      back over earlier tiles' published counts (decoupled look-back) for its global
  *      digit offsets.  Keys are then reordered in shared memory by digit and written out
@@ -40,6 +40,7 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagInc = 2u << 30;
 constexpr uint32_t kValMask = (1u << 30) - 1u;
 constexpr long long kSpinLimit = 1LL << 22;
+constexpr int kLookBack = 4;   /* earlier tiles' words in flight in the look-back */
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {
     return *reinterpret_cast<const volatile uint32_t*>(p);
@@ -48,7 +49,27 @@ __device__ __forceinline__ void st_volatile(uint32_t* p, uint32_t v) {
     *reinterpret_cast<volatile uint32_t*>(p) = v;
 }
 
-/* Exclusive prefix sum over the 256 values held one per thread (blockDim = 256). */
+/* The lanes of the warp (all in) that hold the same 8-bit digit.  FEW: by match_any, whose time
+ * grows with the number of different digits in the warp (the step's keys, nearly sorted: a
+ * handful); else by one ballot per bit unless all are equal.  Measured on GB300: 1,062,234
+ * random 24-bit pairs 111 us by match_any, 93 by ballots, 6,000,000 of 32 bits 458 and 331;
+ * the nearly sorted keys of a 4,194,304-particle step 40 us faster by match_any. */
+template <bool FEW>
+__device__ __forceinline__ unsigned same_digit(uint32_t d) {
+    if (FEW) return __match_any_sync(0xffffffffu, d);
+    unsigned peers = 0xffffffffu;
+    if (__all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0))) return peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (d >> b) & 1u;
+        const unsigned v = __ballot_sync(0xffffffffu, one);
+        peers &= one ? v : ~v;
+    }
+    return peers;
+}
+
+/* Exclusive prefix sum over the 256 values held one per thread by the first 256 threads
+ * (every thread of the block calls it). */
 __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_t* s_warp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t x = v;
@@ -57,7 +78,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
         uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
         if (lane >= d) x += y;
     }
-    if (lane == 31) s_warp[warp] = x;
+    if (lane == 31 && warp < kWarps) s_warp[warp] = x;
     __syncthreads();
     if (warp == 0) {
         uint32_t w = lane < kWarps ? s_warp[lane] : 0u;
@@ -69,7 +90,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
         if (lane < kWarps) s_warp[lane] = w;
     }
     __syncthreads();
-    uint32_t before = warp > 0 ? s_warp[warp - 1] : 0u;
+    uint32_t before = warp > 0 && warp < kWarps ? s_warp[warp - 1] : 0u;
     __syncthreads();
     return before + x - v;
 }
@@ -79,6 +100,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
  * (coalesced across the warp) before it ranks any, so that their loads are in flight
  * together; per key and pass, the lanes holding the same digit add their count once. */
 constexpr int kHistItems = 8;
+template <bool FEW>
 __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restrict__ keys, int n, int passes,
                                                         uint32_t* __restrict__ hist, const unsigned* __restrict__ gate) {
     __shared__ uint32_t s_hist[4][256];
@@ -99,12 +121,10 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
             const long long i = base + (long long)u * kThreads + threadIdx.x;
             const bool valid = i < n;
             const unsigned active = __ballot_sync(0xffffffffu, valid);
-            if (valid) {
-                for (int p = 0; p < passes; ++p) {
-                    const uint32_t d = (k[u] >> (8 * p)) & 255u;
-                    const unsigned peers = __match_any_sync(active, d);
-                    if (lane == __ffs(peers) - 1) atomicAdd(&s_hist[p][d], (uint32_t)__popc(peers));
-                }
+            for (int p = 0; p < passes; ++p) {
+                const uint32_t d = (k[u] >> (8 * p)) & 255u;
+                const unsigned peers = same_digit<FEW>(d) & active;
+                if (valid && lane == __ffs(peers) - 1) atomicAdd(&s_hist[p][d], (uint32_t)__popc(peers));
             }
         }
     }
@@ -115,6 +135,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
     }
 }
 
+template <bool FEW>
 __global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                                                        uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int n,
                                                        int shift, int pass, int tiles,
@@ -156,7 +177,7 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restric
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
         const uint32_t d = (key[k] >> shift) & 255u;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned peers = same_digit<FEW>(d);
         const uint32_t before = s_whist[warp][d];
         __syncwarp();
         if ((peers & lt_mask) == 0u) s_whist[warp][d] = before + (uint32_t)__popc(peers);
@@ -181,21 +202,33 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restric
         st_volatile(&st[d], kFlagInc | cnt);
     } else {
         st_volatile(&st[d], kFlagAgg | cnt);
-        for (int t = tile - 1; t >= 0; --t) {
+        /* kLookBack earlier tiles a step, their words read together: a tile's walk is a chain
+         * of L2 latencies, and with every tile resident it is half as long as there are tiles
+         * before it */
+        bool done = false;
+        for (int t = tile - 1; !done; t -= kLookBack) {
             const uint32_t* sp = status + ((size_t)pass * tiles + t) * 256 + d;
-            uint32_t s = ld_volatile(sp);
-            long long spins = 0;
-            while ((s & (kFlagAgg | kFlagInc)) == 0u) {
-                if (++spins > kSpinLimit) {
-                    atomicOr(flags, kFlagTimeout);
-                    s = kFlagInc;
-                    break;
+            uint32_t word[kLookBack];
+#pragma unroll
+            for (int u = 0; u < kLookBack; ++u)
+                word[u] = t - u >= 0 ? ld_volatile(sp - u * 256) : kFlagInc;   /* nothing before tile 0 */
+#pragma unroll
+            for (int u = 0; u < kLookBack; ++u) {
+                if (done) break;
+                uint32_t s = word[u];
+                long long spins = 0;
+                while ((s & (kFlagAgg | kFlagInc)) == 0u) {
+                    if (++spins > kSpinLimit) {
+                        atomicOr(flags, kFlagTimeout);
+                        s = kFlagInc;
+                        break;
+                    }
+                    __nanosleep(32);
+                    s = ld_volatile(sp - u * 256);
                 }
-                __nanosleep(32);
-                s = ld_volatile(sp);
+                prior += s & kValMask;
+                done = (s & kFlagInc) != 0u;
             }
-            prior += s & kValMask;
-            if (s & kFlagInc) break;
         }
         st_volatile(&st[d], kFlagInc | ((prior + cnt) & kValMask));
     }
@@ -228,43 +261,177 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restric
     }
 }
 
+/* The whole sort of up to kOneTiles tiles of 2,048 pairs (4,096 in a single CTA) in one
+ * cooperative launch, a tile per CTA: for a small sort the launches of the memset, the
+ * histogram and the passes are its time.  Measured on GB300 against those launches (24-bit
+ * keys, us): 2,387 pairs 20 / 41, 40,000 32 / 45, 150,000 38 / 49, 300,000 44 / 52, 500,000
+ * 56 / 59, 600,000 (32-bit keys) 76 / 75.  Per
+ * pass each CTA ranks its tile, publishes its digit counts, and after a grid barrier adds the
+ * counts of the tiles before it (and of all tiles, for the buckets), which it reads row by
+ * row, so there is no separate histogram and no look-back; a second barrier ends the pass. */
+constexpr int kOneThreads = 512;
+constexpr int kOneWarps = kOneThreads / 32;
+constexpr int kOneTile = kOneThreads * 4;
+constexpr int kOneTiles = 256;
+constexpr int kOneSolo = kOneThreads * 8;   /* the largest sort of a single CTA */
+template <int ITEMS>
+__global__ void __launch_bounds__(kOneThreads) k_sort_one(SortBufs b, int n, int passes, uint32_t* __restrict__ counts,
+                                                          unsigned* bar, unsigned* __restrict__ flags,
+                                                          const unsigned* __restrict__ gate) {
+    __shared__ uint32_t s_keys[kOneThreads * ITEMS];
+    __shared__ int32_t s_vals[kOneThreads * ITEMS];
+    __shared__ uint32_t s_whist[kOneWarps][256];
+    __shared__ uint32_t s_part[2][2][256];
+    __shared__ uint32_t s_tprefix[256], s_dbase[256];
+    __shared__ uint32_t s_scan[kWarps];
+    if (gate && *gate == 0u) return;   /* the whole grid leaves together */
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tile = blockIdx.x, tiles = gridDim.x, base = tile * (kOneThreads * ITEMS), wbase = base + warp * (32 * ITEMS);
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const int d = tid & 255, half = tid >> 8;
+    for (int p = 0; p < passes; ++p) {
+        const uint32_t* kin = p == 0 ? b.kin : b.k[p - 1];
+        const int32_t* vin = p == 0 ? b.vin : b.v[p - 1];
+        uint32_t* kout = b.k[p];
+        int32_t* vout = b.v[p];
+        uint32_t key[ITEMS], rank[ITEMS];
+        int32_t val[ITEMS];
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int idx = wbase + k * 32 + lane;
+            key[k] = idx < n ? __ldcg(&kin[idx]) : 0xffffffffu;   /* past the end: last, not written */
+            val[k] = idx < n ? (vin ? __ldcg(&vin[idx]) : idx) : 0;
+        }
+        for (int t = tid; t < kOneWarps * 256; t += kOneThreads) (&s_whist[0][0])[t] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint32_t dk = (key[k] >> (8 * p)) & 255u;
+            const unsigned peers = same_digit<false>(dk);
+            const uint32_t before = s_whist[warp][dk];
+            __syncwarp();
+            if ((peers & lt_mask) == 0u) s_whist[warp][dk] = before + (uint32_t)__popc(peers);
+            __syncwarp();
+            rank[k] = before + (uint32_t)__popc(peers & lt_mask);
+        }
+        __syncthreads();
+        uint32_t cnt = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int w = 0; w < kOneWarps; ++w) {
+                const uint32_t c = s_whist[w][d];
+                s_whist[w][d] = cnt;
+                cnt += c;
+            }
+            __stcg(&counts[(size_t)tile * 256 + d], cnt);
+        }
+        if (tiles > 1) {
+            if (!grid_barrier(bar, flags, 0u)) return;
+        } else {
+            __syncthreads();
+        }
+        /* digit d of the tiles: half the rows per half of the block */
+        uint32_t prior = 0, total = 0;
+        const int mid = (tiles + 1) / 2, t1 = half ? tiles : mid;
+#pragma unroll 8
+        for (int t = half ? mid : 0; t < t1; ++t) {
+            const uint32_t c = __ldcg(&counts[(size_t)t * 256 + d]);
+            total += c;
+            if (t < tile) prior += c;
+        }
+        s_part[0][half][d] = prior;
+        s_part[1][half][d] = total;
+        __syncthreads();
+        /* the scans are of 256 values: the first half of the block's, with the barriers inside
+         * run by all threads */
+        const uint32_t all = tid < 256 ? s_part[1][0][d] + s_part[1][1][d] : 0u;
+        const uint32_t bucket = block_exclusive_scan_256(all, s_scan);
+        const uint32_t tpre = block_exclusive_scan_256(cnt, s_scan);
+        if (tid < 256) {
+            s_tprefix[d] = tpre;
+            s_dbase[d] = bucket + s_part[0][0][d] + s_part[0][1][d];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint32_t dk = (key[k] >> (8 * p)) & 255u;
+            const uint32_t slot = s_tprefix[dk] + s_whist[warp][dk] + rank[k];
+            s_keys[slot] = key[k];
+            s_vals[slot] = val[k];
+        }
+        __syncthreads();
+        const int nvalid = min(kOneThreads * ITEMS, n - base);
+        for (int s = tid; s < nvalid; s += kOneThreads) {
+            const uint32_t kk = s_keys[s];
+            const uint32_t dk = (kk >> (8 * p)) & 255u;
+            const uint32_t dest = s_dbase[dk] + (uint32_t)s - s_tprefix[dk];
+            __stcg(&kout[dest], kk);
+            __stcg(&vout[dest], s_vals[s]);
+        }
+        if (p + 1 < passes) {
+            if (tiles > 1) {
+                if (!grid_barrier(bar, flags, 0u)) return;
+            } else {
+                __syncthreads();
+            }
+        }
+    }
+}
+
 int sort_passes(int key_bits) { return key_bits <= 0 ? 0 : (key_bits + 7) / 8; }
 int sort_tiles(int n) { return (n + kTile - 1) / kTile; }
 
 size_t sort_workspace_bytes(int n, int key_bits) {
     const int passes = sort_passes(key_bits);
-    return (size_t)(4 * 256 + 64) * 4 + (size_t)passes * sort_tiles(n) * 256 * 4;
+    const size_t rows = (size_t)passes * sort_tiles(n), one = (size_t)min((n + kOneTile - 1) / kOneTile, kOneTiles);
+    return (size_t)(4 * 256 + 64) * 4 + (rows > one ? rows : one) * 256 * 4;
 }
 
-/* gate: null, or a flag word an earlier kernel of the stream wrote; every kernel of the sort
- * leaves at once while it is 0.  v0 may be null for identity values. */
-static void sort_pairs_impl(cudaStream_t s, const uint32_t* k0, const int32_t* v0, uint32_t* k1, int32_t* v1,
-                            uint32_t* k2, int32_t* v2, int n, const unsigned* gate, int key_bits, void* ws,
-                            unsigned* flags, int num_sms, uint32_t** kres, int32_t** vres) {
+/* The histogram and the passes; hist: 4 x 256 counts, 64 counters, the look-back words, zero. */
+void sort_launches(cudaStream_t s, const SortBufs& b, int n, int passes, uint32_t* hist, unsigned* flags,
+                   const unsigned* gate, int hblocks, int sblocks) {
+    uint32_t* counters = hist + 4 * 256;
+    uint32_t* status = counters + 64;
+    /* gated: the step's full sort, of nearly sorted keys */
+    auto hist_kernel = gate ? k_sort_hist<true> : k_sort_hist<false>;
+    auto pass_kernel = gate ? k_onesweep<true> : k_onesweep<false>;
+    hist_kernel<<<hblocks, kThreads, 0, s>>>(b.kin, n, passes, hist, gate);
+    const uint32_t* ki = b.kin;
+    const int32_t* vi = b.vin;
+    for (int p = 0; p < passes; ++p) {
+        pass_kernel<<<sblocks, kThreads, 0, s>>>(ki, vi, b.k[p], b.v[p], n, 8 * p, p, sort_tiles(n), hist, counters,
+                                                 status, flags, gate);
+        ki = b.k[p];
+        vi = b.v[p];
+    }
+}
+
+/* The sort of (b.kin, b.vin) by passes whose outputs b names.  ws: sort_workspace_bytes, zero
+ * before the first call.  gate: null, or a flag word an earlier kernel of the stream wrote;
+ * every kernel of the sort leaves at once while it is 0. */
+void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned* gate, int key_bits, void* ws,
+                       unsigned* flags, int num_sms) {
     const int passes = sort_passes(key_bits);
     const int tiles = sort_tiles(n);
     uint32_t* hist = reinterpret_cast<uint32_t*>(ws);
     uint32_t* counters = hist + 4 * 256;
     uint32_t* status = counters + 64;
+    const int one = n <= kOneSolo ? 1 : (n + kOneTile - 1) / kOneTile;
+    if (one <= kOneTiles && one <= 2 * num_sms) {
+        SortBufs bb = b;
+        unsigned* bar = counters + 32;   /* zero between sorts */
+        uint32_t* counts = status;
+        int nn = n, np = passes;
+        void* args[] = {&bb, &nn, &np, &counts, &bar, &flags, &gate};
+        void* fn = n <= kOneSolo ? (void*)k_sort_one<8> : (void*)k_sort_one<4>;
+        if (cudaLaunchCooperativeKernel(fn, dim3(one), dim3(kOneThreads), args, 0, s) == cudaSuccess) return;
+        cudaGetLastError();   /* then by several launches */
+    }
     cudaMemsetAsync(ws, 0, sort_workspace_bytes(n, key_bits), s);
     /* a gated sort usually leaves at once: its grids are one wave of looping CTAs */
     int hblocks = min((n + kThreads * kHistItems - 1) / (kThreads * kHistItems), (gate ? 1 : 4) * num_sms);
     if (hblocks < 1) hblocks = 1;
-    const int sblocks = gate ? min(tiles, 2 * num_sms) : tiles;
-    k_sort_hist<<<hblocks, kThreads, 0, s>>>(k0, n, passes, hist, gate);
-    /* pass p reads the previous pass's output and writes (k1, v1) or (k2, v2) in turn */
-    const uint32_t* ki = k0;
-    const int32_t* vi = v0;
-    for (int p = 0; p < passes; ++p) {
-        uint32_t* ko = (p & 1) ? k2 : k1;
-        int32_t* vo = (p & 1) ? v2 : v1;
-        k_onesweep<<<sblocks, kThreads, 0, s>>>(ki, vi, ko, vo, n, 8 * p, p, tiles, hist, counters, status, flags,
-                                                gate);
-        ki = ko;
-        vi = vo;
-    }
-    *kres = const_cast<uint32_t*>(ki);
-    *vres = const_cast<int32_t*>(vi);
+    sort_launches(s, b, n, passes, hist, flags, gate, hblocks, gate ? min(tiles, 2 * num_sms) : tiles);
 }
 
 void sort_pairs(cudaStream_t s, uint32_t* k0, int32_t* v0, uint32_t* k1, int32_t* v1, int n, int key_bits,
@@ -272,7 +439,11 @@ void sort_pairs(cudaStream_t s, uint32_t* k0, int32_t* v0, uint32_t* k1, int32_t
     *kres = k0;
     *vres = v0;
     if (n <= 1 || sort_passes(key_bits) == 0) return;
-    sort_pairs_impl(s, k0, v0, k1, v1, k0, v0, n, nullptr, key_bits, ws, flags, num_sms, kres, vres);
+    SortBufs b{k0, v0, {k1, k0, k1, k0}, {v1, v0, v1, v0}};
+    sort_pairs_passes(s, b, n, nullptr, key_bits, ws, flags, num_sms);
+    const int last = sort_passes(key_bits) - 1;
+    *kres = b.k[last];
+    *vres = b.v[last];
 }
 
 /* ---------------------------------------------------------------------------------------
@@ -729,12 +900,12 @@ void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key
         cudaStreamWaitEvent(side, fork, 0);
     }
     if (n > 1 && sort_passes(key_bits) > 0) {
-        uint32_t* kr;
-        int32_t* vr;
         int32_t* vscr = reinterpret_cast<int32_t*>(w + L.vscr);
         const bool odd = (sort_passes(key_bits) & 1) != 0;
-        sort_pairs_impl(gs, keys, nullptr, odd ? kout : prev, odd ? vout : vscr, odd ? prev : kout,
-                        odd ? vscr : vout, n, over, key_bits, sort_ws, flags, num_sms, &kr, &vr);
+        uint32_t *ka = odd ? kout : prev, *kb = odd ? prev : kout;
+        int32_t *va = odd ? vout : vscr, *vb = odd ? vscr : vout;
+        sort_pairs_passes(gs, SortBufs{keys, nullptr, {ka, kb, ka, kb}, {va, vb, va, vb}}, n, over, key_bits, sort_ws,
+                          flags, num_sms);
     }
     if (fork_side) cudaEventRecord(join, side);
     k_inc_merge<<<L.tiles, kThreads, 0, s>>>(keys, n, bits, tcnt, tpre, boff, bcnt, store, over, kout, vout, prev,

@@ -43,16 +43,11 @@
 #include "sph_kernels.cuh"
 
 namespace sph {
-__global__ void k_sort_hist(const uint32_t* keys, int n, int passes, uint32_t* hist, const unsigned* gate);
-__global__ void k_onesweep(const uint32_t* kin, const int32_t* vin, uint32_t* kout, int32_t* vout, int n,
-                           int shift, int pass, int tiles, const uint32_t* hist, uint32_t* counters,
-                           uint32_t* status, unsigned* flags, const unsigned* gate);
 int sort_tiles(int n);
 }  // namespace sph
 
 namespace {
 constexpr int kMaxPairs = SPH_NOALLOC_SORT_MAX_PAIRS;
-constexpr int kCtaThreads = 256;                        /* block size of the sort kernels */
 constexpr size_t kStatusBytes = (size_t)4 * (kMaxPairs / 4096) * 256 * 4;
 constexpr size_t kWorkspaceBytes = (size_t)(4 * 256 + 64) * 4 + kStatusBytes;   /* hist, counters, status */
 constexpr size_t kFlagsOffset = kWorkspaceBytes;
@@ -140,8 +135,6 @@ extern "C" int sph_sort_pairs_noalloc(const uint32_t* d_keys_in, const int32_t* 
     const size_t ws = sph::sort_workspace_bytes(n, key_bits);
     if (ws > kWorkspaceBytes) return SPH_E_OVERFLOW;
     uint32_t* hist = reinterpret_cast<uint32_t*>(base);
-    uint32_t* counters = hist + 4 * 256;
-    uint32_t* status = counters + 64;
     unsigned* flags = reinterpret_cast<unsigned*>(base + kFlagsOffset);
     uint32_t* kalt = reinterpret_cast<uint32_t*>(base + kKeysOffset);
     int32_t* valt = reinterpret_cast<int32_t*>(base + kValsOffset);
@@ -150,20 +143,15 @@ extern "C" int sph_sort_pairs_noalloc(const uint32_t* d_keys_in, const int32_t* 
         cudaGetLastError();
         return SPH_E_CUDA;
     }
-    sph::k_sort_hist<<<2 * sms, kCtaThreads, 0, s>>>(d_keys_in, n, passes, hist, nullptr);
     /* pass p writes the caller's output when (passes - 1 - p) is even, the copy otherwise,
      * so the last pass lands in the output and the input is never written */
-    const uint32_t* ki = d_keys_in;
-    const int32_t* vi = d_vals_in;
+    sph::SortBufs b{d_keys_in, d_vals_in, {}, {}};
     for (int p = 0; p < passes; ++p) {
         const bool to_out = ((passes - 1 - p) % 2) == 0;
-        uint32_t* ko = to_out ? d_keys_out : kalt;
-        int32_t* vo = to_out ? d_vals_out : valt;
-        sph::k_onesweep<<<tiles, kCtaThreads, 0, s>>>(ki, vi, ko, vo, n, 8 * p, p, tiles, hist, counters, status,
-                                                      flags, nullptr);
-        ki = ko;
-        vi = vo;
+        b.k[p] = to_out ? d_keys_out : kalt;
+        b.v[p] = to_out ? d_vals_out : valt;
     }
+    sph::sort_launches(s, b, n, passes, hist, flags, nullptr, 2 * sms, tiles);
     if (cudaGetLastError() != cudaSuccess) {
         forget_scratch_for_current_device();
         return SPH_E_CUDA;
