@@ -479,7 +479,6 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
         if (pre[k] == SPH_S_BOUNDARY_SYNC && !(x->NB > 0 && x->any_movable)) continue;
         if (pre[k] == SPH_S_HASHES) {
             /* the hashes with the incremental sort's first pass */
-            sph::sort_inc_begin(s, b.inc_ws, x->N);
             sph::launch_hashes_flags(s, c, b.pos, x->N, b.keys, b.tab, b.cell_prev, b.flags, b.scenes, b.scene_of,
                                      sph::sort_inc_flags_args(b.inc_ws, x->N));
             x->cur_keys = b.keys;
@@ -500,7 +499,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
     float4* const vh = x->p.method == SPH_WCSPH ? b.vhalf : nullptr;
     sph::launch_gather_ranges(s, c, x->N, b.mask_sorted, b.pos, b.pos_s, late_vel ? nullptr : b.vel, b.vel_s,
                               late_vel ? nullptr : vh, b.vhalf_s, b.ids, b.ids_s, b.keys_sorted, b.tab, b.cell_prev,
-                              b.flags, bs, b.scenes, b.scene_of);
+                              b.flags, bs, b.scenes, b.scene_of, sph::sort_inc_keep_args(b.inc_ws, x->N));
     mark(x, "k_gather_ranges");
     /* the velocities' part of the gather, once they have arrived (after the list pass) */
     auto gather_vel = [&]() {

@@ -85,8 +85,8 @@ void sort_pairs(cudaStream_t s, uint32_t* k0, int32_t* v0, uint32_t* k1, int32_t
  * sort_pairs over (keys, identity) for every input.  side / fork / join (all or none): a
  * second stream and two events on which the gated full sort runs beside the merge. */
 size_t sort_inc_workspace_bytes(int n);
-/* The incremental sort's first pass fused into the step's hash kernel: the sort then starts
- * with sort_inc_begin (before the hash kernel) and skips that pass (flags_done). */
+/* The step runs the incremental sort's first pass in its hash kernel and its last one in its
+ * gather kernel (in_step). */
 constexpr int kIncItems = 8;
 constexpr int kIncTile = 256 * kIncItems;
 struct IncFlags {
@@ -99,11 +99,27 @@ struct IncFlags {
     uint32_t* lcount;
 };
 IncFlags sort_inc_flags_args(void* inc_ws, int n);
-void sort_inc_begin(cudaStream_t s, void* inc_ws, int n);
+struct IncKeep {
+    const unsigned* opened;   /* 1: the full sort ran, so the previous keys are to be kept */
+    unsigned *over, *valid;
+    uint32_t *prev, *first, *sub;
+    __device__ __forceinline__ void keep(int j, uint32_t key) const {
+        if (j == 0) {
+            *over = 0u;
+            *valid = 1u;
+        }
+        if (*opened != 0u) {
+            prev[j] = key;
+            if ((j & 31) == 0) sub[j >> 5] = key;
+            if ((j & (kIncTile - 1)) == 0) first[j / kIncTile] = key;
+        }
+    }
+};
+IncKeep sort_inc_keep_args(void* inc_ws, int n);
 void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key_bits, uint32_t* kout,
                             int32_t* vout, void* inc_ws, void* sort_ws, unsigned* flags, int num_sms,
                             cudaStream_t side = nullptr, cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr,
-                            bool flags_done = false);
+                            bool in_step = false);
 
 /* sph_grid.cu */
 /* scenes: the context's scene table (never null); scene_of: scene of each particle, or
@@ -117,7 +133,7 @@ void launch_hashes_flags(cudaStream_t s, const Const& c, const float4* pos, int 
 void launch_gather_ranges(cudaStream_t s, const Const& c, int n, const int32_t* perm, const float4* a, float4* as,
                           const float4* b, float4* bs_, const float4* c3, float4* cs, const int32_t* ids,
                           int32_t* ids_s, const uint32_t* keys, int2* tab, int32_t* cell_out, unsigned* flags, int bs,
-                          const SceneDev* scenes, const int32_t* scene_of);
+                          const SceneDev* scenes, const int32_t* scene_of, const IncKeep& inc);
 void launch_gather(cudaStream_t s, int n, const int32_t* perm, const float4* a, float4* as, const float4* b,
                    float4* bs_, const float4* c3, float4* cs, const int32_t* ids, int32_t* ids_s, int bs);
 void launch_gather_boundary(cudaStream_t s, int n, const int32_t* perm, const float4* pos, float4* pos_s,

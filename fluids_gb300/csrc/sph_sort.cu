@@ -478,7 +478,8 @@ void sort_pairs(cudaStream_t s, uint32_t* k0, int32_t* v0, uint32_t* k1, int32_t
  *                particles of the buckets below t) + its rank, a stayed particle of stayed
  *                rank a to a + (moved particles of the buckets below t) + (bucket particles
  *                below it).
- *   k_inc_keep   after an overflow, keeps the full sort's keys as prev; marks prev valid.
+ *   k_inc_keep   after an overflow, keeps the full sort's keys as prev; marks prev valid (in
+ *                the step, k_gather_ranges does).
  * A bucket holds kIncBucket particles.  When one overflows, when more than a sixth of the
  * particles moved (their searches would cost more than a full sort), or when there is no
  * previous result (the first call), the overflow word opens the gated full onesweep sort of
@@ -494,8 +495,8 @@ constexpr int kIncWords = kIncTile / 32;
 constexpr int kIncBucket = 1024;                 /* moved particles per merge tile before overflow */
 
 struct IncLayout {
-    size_t valid, prev, first, sub, bits, list, store, zero, over, lcount, done, bcnt, tcnt, tpre, boff, vscr, total,
-        zero_bytes;
+    size_t valid, opened, prev, first, sub, bits, list, store, zero, over, lcount, done, bcnt, tcnt, tpre, boff, vscr,
+        total, zero_bytes;
     int tiles, words;
     IncLayout(int n) {
         const size_t nn = (size_t)(n > 0 ? n : 1);
@@ -508,14 +509,16 @@ struct IncLayout {
             return at;
         };
         valid = take(4);
+        opened = take(4);                  /* the overflow word as the merge found it, for the pass after it */
         prev = take(4 * nn);
         first = take(4 * (size_t)tiles);   /* prev at each tile's first position */
         sub = take(4 * (size_t)words);     /* prev at each word's first position */
         bits = take(4 * (size_t)words);
         list = take(8 * nn);
         store = take(16 * (size_t)tiles * kIncBucket);
-        /* zeroed by every call: the overflow word, the list length, the count of finished
-         * placing CTAs and the bucket counts (the other arrays are written whole) */
+        /* zero before every call: the overflow word, the list length, the count of finished
+         * placing CTAs and the bucket counts (the other arrays are written whole); each call
+         * leaves them zero (the merge, and for the overflow word the pass after it) */
         zero_bytes = 4 * (3 + (size_t)tiles);
         zero = take(zero_bytes);
         over = zero;
@@ -712,12 +715,13 @@ __global__ void __launch_bounds__(kThreads) k_inc_merge(const uint32_t* __restri
                                                         const uint32_t* __restrict__ tcnt,
                                                         const uint32_t* __restrict__ tpre,
                                                         const uint32_t* __restrict__ boff,
-                                                        const uint32_t* __restrict__ bcnt,
+                                                        uint32_t* __restrict__ bcnt,
                                                         const int4* __restrict__ store,
                                                         const unsigned* __restrict__ over,
-                                                        uint32_t* __restrict__ kout, int32_t* __restrict__ vout,
-                                                        uint32_t* __restrict__ prev, uint32_t* __restrict__ first,
-                                                        uint32_t* __restrict__ sub) {
+                                                        unsigned* __restrict__ opened, uint32_t* __restrict__ lcount,
+                                                        unsigned* __restrict__ done, uint32_t* __restrict__ kout,
+                                                        int32_t* __restrict__ vout, uint32_t* __restrict__ prev,
+                                                        uint32_t* __restrict__ first, uint32_t* __restrict__ sub) {
     __shared__ uint32_t s_k[kIncBucket], s_gk[kIncBucket];
     __shared__ int32_t s_i[kIncBucket], s_p[kIncBucket], s_g[kIncBucket], s_gi[kIncBucket];
     __shared__ uint32_t s_at[kIncTile + 1];   /* bucket particles inserted at each position */
@@ -727,7 +731,20 @@ __global__ void __launch_bounds__(kThreads) k_inc_merge(const uint32_t* __restri
     const int t = blockIdx.x;
     const int tbase = t << kIncShift;
     const int tlen = min(kIncTile, n - tbase);
-    if (*over != 0u) return;   /* the gated full sort writes the result */
+    const bool full = *over != 0u;
+    if (t == 0 && tid == 0) {
+        *opened = full ? 1u : 0u;
+        *lcount = 0u;
+        *done = 0u;
+    }
+    if (full) {   /* the gated full sort writes the result (of more than one pair) */
+        if (tid == 0) bcnt[t] = 0u;
+        if (n == 1 && tid == 0) {
+            kout[0] = __ldg(&keys[0]);
+            vout[0] = 0;
+        }
+        return;
+    }
     /* this tile's keys and moved words first (their loads in flight together) */
     const int wbase = warp * (32 * kIncItems);   /* tile-local */
     uint32_t key[kIncItems], word[kIncItems];
@@ -738,7 +755,7 @@ __global__ void __launch_bounds__(kThreads) k_inc_merge(const uint32_t* __restri
         word[k] = wbase + k * 32 < tlen ? __ldg(&bits[(tbase + wbase + k * 32) >> 5]) : 0u;
     }
     const uint32_t tile_pre = __ldg(&tpre[t]), off = __ldg(&boff[t]), tile_moved = __ldg(&tcnt[t]);
-    const int c = min((int)__ldg(&bcnt[t]), kIncBucket);   /* no overflow: at most kIncBucket */
+    const int c = min((int)bcnt[t], kIncBucket);   /* no overflow: at most kIncBucket */
 #pragma unroll
     for (int k = 0; k < kIncItems; ++k) s_at[tid * kIncItems + k] = 0u;
     if (tid == 0) s_at[kIncTile] = 0u;
@@ -747,6 +764,7 @@ __global__ void __launch_bounds__(kThreads) k_inc_merge(const uint32_t* __restri
     for (int k = 0; k < kIncItems; ++k) wc += (uint32_t)__popc(word[k]);
     if (lane == 0) s_wpre[warp] = wc;   /* per-warp totals, scanned below */
     __syncthreads();
+    if (tid == 0) bcnt[t] = 0u;   /* every thread of the tile's block has read it */
     for (int e = tid; e < c; e += kThreads) {
         const int4 v = __ldg(&store[(size_t)t * kIncBucket + e]);
         s_k[e] = (uint32_t)v.x;
@@ -827,25 +845,11 @@ __global__ void __launch_bounds__(kThreads) k_inc_merge(const uint32_t* __restri
     }
 }
 
-/* After the gated full sort: its keys become prev (with the word and tile tables); a
- * single pair needs no sort.  Marks prev valid for the next call either way. */
-__global__ void __launch_bounds__(kThreads) k_inc_keep(const uint32_t* __restrict__ keys, int n,
-                                                       const unsigned* __restrict__ over, uint32_t* __restrict__ kout,
-                                                       int32_t* __restrict__ vout, uint32_t* __restrict__ prev,
-                                                       uint32_t* __restrict__ first, uint32_t* __restrict__ sub,
-                                                       unsigned* __restrict__ valid) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *valid = 1u;
-    if (*over == 0u) return;
-    if (n == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
-        kout[0] = __ldg(&keys[0]);
-        vout[0] = 0;
-    }
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
-        const uint32_t k = n == 1 ? __ldg(&keys[0]) : kout[j];
-        prev[j] = k;
-        if ((j & 31) == 0) sub[j >> 5] = k;
-        if ((j & (kIncTile - 1)) == 0) first[j >> kIncShift] = k;
-    }
+/* After the gated full sort: its keys become prev (with the word and tile tables).  Marks prev
+ * valid for the next call either way.  The step does this in k_gather_ranges. */
+__global__ void __launch_bounds__(kThreads) k_inc_keep(int n, const uint32_t* __restrict__ kout, IncKeep inc) {
+    const int j = blockIdx.x * kThreads + threadIdx.x;
+    if (j < n) inc.keep(j, kout[j]);
 }
 
 size_t sort_inc_workspace_bytes(int n) { return IncLayout(n).total; }
@@ -859,14 +863,17 @@ IncFlags sort_inc_flags_args(void* inc_ws, int n) {
                     reinterpret_cast<uint32_t*>(w + L.lcount)};
 }
 
-void sort_inc_begin(cudaStream_t s, void* inc_ws, int n) {
+IncKeep sort_inc_keep_args(void* inc_ws, int n) {
     const IncLayout L(n);
-    cudaMemsetAsync(static_cast<char*>(inc_ws) + L.zero, 0, L.zero_bytes, s);
+    char* w = static_cast<char*>(inc_ws);
+    return IncKeep{reinterpret_cast<const unsigned*>(w + L.opened), reinterpret_cast<unsigned*>(w + L.over),
+                   reinterpret_cast<unsigned*>(w + L.valid),        reinterpret_cast<uint32_t*>(w + L.prev),
+                   reinterpret_cast<uint32_t*>(w + L.first),        reinterpret_cast<uint32_t*>(w + L.sub)};
 }
 
 void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key_bits, uint32_t* kout,
                             int32_t* vout, void* inc_ws, void* sort_ws, unsigned* flags, int num_sms,
-                            cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, bool flags_done) {
+                            cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, bool in_step) {
     if (n <= 0) return;
     const IncLayout L(n);
     char* w = static_cast<char*>(inc_ws);
@@ -884,8 +891,7 @@ void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key
     int2* list = reinterpret_cast<int2*>(w + L.list);
     uint32_t* lcount = reinterpret_cast<uint32_t*>(w + L.lcount);
     unsigned* done = reinterpret_cast<unsigned*>(w + L.done);
-    if (!flags_done) {
-        cudaMemsetAsync(w + L.zero, 0, L.zero_bytes, s);
+    if (!in_step) {
         k_inc_flags<<<L.tiles, kThreads, 0, s>>>(keys, prev, n, valid, bits, tcnt, over, list, lcount);
     }
     const size_t fsm = L.tiles <= kIncSmemTiles ? 4 * (size_t)L.tiles : 0;
@@ -908,10 +914,11 @@ void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key
                           flags, num_sms);
     }
     if (fork_side) cudaEventRecord(join, side);
-    k_inc_merge<<<L.tiles, kThreads, 0, s>>>(keys, n, bits, tcnt, tpre, boff, bcnt, store, over, kout, vout, prev,
-                                             first, sub);
+    k_inc_merge<<<L.tiles, kThreads, 0, s>>>(keys, n, bits, tcnt, tpre, boff, bcnt, store, over,
+                                             reinterpret_cast<unsigned*>(w + L.opened), lcount, done, kout, vout,
+                                             prev, first, sub);
     if (fork_side) cudaStreamWaitEvent(s, join, 0);
-    k_inc_keep<<<2 * num_sms, kThreads, 0, s>>>(keys, n, over, kout, vout, prev, first, sub, valid);
+    if (!in_step) k_inc_keep<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, kout, sort_inc_keep_args(inc_ws, n));
 }
 
 }  // namespace sph
