@@ -141,6 +141,14 @@ __device__ __forceinline__ long long scene_setup_t(Const& c, const SceneDev* sce
     else return 0;
 }
 
+/* First statement of a kernel of the step's chain: lets the next kernel's blocks be set up, and
+ * waits until the kernel before it has finished and its writes are visible (at once when it was
+ * not launched by launch_chained). */
+__device__ __forceinline__ void chain_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr unsigned kFlagNan = 1u, kFlagEscaped = 2u, kFlagTimeout = 4u, kFlagOverflow = 8u,
                    kFlagNonconverged = 16u;
 

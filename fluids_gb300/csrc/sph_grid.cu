@@ -54,16 +54,21 @@ __global__ void k_hashes(Const c0, const float4* __restrict__ pos, int n, uint32
 }
 
 /* k_hashes of the fused step with the incremental sort's first pass (k_inc_flags of
- * sph_sort.cu) on the keys it computes: tiles of kIncTile particles, kIncItems a thread. */
-__global__ void __launch_bounds__(256) k_hashes_flags(Const c0, const float4* __restrict__ pos, int n,
+ * sph_sort.cu) on the keys it computes: tiles of kIncTile particles, a block each. */
+/* particles a thread: the divisions of a thread's particles are a serial chain; a step of 2,197
+ * particles 39.6, 38.9 and 37.8 us with 8, 4 and 2, of 1,000,000 503.4, 501.7 and 501.3 */
+constexpr int kHashItems = 2;
+constexpr int kHashThreads = kIncTile / kHashItems;
+__global__ void __launch_bounds__(kHashThreads) k_hashes_flags(Const c0, const float4* __restrict__ pos, int n,
                                                       uint32_t* __restrict__ keys, int2* __restrict__ tab,
                                                       const int32_t* __restrict__ cell_prev,
                                                       unsigned* __restrict__ flags,
                                                       const SceneDev* __restrict__ scenes,
                                                       const int32_t* __restrict__ scene_of, IncFlags inc) {
-    constexpr int kItems = kIncItems;
-    __shared__ uint32_t s_wcnt[8];
+    constexpr int kItems = kHashItems;
+    __shared__ uint32_t s_wcnt[kHashThreads / 32];
     __shared__ uint32_t s_base;
+    chain_next();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wbase = ((int)blockIdx.x * kIncTile) + warp * (32 * kItems);   /* n < 2^31 */
     const bool have_prev = *inc.valid != 0u;
@@ -97,7 +102,7 @@ __global__ void __launch_bounds__(256) k_hashes_flags(Const c0, const float4* __
     if (tid == 0) {
         uint32_t total = 0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) total += s_wcnt[w];
+        for (int w = 0; w < kHashThreads / 32; ++w) total += s_wcnt[w];
         inc.tcnt[blockIdx.x] = total;
         s_base = have_prev && total ? atomicAdd(inc.lcount, total) : 0u;
     }
@@ -185,6 +190,7 @@ __global__ void k_gather_ranges(Const c, int n, const int32_t* __restrict__ perm
                                 int32_t* __restrict__ cell_out, unsigned* __restrict__ flags,
                                 const SceneDev* __restrict__ scenes, const int32_t* __restrict__ scene_of,
                                 IncKeep inc) {
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int src = __ldg(&perm[i]);
@@ -258,7 +264,7 @@ void launch_hashes_flags(cudaStream_t s, const Const& c, const float4* pos, int 
                          const int32_t* cell_prev, unsigned* flags, const SceneDev* scenes, const int32_t* scene_of,
                          const IncFlags& inc) {
     if (n <= 0) return;
-    k_hashes_flags<<<blocks_for(n, kIncTile), 256, 0, s>>>(c, pos, n, keys, tab, cell_prev, flags, scenes, scene_of,
+    k_hashes_flags<<<blocks_for(n, kIncTile), kHashThreads, 0, s>>>(c, pos, n, keys, tab, cell_prev, flags, scenes, scene_of,
                                                            inc);
 }
 void launch_gather(cudaStream_t s, int n, const int32_t* perm, const float4* a, float4* as, const float4* b,

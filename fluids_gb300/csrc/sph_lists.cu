@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kSplitThreads)
                   float4* __restrict__ prho) {
     extern __shared__ float2 s_term[];   /* per particle: cap entries, padded to an odd number */
     __shared__ int2 s_rng[kPer][27];
+    chain_next();
     const int g = threadIdx.x & (kLanes - 1), slot = threadIdx.x / kLanes;
     const int i = blockIdx.x * kPer + slot;
     const bool live = i < c0.n;
@@ -184,10 +185,10 @@ constexpr int kMaxCap = 128;
 
 template <bool BATCH, bool REMAP, bool PCI>
 static void split_launch(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap) {
-    k_lists_split<BATCH, REMAP, PCI>
-        <<<(c.n + kPer - 1) / kPer, kSplitThreads, sizeof(float2) * kPer * (size_t)(c.cap | 1), s>>>(
-            c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
-            b.aux, b.scenes, b.scene_of, remap, b.flags, b.bnear, b.prho);
+    launch_chained(s, k_lists_split<BATCH, REMAP, PCI>, (c.n + kPer - 1) / kPer, kSplitThreads,
+                   sizeof(float2) * kPer * (size_t)(c.cap | 1), c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist,
+                   b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes, b.scene_of, remap, b.flags,
+                   b.bnear, b.prho);
 }
 
 bool launch_lists_split(cudaStream_t s, const Const& c, const Bufs& b, bool pci, const int32_t* remap, int num_sms) {

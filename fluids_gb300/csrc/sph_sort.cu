@@ -605,6 +605,7 @@ __global__ void __launch_bounds__(kThreads) k_inc_place(const int2* __restrict__
     extern __shared__ uint32_t s_first[];   /* min(tiles, kIncSmemTiles) entries */
     __shared__ uint32_t s_scan[kWarps];
     __shared__ bool s_last;
+    chain_next();
     if (*valid == 0u) return;   /* no previous result: the full sort runs */
     const int m = (int)*lcount;
     if (m > n / 6) {
@@ -731,6 +732,7 @@ __global__ void __launch_bounds__(kThreads) k_inc_merge(const uint32_t* __restri
     const int t = blockIdx.x;
     const int tbase = t << kIncShift;
     const int tlen = min(kIncTile, n - tbase);
+    chain_next();
     const bool full = *over != 0u;
     if (t == 0 && tid == 0) {
         *opened = full ? 1u : 0u;
@@ -895,8 +897,10 @@ void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key
         k_inc_flags<<<L.tiles, kThreads, 0, s>>>(keys, prev, n, valid, bits, tcnt, over, list, lcount);
     }
     const size_t fsm = L.tiles <= kIncSmemTiles ? 4 * (size_t)L.tiles : 0;
-    k_inc_place<<<4 * num_sms, kThreads, fsm, s>>>(list, lcount, prev, first, sub, n, L.tiles, valid, bcnt, store,
-                                                   over, done, tcnt, tpre, boff);
+    /* at most a sixth of the particles is placed, a thread each */
+    const int pblocks = max(1, min(4 * num_sms, (n / 6 + kThreads - 1) / kThreads));
+    launch_chained(s, k_inc_place, pblocks, kThreads, fsm, list, lcount, prev, first, sub, n, L.tiles, valid, bcnt,
+                   store, over, done, tcnt, tpre, boff);
     /* the gated full sort of (keys, identity) on the side stream, beside the merge (one of
      * the two writes the result); prev is its scratch and its last pass writes kout / vout */
     const bool fork_side = side != nullptr && fork != nullptr && join != nullptr;
@@ -914,9 +918,8 @@ void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key
                           flags, num_sms);
     }
     if (fork_side) cudaEventRecord(join, side);
-    k_inc_merge<<<L.tiles, kThreads, 0, s>>>(keys, n, bits, tcnt, tpre, boff, bcnt, store, over,
-                                             reinterpret_cast<unsigned*>(w + L.opened), lcount, done, kout, vout,
-                                             prev, first, sub);
+    launch_chained(s, k_inc_merge, L.tiles, kThreads, 0, keys, n, bits, tcnt, tpre, boff, bcnt, store, over,
+                   reinterpret_cast<unsigned*>(w + L.opened), lcount, done, kout, vout, prev, first, sub);
     if (fork_side) cudaStreamWaitEvent(s, join, 0);
     if (!in_step) k_inc_keep<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, kout, sort_inc_keep_args(inc_ws, n));
 }

@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
                                                        const uint8_t* __restrict__ bnear = nullptr,
                                                        const int32_t* __restrict__ noff = nullptr,
                                                        float4* __restrict__ prho = nullptr) {
+  chain_next();
   for_each_particle<BATCH>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
     const int2* __restrict__ ftab = tab0 + base;
     const int2* __restrict__ fbtab = btab0 + base;
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl
                                                  const SceneTile* __restrict__ tiles, unsigned* next,
                                                  const float4* __restrict__ vel_s = nullptr,
                                                  float4* __restrict__ nrec = nullptr) {
+  chain_next();
   for_each_particle<BATCH, W>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
     Neigh<LIST, EXACT> fl = fl0;
     fl.tab += base;
@@ -291,6 +293,7 @@ __device__ __forceinline__ void wc_integrate_one(const Const& c, float4 p, float
  * factor 2 rho0 / (rho_i + rho_j) = 2 rho0 R_j / (rho_i R_j + 1). */
 template <bool COMPAT, bool LIST, bool FUSE, bool WRITE_ACC, bool ST, bool BATCH, bool PACK = false, int W = 1>
 __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const c0, Neigh<LIST, COMPAT> fl0, Neigh<LIST, COMPAT> bl0, Bufs b) {
+  chain_next();
   for_each_particle<BATCH, W>(c0, b.tiles, b.scenes, b.tile_next + 3, [&](const Const& c, long long base, int i) {
     const int w = W > 1 ? lane_of_particle<W>(c) : 0;
     Neigh<LIST, COMPAT> fl = fl0, bl = bl0;
@@ -531,8 +534,8 @@ static void normals_split(cudaStream_t s, const Const& c0, const Bufs& b, float4
     c.last = c.n;
     auto fl = fluid_src<true, true>(b);
     fl.npos = b.prho;
-    k_normals<true, true, false, false, true, W><<<nblk(c.n * W, 256), 256, 0, s>>>(
-        c, fl, b.aux, b.density, b.normal, b.scenes, b.tiles, nullptr, b.vel_s, nrec);
+    launch_chained(s, k_normals<true, true, false, false, true, W>, nblk(c.n * W, 256), 256, 0, c, fl, b.aux,
+                   b.density, b.normal, b.scenes, b.tiles, nullptr, b.vel_s, nrec);
 }
 
 void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack, bool prho) {
@@ -595,8 +598,8 @@ static void forces_split(cudaStream_t s, const Const& c0, const Bufs& b, int bs,
     auto fs = fluid_src<true, false>(b);
     auto bsrc = bnd_src<true, false>(b);
     const int g = nblk((c.last - c.first) * W, 256);
-    if (st) k_wc_forces<false, true, true, false, true, false, true, W><<<g, 256, 0, s>>>(c, fs, bsrc, b);
-    else k_wc_forces<false, true, true, false, false, false, false, W><<<g, 256, 0, s>>>(c, fs, bsrc, b);
+    if (st) launch_chained(s, k_wc_forces<false, true, true, false, true, false, true, W>, g, 256, 0, c, fs, bsrc, b);
+    else launch_chained(s, k_wc_forces<false, true, true, false, false, false, false, W>, g, 256, 0, c, fs, bsrc, b);
 }
 
 template <bool COMPAT, bool LIST, bool BATCH>
