@@ -409,7 +409,7 @@ int run_stage_impl(sph_ctx* x, int stage) {
     case SPH_S_PCI_LOOP: {
         cudaMemsetAsync(b.pci_maxerr, 0, sizeof(float) * x->max_iter_slots, s);
         cudaMemsetAsync(b.barrier, 0, 4 * sizeof(unsigned), s);
-        cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, c.pci_max_iter, x->coop_blocks, bs, false);
+        cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, c.pci_max_iter, x->coop_blocks, x->num_sms, false);
         if (e != cudaSuccess) return cuda_fail(x, e, "cooperative launch of the PCISPH loop");
         break;
     }
@@ -577,7 +577,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
         cudaMemsetAsync(b.pci_maxerr, 0, sizeof(float) * x->max_iter_slots, s);
         cudaMemsetAsync(b.barrier, 0, 4 * sizeof(unsigned), s);
         if (x->any_massive) {
-            cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, pci_max_iter, x->coop_blocks, bs, false);
+            cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, pci_max_iter, x->coop_blocks, x->num_sms, false);
             if (e != cudaSuccess) return cuda_fail(x, e, "cooperative launch of the PCISPH loop");
             mark(x, "k_pci_loop");
             sph::launch_bnd_forces(s, c, b, (int)x->bodies.size(), bs);
@@ -586,7 +586,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
             sph::launch_pci_integrate(s, c, b, bs);
             mark(x, "k_pci_integrate");
         } else {
-            cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, pci_max_iter, x->coop_blocks, bs, true);
+            cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, pci_max_iter, x->coop_blocks, x->num_sms, true);
             if (e != cudaSuccess) return cuda_fail(x, e, "cooperative launch of the PCISPH loop");
             mark(x, "k_pci_loop");
         }

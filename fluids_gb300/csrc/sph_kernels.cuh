@@ -192,7 +192,7 @@ void launch_pci_init_density(cudaStream_t s, const Const& c, const Bufs& b, int 
 void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms, bool pack = false);
 int pci_loop_blocks(int num_sms, int bs);
 cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter, int blocks,
-                            int bs, bool fuse_integrate);
+                            int num_sms, bool fuse_integrate);
 void launch_pci_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_pci_predict(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_pci_update_pressure(cudaStream_t s, const Const& c, const Bufs& b, int bs);

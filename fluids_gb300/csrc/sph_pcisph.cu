@@ -120,8 +120,11 @@ __device__ __forceinline__ void walk_list(const int* __restrict__ e, size_t n, i
             if (k + u < len) visit(q[u]);
     }
 }
-template <bool COMPAT>
-__device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, int i) {
+/* W > 1: W lanes of a particle (small scenes, PHYSICS): each forms the terms of entries w, w +
+ * W, ..., and all add them in list order, so the sum is that of one thread.  w >= W: a lane
+ * without a particle, which only takes part in the exchange. */
+template <bool COMPAT, int W = 1>
+__device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, int i, int w = 0) {
     const float4 pi = b.pos_pred[i];
     const float H = c.h_def, HH = H * H;
     const size_t n = (size_t)c.n;
@@ -142,10 +145,46 @@ __device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, i
             pd = __fadd_rn(pd, __fmul_rn(__fmul_rn(t, t), t));
         }
     };
-    walk_list<SPH_PCI_WALK_DEPTH>(e, n, len, i, [&](int j) { return b.pos_pred[j]; }, visit);
-    pd *= c.default_eval * c.mass_def;
     const int blen = __ldg(&b.sblen[i]);
-    for (int k = 0; k < blen; ++k) {
+    if constexpr (W > 1) {
+        auto cube = [&](float4 pj) {
+            const float r2 = r2_exact(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z);
+            const float t = r2 < HH ? HH - r2 : 0.f;
+            return __fmul_rn(__fmul_rn(t, t), t);
+        };
+        const int most = __reduce_max_sync(0xffffffffu, w < W ? len : 0);
+        for (int k0 = 0; k0 < most; k0 += 4 * W) {
+            float term[4];
+            int j[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = k0 + u * W + w;
+                j[u] = w < W && k < len ? __ldg(e + k * n) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) term[u] = j[u] >= 0 ? cube(b.pos_pred[j[u]]) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < W; ++v) pd = __fadd_rn(pd, __shfl_sync(0xffffffffu, term[u], v, W));
+        }
+        const int bmost = __reduce_max_sync(0xffffffffu, w < W ? blen : 0);
+        for (int k0 = 0; k0 < bmost; k0 += W) {
+            const int k = k0 + w;
+            float term = 0.f;
+            if (w < W && k < blen) {
+                const int j = __ldg(&b.sblist[k * n + i]);
+                term = __fmul_rn(cube(__ldg(&b.bpos_s[j])), __ldg(&b.bphi_s[j]));
+            }
+#pragma unroll
+            for (int v = 0; v < W; ++v) pdb = __fadd_rn(pdb, __shfl_sync(0xffffffffu, term, v, W));
+        }
+        if (w != 0) return 0.f;
+    } else {
+        walk_list<SPH_PCI_WALK_DEPTH>(e, n, len, i, [&](int j) { return b.pos_pred[j]; }, visit);
+    }
+    pd *= c.default_eval * c.mass_def;
+    for (int k = 0; k < (W > 1 ? 0 : blen); ++k) {
         const int j = __ldg(&b.sblist[k * n + i]);
         const float4 pj = __ldg(&b.bpos_s[j]);
         const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
@@ -175,8 +214,9 @@ __device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, i
  * (p_i / rho_i^2 + p_j / rho_j^2) per pair with the quotients of pci_c; each neighbour's
  * position and quotient come as one record from pci_pc (both written by the update phase
  * of this kernel, so plain loads). */
-template <bool MON = false>
-__device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Bufs& b, int i) {
+/* W > 1: W lanes of a particle, their sums added (w >= W as in pci_update_one). */
+template <bool MON = false, int W = 1>
+__device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Bufs& b, int i, int w = 0) {
     const float4 pi = __ldg(&b.pos_s[i]);
     const float H = c.h_def;
     const size_t n = (size_t)c.n;
@@ -209,12 +249,25 @@ __device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Buf
         fy += q * ((dy * il) * t);
         fz += q * ((dz * il) * t);
     };
-    walk_list<SPH_PCI_WALK_DEPTH>(e, n, len, i, [&](int j) { return b.pci_pc[j]; },
-                                  [&](const float4& v) { visit(v, v.w); });
+    if constexpr (W > 1) {
+        for (int k0 = w; k0 < (w < W ? len : 0); k0 += 4 * W) {
+            int j[4];
+            float4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) j[u] = k0 + u * W < len ? __ldg(e + (k0 + u * W) * n) : i;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) q[u] = b.pci_pc[j[u]];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) visit(q[u], q[u].w);   /* the particle itself adds zeros */
+        }
+    } else {
+        walk_list<SPH_PCI_WALK_DEPTH>(e, n, len, i, [&](int j) { return b.pci_pc[j]; },
+                                      [&](const float4& v) { visit(v, v.w); });
+    }
     const float sf = (-(c.mass_def * c.mass_def)) * c.spiky_grad;
     fx *= sf; fy *= sf; fz *= sf;
     const int blen = __ldg(&b.sblen[i]);
-    for (int k = 0; k < blen; ++k) {
+    for (int k = w; k < (w < W ? blen : 0); k += W) {
         const int j = __ldg(&b.sblist[k * n + i]);
         const float4 pj = __ldg(&b.bpos_s[j]);
         const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
@@ -234,6 +287,13 @@ __device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Buf
         gz += q * ((dz * il) * t);
     }
     const float sb = (-c.mass_def) * c.spiky_grad;
+    if constexpr (W > 1) {
+        fx = sum_lanes<W>(fx + gx * sb);
+        fy = sum_lanes<W>(fy + gy * sb);
+        fz = sum_lanes<W>(fz + gz * sb);
+        if (w == 0) b.f_press[i] = make_float4(fx, fy, fz, 0.f);
+        return;
+    }
     b.f_press[i] = make_float4(fx + gx * sb, fy + gy * sb, fz + gz * sb, 0.f);
 }
 }  // namespace
@@ -366,17 +426,26 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
 #define SPH_PCI_LOOP_THREADS 256
 #endif
 constexpr int kLoopThreads = SPH_PCI_LOOP_THREADS;
-template <bool COMPAT, bool FUSE_INTEGRATE>
+/* W lanes a particle in small scenes (walk_lanes): with one, a loop of 9,177 particles ran on 36
+ * SMs; measured on GB300, its three iterations 79 -> 45 us. */
+template <bool COMPAT, bool FUSE_INTEGRATE, int W = 1>
 __global__ void __launch_bounds__(kLoopThreads, SPH_PCI_LOOP_MIN_BLOCKS) k_pci_loop(Const c, Bufs b, int min_iter, int max_iter) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
     const int n = c.n;
+    /* the walks: W threads a particle, whole warps */
+    const int walks = W > 1 ? (n * W + 31) & ~31 : n;
+    auto lane_of = [&](int t) { return W > 1 ? (t / W < n ? t & (W - 1) : W) : 0; };
+    auto particle = [&](int t) { return W > 1 ? min(t / W, n - 1) : t; };
     int it = 1;
     for (; it <= max_iter; ++it) {
-        for (int i = tid; i < n; i += stride) pci_predict_one(c, b, i);
+        /* a particle's lane 0 predicts it: the force it reads is its own write */
+        for (int t = tid; t < walks; t += stride)
+            if (lane_of(t) == 0) pci_predict_one(c, b, particle(t));
         if (!grid_barrier(b.barrier, b.flags, (unsigned)c.barrier_extra)) return;
         float lmax = 0.f;
-        for (int i = tid; i < n; i += stride) lmax = fmaxf(lmax, pci_update_one<COMPAT>(c, b, i));
+        for (int t = tid; t < walks; t += stride)
+            lmax = fmaxf(lmax, pci_update_one<COMPAT, W>(c, b, particle(t), lane_of(t)));
         lmax = block_max(lmax);
         if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned*>(&b.pci_maxerr[it - 1]), __float_as_uint(lmax));
         if (!grid_barrier(b.barrier, b.flags, (unsigned)c.barrier_extra)) return;
@@ -384,7 +453,8 @@ __global__ void __launch_bounds__(kLoopThreads, SPH_PCI_LOOP_MIN_BLOCKS) k_pci_l
         if (COMPAT && c.monaghan) {
             for (int i = tid; i < n; i += stride) pci_pressure_force_one<true>(c, b, i);
         } else {
-            for (int i = tid; i < n; i += stride) pci_pressure_force_one(c, b, i);
+            for (int t = tid; t < walks; t += stride)
+                pci_pressure_force_one<false, W>(c, b, particle(t), lane_of(t));
         }
         bool stop = false;
         if (it >= min_iter) {
@@ -398,7 +468,8 @@ __global__ void __launch_bounds__(kLoopThreads, SPH_PCI_LOOP_MIN_BLOCKS) k_pci_l
         if (it > max_iter && !COMPAT) atomicOr(b.flags, kFlagNonconverged);
     }
     if (FUSE_INTEGRATE) {
-        for (int i = tid; i < n; i += stride) pci_integrate_one(c, b, i);
+        for (int t = tid; t < walks; t += stride)
+            if (lane_of(t) == 0) pci_integrate_one(c, b, particle(t));
     }
 }
 
@@ -480,7 +551,11 @@ void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int b
     else k_pci_init_forces<false><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
 }
 
-static void* loop_fn(bool compat, bool fuse) {
+static void* loop_fn(bool compat, bool fuse, int w) {
+    if (compat) w = 1;
+    if (w == 8) return fuse ? (void*)k_pci_loop<false, true, 8> : (void*)k_pci_loop<false, false, 8>;
+    if (w == 4) return fuse ? (void*)k_pci_loop<false, true, 4> : (void*)k_pci_loop<false, false, 4>;
+    if (w == 2) return fuse ? (void*)k_pci_loop<false, true, 2> : (void*)k_pci_loop<false, false, 2>;
     if (compat) return fuse ? (void*)k_pci_loop<true, true> : (void*)k_pci_loop<true, false>;
     return fuse ? (void*)k_pci_loop<false, true> : (void*)k_pci_loop<false, false>;
 }
@@ -488,26 +563,28 @@ static void* loop_fn(bool compat, bool fuse) {
 int pci_loop_blocks(int num_sms, int bs) {
     (void)bs;   /* the loop runs with its own block size */
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pci_loop<false, true>, kLoopThreads, 0);
-    int per_sm2 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_pci_loop<true, false>, kLoopThreads, 0);
-    per_sm = per_sm < per_sm2 ? per_sm : per_sm2;
+    for (int w = 1; w <= 8; w *= 2)
+        for (int k = 0; k < 4; ++k) {
+            int v = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, loop_fn((k & 1) != 0, (k & 2) != 0, w), kLoopThreads, 0);
+            per_sm = per_sm == 0 || v < per_sm ? v : per_sm;
+        }
     if (per_sm < 1) per_sm = 1;
     return per_sm * num_sms;
 }
 
 cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter, int blocks,
-                            int bs, bool fuse) {
+                            int num_sms, bool fuse) {
     if (c.n <= 0) return cudaSuccess;
-    (void)bs;
-    int need = nblk(c.n, kLoopThreads);
+    const int w = c.compat ? 1 : walk_lanes(c.n, num_sms);
+    int need = nblk(c.n * w, kLoopThreads);
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     Const cc = c;
     Bufs bb = b;
     int mi = min_iter, ma = max_iter;
     void* args[] = {&cc, &bb, &mi, &ma};
-    return cudaLaunchCooperativeKernel(loop_fn(c.compat != 0, fuse), dim3(blocks), dim3(kLoopThreads), args, 0, s);
+    return cudaLaunchCooperativeKernel(loop_fn(c.compat != 0, fuse, w), dim3(blocks), dim3(kLoopThreads), args, 0, s);
 }
 
 void launch_pci_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
