@@ -430,6 +430,15 @@ __device__ __forceinline__ int build_scan(const Const& c, float px, float py, fl
     return cnt;
 }
 
+/* Two adjacent float4 (32-byte aligned, read-only for the kernel) by one 256-bit load.  The
+ * gather of a neighbour's record is bound by the L1 data pipe, one cycle per distinct line of
+ * each 128 bytes a warp asks for. */
+__device__ __forceinline__ void load_pair(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
 /* Entry k of a column-major list row (row + k * n): one widening multiply-add on the entry
  * count instead of a 64-bit pointer advanced per candidate; n4 = 4 n bytes (n < 2^30). */
 __device__ __forceinline__ int* list_slot(char* row, int k, unsigned n4) {

@@ -364,8 +364,7 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
                        float rn, inv, w, K;
                        const float r2 = dx * dx + dy * dy + dz * dz;
                        if constexpr (PACK) {
-                           vj = __ldg(&b.nrec[2 * (size_t)j]);
-                           nj = __ldg(&b.nrec[2 * (size_t)j + 1]);
+                           load_pair(&b.nrec[2 * (size_t)j], vj, nj);
                            const float Rj = nj.w;
                            inv = r2 > 0.f ? rsqrtf(r2) : 0.f;
                            rn = r2 * inv;

@@ -339,8 +339,7 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
         /* loaded ahead of the guard so that the list loop can issue them early */
         float4 aj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
         if constexpr (PACK) {
-            vj = __ldg(&b.nrec[2 * (size_t)j]);
-            nj = __ldg(&b.nrec[2 * (size_t)j + 1]);
+            load_pair(&b.nrec[2 * (size_t)j], vj, nj);
             aj = make_float4(vj.w, nj.w, 1.0f, 0.f);   /* (C_j, R_j, -, -); the guard uses R_j > 0 */
         } else {
             aj = __ldg(&b.aux[j]);
