@@ -269,6 +269,7 @@ void carve(sph_ctx* x, Carver& cv) {
     b.body_range = cv.take<int32_t>(4 * nbod);
     b.body_force = cv.take<float4>(nbod); b.body_torque = cv.take<float4>(nbod);
     b.bft = cv.take<float4>(2 * nb);
+    b.bmass = cv.take<int32_t>(nb);
     b.body_dyn = cv.take<float>(8 * nbod);
     b.flags = cv.take<unsigned>(4);
     b.pci_iters = cv.take<int32_t>(4);
@@ -329,9 +330,8 @@ void drop_graph(sph_ctx* x) {
 }
 
 /* Sorts the boundary particles (boundaryhandler.cpp:216-236) and builds their cell table. */
-void boundary_sort(sph_ctx* x) {
+void boundary_sort(sph_ctx* x, cudaStream_t s) {
     Bufs& b = x->b;
-    const cudaStream_t s = x->stream;
     Const cb = x->c;
     /* batched: the boundary body of scene s is body s, so body ids are scene ids */
     sph::launch_hashes(s, cb, b.bpos, x->NB, b.bkeys, b.bmask, b.btab, b.bcell_prev, b.flags, x->bs, b.scenes,
@@ -345,6 +345,27 @@ void boundary_sort(sph_ctx* x) {
     sph::launch_bnd_near(s, cb, b, x->NB, x->bs);
 }
 
+/* The BOUNDARY_SYNC stage: movable bodies' particles to their new pose, all of them sorted. */
+void boundary_sync(sph_ctx* x, cudaStream_t s) {
+    sph::launch_bnd_transform(s, x->b, (int)x->bodies.size(), x->NB, x->c.compat != 0, true, x->bs);
+    boundary_sort(x, s);
+}
+
+/* Work of the step on the boundary's stream, after what is on the main stream now; the main
+ * stream waits for it at bnd_join.  On the main stream itself without the streams and while
+ * the step's parts are timed. */
+cudaStream_t bnd_fork(sph_ctx* x) {
+    if (!x->bnd_stream || x->prof) return x->stream;
+    cudaEventRecord(x->ev_bnd_fork, x->stream);
+    cudaStreamWaitEvent(x->bnd_stream, x->ev_bnd_fork, 0);
+    return x->bnd_stream;
+}
+void bnd_join(sph_ctx* x, cudaStream_t s) {
+    if (s == x->stream) return;
+    cudaEventRecord(x->ev_bnd_join, s);
+    cudaStreamWaitEvent(x->stream, x->ev_bnd_join, 0);
+}
+
 bool uses_lists(const sph_ctx* x) { return x->p.method == SPH_PCISPH || x->p.neighbor_mode == SPH_NEIGH_LIST; }
 
 int run_stage_impl(sph_ctx* x, int stage) {
@@ -355,8 +376,7 @@ int run_stage_impl(sph_ctx* x, int stage) {
     switch (stage) {
     case SPH_S_BOUNDARY_SYNC:
         if (x->NB > 0 && x->any_movable) {
-            sph::launch_bnd_transform(s, b, (int)x->bodies.size(), x->NB, c.compat != 0, true, bs);
-            boundary_sort(x);
+            boundary_sync(x, s);
         }
         break;
     case SPH_S_HASHES:
@@ -417,8 +437,7 @@ int run_stage_impl(sph_ctx* x, int stage) {
         sph::launch_pci_integrate(s, c, b, bs);
         break;
     case SPH_S_BOUNDARY_FORCES:
-        if (x->any_massive) sph::launch_bnd_forces(s, c, b, (int)x->bodies.size(), bs);
-        if (x->any_dynamic) sph::launch_body_integrate(s, c, b, (int)x->bodies.size());
+        if (x->any_massive) sph::launch_bnd_forces(s, c, b, (int)x->bodies.size(), x->nmass, x->any_dynamic, bs);
         break;
     case SPH_S_PCI_PREDICT:
     case SPH_S_PCI_UPDATE_PRESSURE:
@@ -471,29 +490,26 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
     const Const& c = x->c;
     const cudaStream_t s = x->stream;
     const int bs = x->bs;
-    int rc;
     mark(x, "start");
-    const int pre[] = {SPH_S_BOUNDARY_SYNC, SPH_S_HASHES, SPH_S_SORT};
-    const char* pre_names[] = {"boundary_sync", "k_hashes", "sort"};
-    for (int k = 0; k < 3; ++k) {
-        if (pre[k] == SPH_S_BOUNDARY_SYNC && !(x->NB > 0 && x->any_movable)) continue;
-        if (pre[k] == SPH_S_HASHES) {
-            /* the hashes with the incremental sort's first pass */
-            sph::launch_hashes_flags(s, c, b.pos, x->N, b.keys, b.tab, b.cell_prev, b.flags, b.scenes, b.scene_of,
-                                     sph::sort_inc_flags_args(b.inc_ws, x->N));
-            x->cur_keys = b.keys;
-        } else if (pre[k] == SPH_S_SORT) {
-            sph::sort_pairs_incremental(s, b.keys, x->N, c.key_bits, b.keys_alt, b.mask_alt, b.inc_ws, b.sort_ws,
-                                        b.flags, x->num_sms, x->side, x->ev_fork, x->ev_join, true);
-            b.keys_sorted = b.keys_alt;
-            b.mask_sorted = b.mask_alt;
-            x->cur_keys = b.keys_sorted;
-            x->cur_mask = b.mask_sorted;
-        } else if ((rc = run_stage_impl(x, pre[k])) != SPH_OK) {
-            return rc;
-        }
-        mark(x, pre_names[k]);
+    /* beside the fluid's binning: the list pass is the first to read the boundary's */
+    const bool sync = x->NB > 0 && x->any_movable;
+    cudaStream_t bnd = s;
+    if (sync) {
+        bnd = bnd_fork(x);
+        boundary_sync(x, bnd);
+        mark(x, "boundary_sync");
     }
+    /* the hashes with the incremental sort's first pass, then the sort */
+    sph::launch_hashes_flags(s, c, b.pos, x->N, b.keys, b.tab, b.cell_prev, b.flags, b.scenes, b.scene_of,
+                             sph::sort_inc_flags_args(b.inc_ws, x->N));
+    mark(x, "k_hashes");
+    sph::sort_pairs_incremental(s, b.keys, x->N, c.key_bits, b.keys_alt, b.mask_alt, b.inc_ws, b.sort_ws, b.flags,
+                                x->num_sms, x->side, x->ev_fork, x->ev_join, true);
+    b.keys_sorted = b.keys_alt;
+    b.mask_sorted = b.mask_alt;
+    x->cur_keys = b.keys_sorted;
+    x->cur_mask = b.mask_sorted;
+    mark(x, "sort");
     /* the SHUFFLE and CELL_INTERVALS stages in one pass */
     const bool late_vel = vel_ready != nullptr;
     float4* const vh = x->p.method == SPH_WCSPH ? b.vhalf : nullptr;
@@ -501,6 +517,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
                               late_vel ? nullptr : vh, b.vhalf_s, b.ids, b.ids_s, b.keys_sorted, b.tab, b.cell_prev,
                               b.flags, bs, b.scenes, b.scene_of, sph::sort_inc_keep_args(b.inc_ws, x->N));
     mark(x, "k_gather_ranges");
+    bnd_join(x, bnd);
     /* the velocities' part of the gather, once they have arrived (after the list pass) */
     auto gather_vel = [&]() {
         if (!late_vel) return;
@@ -518,16 +535,18 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
             sph::launch_wc_density(s, c, b, false, bs);
             mark(x, "k_wc_density");
         }
+        /* the forces on bodies read the densities; nothing of the step reads them */
+        cudaStream_t bf = s;
+        if (x->any_massive) {
+            bf = bnd_fork(x);
+            sph::launch_bnd_forces(bf, c, b, (int)x->bodies.size(), x->nmass, x->any_dynamic, bs);
+            mark(x, "k_bnd_forces");
+        }
         gather_vel();
         const bool pack = lists && c.sigma != 0.f;
         if (c.sigma != 0.f) {
             sph::launch_normals(s, c, b, lists, bs, x->num_sms, pack, lists);   /* k_lists_density wrote prho */
             mark(x, "k_normals");
-        }
-        if (x->any_massive) {
-            sph::launch_bnd_forces(s, c, b, (int)x->bodies.size(), bs);
-            if (x->any_dynamic) sph::launch_body_integrate(s, c, b, (int)x->bodies.size());
-            mark(x, "k_bnd_forces");
         }
         if (out && out->chunked) {
             /* the force pass (with the integration) in parts, each part's new state downloaded
@@ -552,6 +571,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
             sph::launch_wc_forces(s, c, b, lists, true, false, bs, x->num_sms, pack);
         }
         mark(x, "k_wc_forces");
+        bnd_join(x, bf);
     } else {
         if (!c.compat && !c.batched) {
             /* the lists and the initial density in one pass */
@@ -580,8 +600,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
             cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, pci_max_iter, x->coop_blocks, x->num_sms, false);
             if (e != cudaSuccess) return cuda_fail(x, e, "cooperative launch of the PCISPH loop");
             mark(x, "k_pci_loop");
-            sph::launch_bnd_forces(s, c, b, (int)x->bodies.size(), bs);
-            if (x->any_dynamic) sph::launch_body_integrate(s, c, b, (int)x->bodies.size());
+            sph::launch_bnd_forces(s, c, b, (int)x->bodies.size(), x->nmass, x->any_dynamic, bs);
             mark(x, "k_bnd_forces");
             sph::launch_pci_integrate(s, c, b, bs);
             mark(x, "k_pci_integrate");
@@ -781,14 +800,17 @@ int rebuild(sph_ctx* x, bool keep) {
     x->any_movable = false;
     x->any_massive = false;
     x->any_dynamic = false;
+    x->nmass = 0;
     if (x->NB > 0) {
         std::vector<int32_t> body(x->NB), range(4 * x->bodies.size());
         std::vector<float> xf(20 * x->bodies.size()), dyn(8 * x->bodies.size(), 0.f);
         std::vector<float> raw(x->braw_host);
+        std::vector<int32_t> massive;
         for (size_t k = 0; k < x->bodies.size(); ++k) {
             const SphBody& bd = x->bodies[k];
             for (int i = 0; i < bd.count; ++i) {
                 body[bd.origin + i] = (int)k;
+                if (bd.mass > 0.f) massive.push_back(bd.origin + i);
                 raw[4 * (size_t)(bd.origin + i) + 3] = 1.f;
             }
             range[4 * k] = bd.origin; range[4 * k + 1] = bd.count;
@@ -802,13 +824,16 @@ int rebuild(sph_ctx* x, bool keep) {
             dyn[8 * k + 5] = bd.radius;
             x->any_dynamic |= bd.dynamic != 0;
         }
+        x->nmass = (int)massive.size();
+        if (x->nmass > 0)
+            SPH_CUDA(x, cudaMemcpyAsync(b.bmass, massive.data(), 4 * massive.size(), cudaMemcpyHostToDevice, s));
         SPH_CUDA(x, cudaMemcpyAsync(b.body_dyn, dyn.data(), 4 * dyn.size(), cudaMemcpyHostToDevice, s));
         SPH_CUDA(x, cudaMemcpyAsync(b.braw, raw.data(), 16 * (size_t)x->NB, cudaMemcpyHostToDevice, s));
         SPH_CUDA(x, cudaMemcpyAsync(b.bbody, body.data(), 4 * (size_t)x->NB, cudaMemcpyHostToDevice, s));
         SPH_CUDA(x, cudaMemcpyAsync(b.body_range, range.data(), 4 * range.size(), cudaMemcpyHostToDevice, s));
         SPH_CUDA(x, cudaMemcpyAsync(b.body_xf, xf.data(), 4 * xf.size(), cudaMemcpyHostToDevice, s));
         sph::launch_bnd_transform(s, b, (int)x->bodies.size(), x->NB, x->c.compat != 0, false, x->bs);
-        boundary_sort(x);
+        boundary_sort(x, s);
         sph::launch_bnd_phi(s, x->c, b, x->p.boundary_phi_coeff > 0.f ? x->p.boundary_phi_coeff : 1.0f, x->bs);
         SPH_CUDA(x, cudaGetLastError());
     }
@@ -926,6 +951,9 @@ static void release_side(sph_ctx* x) {
     if (x->side) cudaStreamDestroy(x->side);
     if (x->ev_fork) cudaEventDestroy(x->ev_fork);
     if (x->ev_join) cudaEventDestroy(x->ev_join);
+    if (x->bnd_stream) cudaStreamDestroy(x->bnd_stream);
+    if (x->ev_bnd_fork) cudaEventDestroy(x->ev_bnd_fork);
+    if (x->ev_bnd_join) cudaEventDestroy(x->ev_bnd_join);
     if (x->copy_stream) cudaStreamDestroy(x->copy_stream);
     if (x->ev_copy) cudaEventDestroy(x->ev_copy);
     if (x->ev_vel) cudaEventDestroy(x->ev_vel);
@@ -933,7 +961,8 @@ static void release_side(sph_ctx* x) {
         if (e) cudaEventDestroy(e);
         e = nullptr;
     }
-    x->side = x->copy_stream = nullptr;
+    x->side = x->copy_stream = x->bnd_stream = nullptr;
+    x->ev_bnd_fork = x->ev_bnd_join = nullptr;
     x->ev_fork = x->ev_join = x->ev_copy = x->ev_vel = nullptr;
 }
 
@@ -1172,6 +1201,9 @@ int sph_create(const sph_params* params, sph_ctx** out) {
     if (cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&x->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&x->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&x->bnd_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&x->ev_bnd_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&x->ev_bnd_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&x->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&x->ev_copy, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&x->ev_vel, cudaEventDisableTiming) != cudaSuccess ||
@@ -1206,6 +1238,7 @@ int sph_destroy(sph_ctx* x) {
     if (x->own_stream && x->stream) cudaStreamDestroy(x->stream);
     if (x->side) cudaStreamSynchronize(x->side);
     if (x->copy_stream) cudaStreamSynchronize(x->copy_stream);
+    if (x->bnd_stream) cudaStreamSynchronize(x->bnd_stream);
     release_side(x);
     delete x;
     return SPH_OK;

@@ -32,6 +32,10 @@ struct sph_ctx {
      * (the gated full sort of the step's incremental sort) */
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    /* the boundary's stream and events: movable bodies' particles are binned beside the fluid's
+     * binning, and the forces on bodies are summed beside the normal and force passes */
+    cudaStream_t bnd_stream = nullptr;
+    cudaEvent_t ev_bnd_fork = nullptr, ev_bnd_join = nullptr;
     /* sph_simulate_host: the stream and events of the velocity uploads, and the step graph
      * with its copies for one set of host buffers */
     cudaStream_t copy_stream = nullptr;
@@ -52,6 +56,7 @@ struct sph_ctx {
     std::vector<float> braw_host;
     std::vector<SphBody> bodies;
     int N = 0, NB = 0;
+    int nmass = 0;   /* boundary particles of bodies with mass (Bufs::bmass) */
     bool any_movable = false, any_massive = false, any_dynamic = false;
     char* arena = nullptr;
     size_t arena_bytes = 0;

@@ -576,6 +576,87 @@ __device__ __forceinline__ float sum_lanes(float v) {
     return v;
 }
 
+constexpr int kSplitLanes = 8;   /* lanes per particle of split_scan */
+constexpr int kSplitAhead = 2;   /* rounds of a pair of cells loaded ahead */
+/* The entries of a group of kSplitLanes lanes' particle, in list order: put(e, j, r2) for entry e < cap
+ * by the lane that found it.  Returns their number, in all of them.  rng: the group's 27
+ * ranges in shared memory.  The cells go in pairs (the own cell alone), a pair's candidates
+ * kSplitLanes a round in order; the next pair's first rounds are loaded during a pair's. */
+template <class Put>
+__device__ __forceinline__ int split_scan(int nx, int ny, int nz, int cx, int cy, int cz, bool live, float h2,
+                                          int cap, const int2* __restrict__ tab, const float4* __restrict__ npos,
+                                          float4 p, int g, int2* rng, Put&& put) {
+    constexpr int G = kSplitLanes;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < (27 + G - 1) / G; ++k) {
+        const int o = g + k * G;
+        int2 r = make_int2(0, 0);
+        if (o < 27) {
+            int ox, oy, oz;
+            neigh_offset(o, ox, oy, oz);
+            const int x = cx + ox, y = cy + oy, z = cz + oz;
+            if (live && (unsigned)x < (unsigned)nx && (unsigned)y < (unsigned)ny && (unsigned)z < (unsigned)nz)
+                r = __ldg(&tab[x + nx * (y + ny * z)]);
+            rng[o] = make_int2(r.x, r.y - r.x);
+        }
+    }
+    __syncwarp();
+    const int gbase = (threadIdx.x & 31) & ~(G - 1);
+    const unsigned lt = ((1u << g) - 1u) << gbase, all = ((1u << G) - 1u) << gbase;
+    int cnt = 0;
+    /* candidate c of the pair (a, b): its index, or 0 past the pair's end */
+    auto index = [&](int2 a, int2 b, int c) {
+        const int j = c < a.y ? a.x + c : b.x + c - a.y;
+        return c < a.y + b.y ? j : 0;
+    };
+    auto test = [&](bool in, int j, float4 q) {
+        const float r2 = r2_exact(__fsub_rn(p.x, q.x), __fsub_rn(p.y, q.y), __fsub_rn(p.z, q.z));
+        const bool hit = in && r2 < h2;
+        const unsigned b = __ballot_sync(0xffffffffu, hit);
+        const int e = cnt + __popc(b & lt);
+        if (hit && e < cap) put(e, j, r2);
+        cnt += __popc(b & all);
+    };
+    int2 ra = rng[0], rb = make_int2(0, 0);
+    int j[kSplitAhead];
+    float4 q[kSplitAhead];
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) {
+        j[u] = index(ra, rb, u * G + g);
+        q[u] = __ldg(&npos[j[u]]);
+    }
+#pragma unroll 1
+    for (int t = 0; t < 14; ++t) {
+        const int n = ra.y + rb.y;
+        const int2 na = t < 13 ? rng[2 * t + 1] : make_int2(0, 0), nb = t < 13 ? rng[2 * t + 2] : make_int2(0, 0);
+        int jn[kSplitAhead];
+        float4 qn[kSplitAhead];
+#pragma unroll
+        for (int u = 0; u < kSplitAhead; ++u) {   /* the next pair's first rounds */
+            jn[u] = index(na, nb, u * G + g);
+            qn[u] = __ldg(&npos[jn[u]]);
+        }
+#pragma unroll
+        for (int u = 0; u < kSplitAhead; ++u)
+            if (u == 0 || __any_sync(0xffffffffu, u * G < n)) test(u * G + g < n, j[u], q[u]);
+#pragma unroll 1
+        for (int b = kSplitAhead * G; __any_sync(0xffffffffu, b < n); b += G) {
+            const int jj = index(ra, rb, b + g);
+            test(b + g < n, jj, __ldg(&npos[jj]));
+        }
+        ra = na;
+        rb = nb;
+#pragma unroll
+        for (int u = 0; u < kSplitAhead; ++u) {
+            j[u] = jn[u];
+            q[u] = qn[u];
+        }
+    }
+    __syncwarp();
+    return min(cnt, cap);
+}
+
 /* Neighbour source: either the cell scan or the materialised list, same order. */
 template <bool LIST, bool EXACT = true>
 struct Neigh {

@@ -9,7 +9,7 @@
  *
  * k_lists_density walks a particle's 27 cells (about 200 candidates) in one thread.  With
  * fewer particles than the GPU holds threads that walk's latency is the kernel's time,
- * whatever the size.  Here kLanes lanes share a particle: they test as many candidates at a
+ * whatever the size.  Here kSplitLanes lanes share a particle: they test as many candidates at a
  * time, in the list's order, and a ballot gives each hit its place.  The density terms go to shared memory
  * by entry, and one lane adds them in list order, so the sum has the order and rounding of
  * the one-thread walk.
@@ -20,89 +20,9 @@ namespace sph {
 
 namespace {
 constexpr int kSplitThreads = 256;
-constexpr int kLanes = 8;   /* lanes per particle */
-constexpr int kAhead = 2;   /* rounds of a pair of cells loaded ahead */
-constexpr int kPer = kSplitThreads / kLanes;
+constexpr int kPer = kSplitThreads / kSplitLanes;
 constexpr unsigned kAll = 0xffffffffu;
 
-/* The entries of a group of kLanes lanes' particle, in list order: put(e, j, r2) for entry e < cap
- * by the lane that found it.  Returns their number, in all of them.  rng: the group's 27
- * ranges in shared memory.  The cells go in pairs (the own cell alone), a pair's candidates
- * kLanes a round in order; the next pair's first rounds are loaded during a pair's. */
-template <class Put>
-__device__ __forceinline__ int split_scan(int nx, int ny, int nz, int cx, int cy, int cz, bool live, float h2,
-                                          int cap, const int2* __restrict__ tab, const float4* __restrict__ npos,
-                                          float4 p, int g, int2* rng, Put&& put) {
-    constexpr int G = kLanes;
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < (27 + G - 1) / G; ++k) {
-        const int o = g + k * G;
-        int2 r = make_int2(0, 0);
-        if (o < 27) {
-            int ox, oy, oz;
-            neigh_offset(o, ox, oy, oz);
-            const int x = cx + ox, y = cy + oy, z = cz + oz;
-            if (live && (unsigned)x < (unsigned)nx && (unsigned)y < (unsigned)ny && (unsigned)z < (unsigned)nz)
-                r = __ldg(&tab[x + nx * (y + ny * z)]);
-            rng[o] = make_int2(r.x, r.y - r.x);
-        }
-    }
-    __syncwarp();
-    const int gbase = (threadIdx.x & 31) & ~(G - 1);
-    const unsigned lt = ((1u << g) - 1u) << gbase, all = ((1u << G) - 1u) << gbase;
-    int cnt = 0;
-    /* candidate c of the pair (a, b): its index, or 0 past the pair's end */
-    auto index = [&](int2 a, int2 b, int c) {
-        const int j = c < a.y ? a.x + c : b.x + c - a.y;
-        return c < a.y + b.y ? j : 0;
-    };
-    auto test = [&](bool in, int j, float4 q) {
-        const float r2 = r2_exact(__fsub_rn(p.x, q.x), __fsub_rn(p.y, q.y), __fsub_rn(p.z, q.z));
-        const bool hit = in && r2 < h2;
-        const unsigned b = __ballot_sync(kAll, hit);
-        const int e = cnt + __popc(b & lt);
-        if (hit && e < cap) put(e, j, r2);
-        cnt += __popc(b & all);
-    };
-    int2 ra = rng[0], rb = make_int2(0, 0);
-    int j[kAhead];
-    float4 q[kAhead];
-#pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-        j[u] = index(ra, rb, u * G + g);
-        q[u] = __ldg(&npos[j[u]]);
-    }
-#pragma unroll 1
-    for (int t = 0; t < 14; ++t) {
-        const int n = ra.y + rb.y;
-        const int2 na = t < 13 ? rng[2 * t + 1] : make_int2(0, 0), nb = t < 13 ? rng[2 * t + 2] : make_int2(0, 0);
-        int jn[kAhead];
-        float4 qn[kAhead];
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {   /* the next pair's first rounds */
-            jn[u] = index(na, nb, u * G + g);
-            qn[u] = __ldg(&npos[jn[u]]);
-        }
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u)
-            if (u == 0 || __any_sync(kAll, u * G < n)) test(u * G + g < n, j[u], q[u]);
-#pragma unroll 1
-        for (int b = kAhead * G; __any_sync(kAll, b < n); b += G) {
-            const int jj = index(ra, rb, b + g);
-            test(b + g < n, jj, __ldg(&npos[jj]));
-        }
-        ra = na;
-        rb = nb;
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            j[u] = jn[u];
-            q[u] = qn[u];
-        }
-    }
-    __syncwarp();
-    return min(cnt, cap);
-}
 }  // namespace
 
 /* REMAP (the adjoint's tape, particles in id order): the list of sorted particle i is row
@@ -119,7 +39,7 @@ __global__ void __launch_bounds__(kSplitThreads)
     extern __shared__ float2 s_term[];   /* per particle: cap entries, padded to an odd number */
     __shared__ int2 s_rng[kPer][27];
     chain_next();
-    const int g = threadIdx.x & (kLanes - 1), slot = threadIdx.x / kLanes;
+    const int g = threadIdx.x & (kSplitLanes - 1), slot = threadIdx.x / kSplitLanes;
     const int i = blockIdx.x * kPer + slot;
     const bool live = i < c0.n;
     Const c = c0;
@@ -192,7 +112,7 @@ static void split_launch(cudaStream_t s, const Const& c, const Bufs& b, const in
 }
 
 bool launch_lists_split(cudaStream_t s, const Const& c, const Bufs& b, bool pci, const int32_t* remap, int num_sms) {
-    if (c.compat || c.wrap || c.cap > kMaxCap || c.n > 2 * 2048LL * num_sms / kLanes) return false;
+    if (c.compat || c.wrap || c.cap > kMaxCap || c.n > 2 * 2048LL * num_sms / kSplitLanes) return false;
     if (remap) split_launch<false, true, false>(s, c, b, remap);
     else if (pci) split_launch<false, false, true>(s, c, b, nullptr);
     else if (c.batched) split_launch<true, false, false>(s, c, b, nullptr);
