@@ -57,13 +57,6 @@ __global__ void k_adj_init(int n, float4* __restrict__ x, float4* __restrict__ v
     u[i] = w;
 }
 
-__global__ void k_adj_gather(int n, const int32_t* __restrict__ perm, const float4* __restrict__ x,
-                             float4* __restrict__ xs) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    xs[i] = __ldg(&x[__ldg(&perm[i])]);
-}
-
 __global__ void k_adj_iota(int n, int32_t* __restrict__ ids) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) ids[i] = i;
@@ -75,6 +68,7 @@ __global__ void k_adj_integrate_bwd(Const c, int n, const float4* __restrict__ x
                                     const float4* __restrict__ a, const float4* __restrict__ lx1,
                                     const float4* __restrict__ lv1, const float4* __restrict__ lu1,
                                     float4* __restrict__ la, float4* __restrict__ lu0, unsigned* __restrict__ flags) {
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float dt = c.dt, vm = c.vmax;
@@ -109,7 +103,9 @@ __global__ void k_adj_integrate_bwd(Const c, int n, const float4* __restrict__ x
 
 /* Backward of the pressure and viscosity sums (k_wc_forces, PHYSICS, no surface tension,
  * no boundary): lambda_rho (through C and R), the direct position adjoint, the velocity
- * adjoint, and each particle's share of dL/dmu and dL/dk (added to per-particle doubles). */
+ * adjoint, and each particle's share of dL/dmu and dL/dk (added to per-particle doubles).
+ * W lanes a particle (walk_lanes), their sums added. */
+template <int W>
 __global__ void __launch_bounds__(256) k_adj_forces_bwd(Const c, int n, const float4* __restrict__ x,
                                                         const float4* __restrict__ v,
                                                         const float4* __restrict__ aux,
@@ -117,8 +113,9 @@ __global__ void __launch_bounds__(256) k_adj_forces_bwd(Const c, int n, const fl
                                                         const int* __restrict__ len, float* __restrict__ lrho,
                                                         float4* __restrict__ lxf, float4* __restrict__ lv,
                                                         double* __restrict__ gmu, double* __restrict__ gk) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    chain_next();
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w = t0 / W < n ? t0 & (W - 1) : W, i = min(t0 / W, n - 1);   /* w = W: past the end */
     const float4 pi = __ldg(&x[i]), vi = __ldg(&v[i]), ai = __ldg(&aux[i]), A = __ldg(&la[i]);
     const float Ci = ai.x, Ri = ai.y, rho = ai.z, p = ai.w;
     const float h = c.h, m = c.mass, sg = c.spiky_grad, rmin2 = c.rmin2_wc;
@@ -127,9 +124,10 @@ __global__ void __launch_bounds__(256) k_adj_forces_bwd(Const c, int n, const fl
     float lC = 0.f, lR = 0.f;
     float gxx = 0.f, gxy = 0.f, gxz = 0.f, lvx = 0.f, lvy = 0.f, lvz = 0.f;
     float smx = 0.f, smy = 0.f, smz = 0.f;
-    if (rho > 0.f) {
-        list_neighbors(i, n, list, __ldg(&len[i]), x, pi.x, pi.y, pi.z,
-                       [&](int j, float4, float dx, float dy, float dz) {
+    {
+        /* a lane's last batch may visit the particle itself, which the distance guard refuses */
+        list_neighbors_split<W>(i, n, list, w < W && rho > 0.f ? __ldg(&len[i]) : 0, w, i, x, pi.x, pi.y, pi.z,
+                                [&](int j, float4, float dx, float dy, float dz) {
             const float4 aj = __ldg(&aux[j]);
             const float4 B = __ldg(&la[j]);
             const float4 vj = __ldg(&v[j]);
@@ -167,6 +165,13 @@ __global__ void __launch_bounds__(256) k_adj_forces_bwd(Const c, int n, const fl
             }
         });
     }
+    if (W > 1) {
+        lC = sum_lanes<W>(lC); lR = sum_lanes<W>(lR);
+        gxx = sum_lanes<W>(gxx); gxy = sum_lanes<W>(gxy); gxz = sum_lanes<W>(gxz);
+        lvx = sum_lanes<W>(lvx); lvy = sum_lanes<W>(lvy); lvz = sum_lanes<W>(lvz);
+        smx = sum_lanes<W>(smx); smy = sum_lanes<W>(smy); smz = sum_lanes<W>(smz);
+    }
+    if (w != 0) return;
     float lr = 0.f, gki = 0.f;
     if (rho > 0.f) {
         const float q = rho / c.rho0;
@@ -187,7 +192,9 @@ __global__ void __launch_bounds__(256) k_adj_forces_bwd(Const c, int n, const fl
     gk[i] += (double)gki;
 }
 
-/* Backward of the density sum: lambda_x += sum_j -6 poly6 m (h^2 - r^2)^2 (lrho_i + lrho_j) d. */
+/* Backward of the density sum: lambda_x += sum_j -6 poly6 m (h^2 - r^2)^2 (lrho_i + lrho_j) d.
+ * W lanes a particle as above (the particle itself adds zeros). */
+template <int W>
 __global__ void __launch_bounds__(256) k_adj_density_bwd(Const c, int n, const float4* __restrict__ x,
                                                          const float* __restrict__ lrho,
                                                          const int* __restrict__ list,
@@ -195,19 +202,27 @@ __global__ void __launch_bounds__(256) k_adj_density_bwd(Const c, int n, const f
                                                          const float4* __restrict__ lx1,
                                                          const float4* __restrict__ lxf,
                                                          float4* __restrict__ lx0) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    chain_next();
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w = t0 / W < n ? t0 & (W - 1) : W, i = min(t0 / W, n - 1);
     const float4 pi = __ldg(&x[i]);
     const float li = __ldg(&lrho[i]);
     const float hh = c.h * c.h, k6 = -6.0f * c.poly6_eval * c.mass;
     float gx = 0.f, gy = 0.f, gz = 0.f;
-    list_neighbors(i, n, list, __ldg(&len[i]), x, pi.x, pi.y, pi.z, [&](int j, float4, float dx, float dy, float dz) {
+    list_neighbors_split<W>(i, n, list, w < W ? __ldg(&len[i]) : 0, w, i, x, pi.x, pi.y, pi.z,
+                            [&](int j, float4, float dx, float dy, float dz) {
         const float t = hh - r2_exact(dx, dy, dz);
         const float q = k6 * (t * t) * (li + __ldg(&lrho[j]));
         gx += q * dx;
         gy += q * dy;
         gz += q * dz;
     });
+    if (W > 1) {
+        gx = sum_lanes<W>(gx);
+        gy = sum_lanes<W>(gy);
+        gz = sum_lanes<W>(gz);
+    }
+    if (w != 0) return;
     const float4 a = lx1[i], b = lxf[i];
     lx0[i] = make_float4(a.x + b.x + gx, a.y + b.y + gy, a.z + b.z + gz, 0.f);
 }
@@ -343,8 +358,8 @@ int adj_step(sph_adj* a, const float4* x, const float4* v, const float4* u, floa
     int32_t* ms = nullptr;
     sph::sort_pairs(s, a->keys, a->mask, a->keys_alt, a->mask_alt, n, c.key_bits, a->sort_ws, a->flags, ctx->num_sms,
                     &ks, &ms);
-    sph::k_adj_gather<<<sph::blocks(n, bs), bs, 0, s>>>(n, ms, x, a->pos_s);
-    sph::launch_cell_ranges(s, c, a->pos_s, ks, n, a->tab, a->cell_prev, a->flags, bs, ctx->b.scenes, nullptr);
+    sph::launch_gather_ranges(s, c, n, ms, x, a->pos_s, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, ks,
+                              a->tab, a->cell_prev, a->flags, bs, ctx->b.scenes, nullptr, sph::IncKeep{});
     Bufs lb{};
     lb.pos_s = a->pos_s;
     lb.tab = a->tab;
@@ -376,6 +391,18 @@ int adj_step(sph_adj* a, const float4* x, const float4* v, const float4* u, floa
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return afail(a, SPH_E_CUDA, std::string("adjoint forward launch: ") + cudaGetErrorString(e));
     return SPH_OK;
+}
+
+/* The two pair passes of backward step k of the segment. */
+template <int W>
+void backward_pairs(sph_adj* a, int k, const float4* xk, const int32_t* lk, const int32_t* nk, int cur, int nx) {
+    const cudaStream_t s = a->ctx->stream;
+    const size_t sn = (size_t)a->N;
+    const int g = sph::blocks(a->N * W, 256);
+    sph::launch_chained(s, sph::k_adj_forces_bwd<W>, g, 256, 0, a->c, a->N, xk, a->tv + k * sn, a->taux + k * sn, a->la,
+                        lk, nk, a->lrho, a->lxf, a->lv[nx], a->gmu, a->gk);
+    sph::launch_chained(s, sph::k_adj_density_bwd<W>, g, 256, 0, a->c, a->N, xk, a->lrho, lk, nk, a->lx[cur], a->lxf,
+                        a->lx[nx]);
 }
 
 int copy_state(sph_adj* a, float4* dx, float4* dv, float4* du, const float4* sx, const float4* sv, const float4* su) {
@@ -522,14 +549,14 @@ int sph_adj_backward(sph_adj* a, const float* gxT_4, const float* gvT_4, float* 
             const float4* xk = a->tx + k * sn;
             const int32_t* lk = a->tlist + (size_t)k * a->cap * sn;
             const int32_t* nk = a->tlen + k * sn;
-            sph::k_adj_integrate_bwd<<<sph::blocks(n, bs), bs, 0, s>>>(a->c, n, xk, a->tu + k * sn, a->ta + k * sn,
-                                                                        a->lx[cur], a->lv[cur], a->lu[cur], a->la,
-                                                                        a->lu[nx], a->flags);
-            sph::k_adj_forces_bwd<<<sph::blocks(n, 256), 256, 0, s>>>(a->c, n, xk, a->tv + k * sn,
-                                                                       a->taux + k * sn, a->la, lk, nk, a->lrho,
-                                                                       a->lxf, a->lv[nx], a->gmu, a->gk);
-            sph::k_adj_density_bwd<<<sph::blocks(n, 256), 256, 0, s>>>(a->c, n, xk, a->lrho, lk, nk, a->lx[cur],
-                                                                        a->lxf, a->lx[nx]);
+            sph::launch_chained(s, sph::k_adj_integrate_bwd, sph::blocks(n, bs), bs, 0, a->c, n, xk, a->tu + k * sn,
+                                a->ta + k * sn, a->lx[cur], a->lv[cur], a->lu[cur], a->la, a->lu[nx], a->flags);
+            switch (sph::walk_lanes(n, a->ctx->num_sms)) {
+            case 8: backward_pairs<8>(a, k, xk, lk, nk, cur, nx); break;
+            case 4: backward_pairs<4>(a, k, xk, lk, nk, cur, nx); break;
+            case 2: backward_pairs<2>(a, k, xk, lk, nk, cur, nx); break;
+            default: backward_pairs<1>(a, k, xk, lk, nk, cur, nx); break;
+            }
             cur = nx;
         }
         cudaError_t e = cudaGetLastError();

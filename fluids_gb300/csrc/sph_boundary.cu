@@ -326,6 +326,7 @@ void launch_bnd_phi(cudaStream_t s, const Const& c, const Bufs& b, float phi_coe
  * whose particles can have a boundary neighbour); concurrent stores all write 1. */
 __global__ void k_bnd_near(Const c0, int nb, const float4* __restrict__ bpos_s, uint8_t* __restrict__ near,
                            const SceneDev* __restrict__ scenes, const int32_t* __restrict__ scene_of) {
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb) return;
     Const c = c0;
@@ -342,9 +343,8 @@ __global__ void k_bnd_near(Const c0, int nb, const float4* __restrict__ bpos_s, 
 }
 
 void launch_bnd_near(cudaStream_t s, const Const& c, const Bufs& b, int nb, int bs) {
-    cudaMemsetAsync(b.bnear, 0, (size_t)c.ncells, s);
     if (nb <= 0) return;
-    k_bnd_near<<<nblk(nb, bs), bs, 0, s>>>(c, nb, b.bpos_s, b.bnear, b.scenes, b.scene_of ? b.bbody_s : nullptr);
+    launch_chained(s, k_bnd_near, nblk(nb, bs), bs, 0, c, nb, b.bpos_s, b.bnear, b.scenes, b.scene_of ? b.bbody_s : nullptr);
 }
 
 /* One step of a dynamic body (semi-implicit Euler, the default of the reference's rigid-body

@@ -333,6 +333,7 @@ void drop_graph(sph_ctx* x) {
 void boundary_sort(sph_ctx* x, cudaStream_t s) {
     Bufs& b = x->b;
     Const cb = x->c;
+    cudaMemsetAsync(b.bnear, 0, (size_t)cb.ncells, s);
     /* batched: the boundary body of scene s is body s, so body ids are scene ids */
     sph::launch_hashes(s, cb, b.bpos, x->NB, b.bkeys, b.bmask, b.btab, b.bcell_prev, b.flags, x->bs, b.scenes,
                        b.scene_of ? b.bbody : nullptr);

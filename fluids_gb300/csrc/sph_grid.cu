@@ -47,6 +47,7 @@ __global__ void k_hashes(Const c0, const float4* __restrict__ pos, int n, uint32
                          int32_t* __restrict__ mask, int2* __restrict__ tab, const int32_t* __restrict__ cell_prev,
                          unsigned* __restrict__ flags, const SceneDev* __restrict__ scenes,
                          const int32_t* __restrict__ scene_of) {
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     keys[i] = hash_particle(c0, pos[i], i, tab, cell_prev ? cell_prev[i] : -1, flags, scenes, scene_of);
@@ -136,6 +137,7 @@ __global__ void k_gather_boundary(int n, const int32_t* __restrict__ perm, const
                                   float4* __restrict__ pos_s, const int32_t* __restrict__ body,
                                   int32_t* __restrict__ body_s, const float* __restrict__ phi,
                                   float* __restrict__ phi_s) {
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int src = perm[i];
@@ -159,6 +161,7 @@ __device__ __forceinline__ long long global_cell(const Const& c0, const float4& 
 __global__ void k_cell_ranges(Const c, const float4* __restrict__ spos, const uint32_t* __restrict__ keys, int n,
                               int2* __restrict__ tab, int32_t* __restrict__ cell_out, unsigned* __restrict__ flags,
                               const SceneDev* __restrict__ scenes, const int32_t* __restrict__ scene_of) {
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int* t = reinterpret_cast<int*>(tab);
@@ -258,7 +261,7 @@ void launch_hashes(cudaStream_t s, const Const& c, const float4* pos, int n, uin
                    int2* tab, const int32_t* cell_prev, unsigned* flags, int bs, const SceneDev* scenes,
                    const int32_t* scene_of) {
     if (n <= 0) return;
-    k_hashes<<<blocks_for(n, bs), bs, 0, s>>>(c, pos, n, keys, mask, tab, cell_prev, flags, scenes, scene_of);
+    launch_chained(s, k_hashes, blocks_for(n, bs), bs, 0, c, pos, n, keys, mask, tab, cell_prev, flags, scenes, scene_of);
 }
 void launch_hashes_flags(cudaStream_t s, const Const& c, const float4* pos, int n, uint32_t* keys, int2* tab,
                          const int32_t* cell_prev, unsigned* flags, const SceneDev* scenes, const int32_t* scene_of,
@@ -275,21 +278,21 @@ void launch_gather(cudaStream_t s, int n, const int32_t* perm, const float4* a, 
 void launch_gather_boundary(cudaStream_t s, int n, const int32_t* perm, const float4* pos, float4* pos_s,
                             const int32_t* body, int32_t* body_s, const float* phi, float* phi_s, int bs) {
     if (n <= 0) return;
-    k_gather_boundary<<<blocks_for(n, bs), bs, 0, s>>>(n, perm, pos, pos_s, body, body_s, phi, phi_s);
+    launch_chained(s, k_gather_boundary, blocks_for(n, bs), bs, 0, n, perm, pos, pos_s, body, body_s, phi, phi_s);
 }
 void launch_gather_ranges(cudaStream_t s, const Const& c, int n, const int32_t* perm, const float4* a, float4* as,
                           const float4* b, float4* bs_, const float4* c3, float4* cs, const int32_t* ids,
                           int32_t* ids_s, const uint32_t* keys, int2* tab, int32_t* cell_out, unsigned* flags, int bs,
                           const SceneDev* scenes, const int32_t* scene_of, const IncKeep& inc) {
     if (n <= 0) return;
-    k_gather_ranges<<<blocks_for(n, bs), bs, 0, s>>>(c, n, perm, a, as, b, bs_, c3, cs, ids, ids_s, keys, tab,
+    launch_chained(s, k_gather_ranges, blocks_for(n, bs), bs, 0, c, n, perm, a, as, b, bs_, c3, cs, ids, ids_s, keys, tab,
                                                      cell_out, flags, scenes, scene_of, inc);
 }
 void launch_cell_ranges(cudaStream_t s, const Const& c, const float4* spos, const uint32_t* keys, int n,
                         int2* tab, int32_t* cell_out, unsigned* flags, int bs, const SceneDev* scenes,
                         const int32_t* scene_of) {
     if (n <= 0) return;
-    k_cell_ranges<<<blocks_for(n, bs), bs, 0, s>>>(c, spos, keys, n, tab, cell_out, flags, scenes, scene_of);
+    launch_chained(s, k_cell_ranges, blocks_for(n, bs), bs, 0, c, spos, keys, n, tab, cell_out, flags, scenes, scene_of);
 }
 void launch_neigh_lists(cudaStream_t s, const Const& c, const float4* spos, const int2* tab, const float4* bpos_s,
                         const int2* btab, int* nlist, int* nlen, int* sblist, int* sblen, int bs,

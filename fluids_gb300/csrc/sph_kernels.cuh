@@ -123,6 +123,7 @@ struct IncKeep {
     unsigned *over, *valid;
     uint32_t *prev, *first, *sub;
     __device__ __forceinline__ void keep(int j, uint32_t key) const {
+        if (over == nullptr) return;   /* keys of another sort */
         if (j == 0) {
             *over = 0u;
             *valid = 1u;
@@ -203,7 +204,7 @@ void launch_pci_pressure_force(cudaStream_t s, const Const& c, const Bufs& b, in
 void launch_bnd_transform(cudaStream_t s, const Bufs& b, int nbodies, int nb, bool compat, bool only_movable,
                           int bs);
 void launch_bnd_phi(cudaStream_t s, const Const& c, const Bufs& b, float phi_coeff, int bs);
-/* marks bnear for the 27 cells around every sorted boundary particle (after clearing it) */
+/* marks bnear (zero before) for the 27 cells around every sorted boundary particle */
 void launch_bnd_near(cudaStream_t s, const Const& c, const Bufs& b, int nb, int bs);
 /* the fluid's force and torque on every body with mass (nmass particles of such bodies, listed
  * in b.bmass); dynamic: then advances every dynamic body by one step under them and gravity */

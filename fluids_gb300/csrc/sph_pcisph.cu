@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(256) k_pci_init_density(Const c, Bufs b) {
 /* W > 1 (small scenes, PACK): W lanes a particle (list_neighbors_split), their sums added. */
 template <bool PACK, bool MON = false, int W = 1>
 __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
+    chain_next();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (W == 1 && t >= c.n) return;
     const int w = W > 1 ? (t / W < c.n ? t & (W - 1) : W) : 0;
@@ -536,9 +537,9 @@ void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int b
     if (c.n <= 0) return;
     if (pack && !c.compat) {
         switch (walk_lanes(c.n, num_sms)) {
-        case 8: k_pci_init_forces<true, false, 8><<<nblk(8 * c.n, 256), 256, 0, s>>>(c, b); return;
-        case 4: k_pci_init_forces<true, false, 4><<<nblk(4 * c.n, 256), 256, 0, s>>>(c, b); return;
-        case 2: k_pci_init_forces<true, false, 2><<<nblk(2 * c.n, 256), 256, 0, s>>>(c, b); return;
+        case 8: launch_chained(s, k_pci_init_forces<true, false, 8>, nblk(8 * c.n, 256), 256, 0, c, b); return;
+        case 4: launch_chained(s, k_pci_init_forces<true, false, 4>, nblk(4 * c.n, 256), 256, 0, c, b); return;
+        case 2: launch_chained(s, k_pci_init_forces<true, false, 2>, nblk(2 * c.n, 256), 256, 0, c, b); return;
         }
     }
     if (c.monaghan) {
@@ -546,7 +547,7 @@ void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int b
         else k_pci_init_forces<false, true><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
         return;
     }
-    if (pack) k_pci_init_forces<true><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
+    if (pack) launch_chained(s, k_pci_init_forces<true>, nblk(c.n, bs), bs, 0, c, b);
     else k_pci_init_forces<false><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
 }
 

@@ -487,10 +487,9 @@ void launch_wc_density(cudaStream_t s, const Const& c, const Bufs& b, bool lists
 template <bool COMPAT, bool BATCH>
 static void lists_density_launch(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
     unsigned* next = tile_counter(s, b, 1, BATCH);
-    k_lists_density<COMPAT, BATCH><<<grid_for<BATCH>(c, bs), bs, 0, s>>>(c, b.pos_s, b.tab, b.bpos_s, b.btab,
-                                                                b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen,
-                                                                b.density, b.pressure, b.aux, b.scenes, b.tiles,
-                                                                next, nullptr, nullptr, b.bnear, b.noff, b.prho);
+    launch_chained(s, k_lists_density<COMPAT, BATCH>, grid_for<BATCH>(c, bs), bs, 0, c, b.pos_s, b.tab, b.bpos_s,
+                   b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes,
+                   b.tiles, next, nullptr, nullptr, b.bnear, b.noff, b.prho);
 }
 
 void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
@@ -571,8 +570,8 @@ void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, i
                                                               next, b.vel_s, nrec);
         } else {
             if (prho)
-                k_normals<true, true, false, false, true><<<g, bs, 0, s>>>(c, fl, b.aux, b.density, b.normal,
-                                                                          b.scenes, b.tiles, next, b.vel_s, nrec);
+                launch_chained(s, k_normals<true, true, false, false, true>, g, bs, 0, c, fl, b.aux, b.density,
+                               b.normal, b.scenes, b.tiles, next, b.vel_s, nrec);
             else
                 k_normals<true, true, false><<<g, bs, 0, s>>>(c, fl, b.aux, b.density, b.normal, b.scenes, b.tiles,
                                                               next, b.vel_s, nrec);
@@ -621,11 +620,11 @@ static void forces_launch(cudaStream_t s, const Const& c, const Bufs& b, bool fu
     }
     if constexpr (LIST) {
         if (pack && st && fuse && !write_acc) {
-            k_wc_forces<COMPAT, LIST, true, false, true, BATCH, true><<<g, bs, 0, s>>>(c, fs, bsrc, b);
+            launch_chained(s, k_wc_forces<COMPAT, LIST, true, false, true, BATCH, true>, g, bs, 0, c, fs, bsrc, b);
             return;
         }
     }
-#define SPH_WCF(F, W, S) k_wc_forces<COMPAT, LIST, F, W, S, BATCH><<<g, bs, 0, s>>>(c, fs, bsrc, b)
+#define SPH_WCF(F, W, S) launch_chained(s, k_wc_forces<COMPAT, LIST, F, W, S, BATCH>, g, bs, 0, c, fs, bsrc, b)
     if (fuse) {
         if (write_acc) { if (st) SPH_WCF(true, true, true); else SPH_WCF(true, true, false); }
         else { if (st) SPH_WCF(true, false, true); else SPH_WCF(true, false, false); }
