@@ -87,9 +87,10 @@ struct sph_ctx {
     double* d_scene_stats = nullptr;
     int inject = 0;   /* one-shot fault for the next step (sph_inject_fault) */
     bool inject_alloc = false;   /* the next arena allocation fails (sph_inject_fault) */
-    /* depth-test scratch of sph_render_depth: 8 bytes per pixel */
+    /* depth-test scratch of sph_render_depth: 8 bytes per pixel, 4 per tile of 4 x 4 pixels, 8
+     * per particle and 65,536 more for the list of pairs to splat */
     void* render_buf = nullptr;
-    size_t render_pixels = 0;
+    size_t render_bytes = 0;
     void* render_sort = nullptr;   /* sph_render_depth: 16-bit depth keys and particle order */
     size_t render_sort_bytes = 0;
     void* frame_buf = nullptr;     /* sph_render_frame: depth, blur scratch, normals, colour */

@@ -3,7 +3,7 @@
  * kernels writing device images (no graphics API): particle depth sprites, the two
  * smoothing filters, and view-space normals.
  *
- *   k_splat_*        shaders/sspace_fluid_rendering/depth_stage.vert and .frag: each particle
+ *   k_splat_*, k_cover   shaders/sspace_fluid_rendering/depth_stage.vert and .frag: each particle
  *                    is a point sprite of gl_PointSize = point_radius * point_scale / |p_eye|;
  *                    a fragment inside the sprite's disc lies on the sphere of radius
  *                    point_radius around the particle; its normalised depth is written where
@@ -91,10 +91,11 @@ __device__ __forceinline__ bool fragment(const View& v, const float e[4], float 
  * sphere point's eye z, s2 in [e_z, e_z + r]; away from the pole s2 = -pr15 / pr14 it is
  * monotone there, so its smaller end value bounds every fragment.  A margin of 1e-5 covers the
  * fragments' own rounding. */
-__device__ __forceinline__ float depth_floor(const View& v, const float e[4]) {
+/* nz: the largest z of the sphere's unit normal among the fragments asked for. */
+__device__ __forceinline__ float depth_floor(const View& v, const float e[4], float nz = 1.0f) {
     const float* m = v.pr;
     if (m[8] != 0.f || m[9] != 0.f || m[12] != 0.f || m[13] != 0.f) return 0.f;
-    const float lo = e[2] - 1e-3f * v.radius, hi = e[2] + v.radius * 1.001f;
+    const float lo = e[2] - 1e-3f * v.radius, hi = e[2] + v.radius * (nz + 1e-3f);
     if (m[14] != 0.f) {
         const float pole = -m[15] / m[14];
         if (pole >= lo && pole <= hi) return 0.f;
@@ -148,6 +149,170 @@ __global__ void k_splat_keys(View v, int n, const float4* __restrict__ pos, cons
                 if (k < cur[u]) atomicMin(row + px, k);
             }
         }
+    }
+}
+
+/* Depth bounds of square tiles of pixels (side 1 << shift), so that the sprites behind the
+ * surface are not splatted: k_cover takes, for every tile that lies inside a sprite's disc, the
+ * farthest normalised depth that the sprite's fragments have in it, and the tile keeps the
+ * nearest of those.  Every pixel's winner is at least that near, so k_splat_cull skips a
+ * sprite's pixels in the tiles whose bound is nearer than its nearest fragment, without
+ * reading their keys.  Any skipped fragment loses the depth test, so the keys are those of
+ * k_splat_keys for any order; no front-to-back order is needed.  Measured on GB300, 1,062,234
+ * particles at 1920 x 1080 (sprites of about 12 pixels): cover 15 us,
+ * coarse bounds 3, cull 38 and pairs 29, against 40 for the order's sort and 231 for
+ * k_splat_keys; 37,000 of the particles pass in some tile. */
+__global__ void __launch_bounds__(256) k_cover(View v, int n, const float4* __restrict__ pos, int shift, int tw,
+                                               unsigned* __restrict__ tile) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float e[4], wx, wy, size;
+    if (!sprite(v, pos[i], e, wx, wy, size)) return;
+    const float* m = v.pr;
+    auto lin = [&](float s2) { return ((s2 * m[10] + m[11]) / (s2 * m[14] + m[15]) + 1.0f) * 0.5f; };
+    const float hi = e[2] + v.radius * 1.001f;
+    if (m[14] != 0.f) {   /* the depth is monotone in the eye z away from the pole */
+        const float pole = -m[15] / m[14];
+        if (pole >= e[2] - 1e-3f * v.radius && pole <= hi) return;
+    }
+    const float lin_hi = lin(hi);
+    /* the tiles inside the middle of the disc (0.6 of its radius), where the bound is tight */
+    const int side = 1 << shift;
+    const float inv = 2.0f / size, half = 0.3f * size, scale = 1.0f / (float)side;
+    const int tx0 = max(0, (int)ceilf((wx - half) * scale)), tx1 = min(tw, (int)floorf((wx + half) * scale));
+    const int ty0 = max(0, (int)ceilf((wy - half) * scale)),
+              ty1 = min((v.h + side - 1) >> shift, (int)floorf((wy + half) * scale));
+    for (int ty = ty0; ty < ty1; ++ty) {
+        /* the tile's pixel centre farthest from the sprite's, per axis */
+        const int ya = ty << shift, yb = min(ya + side, v.h) - 1;
+        const float dy = inv * fmaxf(fabsf((float)ya + 0.5f - wy), fabsf((float)yb + 0.5f - wy));
+        for (int tx = tx0; tx < tx1; ++tx) {
+            const int xa = tx << shift, xb = min(xa + side, v.w) - 1;
+            const float dx = inv * fmaxf(fabsf((float)xa + 0.5f - wx), fabsf((float)xb + 0.5f - wx));
+            const float mag = dx * dx + dy * dy;
+            if (!(mag < 0.999f)) continue;   /* a pixel of the tile may lie outside the disc */
+            /* margins far above the fragments' own rounding, as in depth_floor */
+            const float far = fmaxf(lin(e[2] + v.radius * (sqrtf(1.0f - mag) - 1e-3f)), lin_hi) + 1e-5f;
+            if (!(far < 1.0f)) continue;     /* fragments beyond the far plane are dropped */
+            const unsigned bits = __float_as_uint(fmaxf(far, 0.0f));
+            unsigned* const t = tile + (size_t)ty * tw + tx;
+            if (bits < __ldca(t)) atomicMin(t, bits);
+        }
+    }
+}
+
+/* The particles test their tiles, and the few (particle, tile) pairs that pass -- about one in a
+ * hundred, nearly all in the blocks of the surface and the silhouette -- go to a list (a block
+ * reserves its part at once), so that k_splat_pairs spreads them over the GPU.  A pair past the
+ * list's end is splatted by its own thread, and so are those of sprites of more than 32 tiles. */
+__device__ __forceinline__ void splat_pixel(const View& v, const float e[4], float wx, float wy, float size, int i,
+                                            int px, int py, unsigned long long* __restrict__ key) {
+    if (px >= v.w || py >= v.h) return;
+    unsigned long long* const at = key + (size_t)py * v.w + px;
+    const unsigned long long cur = __ldca(at);   /* L1 copy: stale is still safe */
+    float nd, lin;
+    if (!fragment(v, e, wx, wy, size, px, py, nd, lin)) return;
+    const unsigned long long k = ((unsigned long long)__float_as_uint(lin) << 32) | (unsigned)i;
+    if (k < cur) atomicMin(at, k);
+}
+
+/* The farthest bound of each 4 x 4 tiles: most hidden sprites are told by one to four of these. */
+__global__ void __launch_bounds__(256) k_tile_max(int tw, int th, const unsigned* __restrict__ tile, int cw, int ch,
+                                                  unsigned* __restrict__ coarse) {
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= cw * ch) return;
+    const int cy = k / cw, cx = k - cy * cw;
+    unsigned m = 0;
+    for (int y = 4 * cy; y < min(4 * cy + 4, th); ++y)
+        for (int x = 4 * cx; x < min(4 * cx + 4, tw); ++x) m = max(m, __ldg(&tile[(size_t)y * tw + x]));
+    coarse[k] = m;
+}
+
+__global__ void __launch_bounds__(256) k_splat_cull(View v, int n, const float4* __restrict__ pos, int shift, int tw,
+                                                    const unsigned* __restrict__ tile, int cw,
+                                                    const unsigned* __restrict__ coarse,
+                                                    unsigned long long* __restrict__ key, int2* __restrict__ list,
+                                                    unsigned cap, unsigned* __restrict__ count) {
+    __shared__ unsigned s_sum[8], s_base;
+    const int t = threadIdx.x, i = blockIdx.x * 256 + t, lane = t & 31, warp = t >> 5;
+    const int side = 1 << shift;
+    float e[4], wx = 0.f, wy = 0.f, size = 1.f;
+    unsigned passed = 0;   /* the tiles that pass, in row order, of the first 32 */
+    int tx0 = 0, ty0 = 0, nx = 0, ny = 0;
+    if (i < n && sprite(v, pos[i], e, wx, wy, size)) {
+        const unsigned floor_bits = __float_as_uint(depth_floor(v, e));
+        const float inv = 2.0f / size;
+        tx0 = max(0, (int)floorf(wx - 0.5f * size)) >> shift;
+        ty0 = max(0, (int)floorf(wy - 0.5f * size)) >> shift;
+        nx = (min(v.w - 1, (int)ceilf(wx + 0.5f * size)) >> shift) - tx0 + 1;
+        ny = (min(v.h - 1, (int)ceilf(wy + 0.5f * size)) >> shift) - ty0 + 1;
+        bool hidden = true;
+        for (int cy = ty0 >> 2; cy <= (ty0 + ny - 1) >> 2; ++cy)
+            for (int cx = tx0 >> 2; cx <= (tx0 + nx - 1) >> 2; ++cx)
+                hidden = hidden && floor_bits > __ldg(&coarse[(size_t)cy * cw + cx]);
+        if (hidden) ny = 0;
+        int q = 0;
+        for (int ty = ty0; ty < ty0 + ny; ++ty)
+            for (int tx = tx0; tx < tx0 + nx; ++tx, ++q) {
+                const unsigned bound = __ldg(&tile[(size_t)ty * tw + tx]);
+                if (floor_bits > bound) continue;
+                /* the nearest fragment in this tile: at its pixel centre nearest to the sprite's */
+                const float xa = (float)(tx << shift) + 0.5f, ya = (float)(ty << shift) + 0.5f;
+                const float dx = inv * fmaxf(0.0f, fmaxf(xa - wx, wx - (xa + (float)(side - 1))));
+                const float dy = inv * fmaxf(0.0f, fmaxf(ya - wy, wy - (ya + (float)(side - 1))));
+                const float mag = (dx * dx + dy * dy) * 0.999f;
+                if (mag > 1.0f) continue;   /* every pixel of it lies outside the disc */
+                if (__float_as_uint(depth_floor(v, e, sqrtf(1.0f - mag))) > bound) continue;
+                if (q < 32) passed |= 1u << q;
+                else
+                    for (int k = 0; k < side * side; ++k)
+                        splat_pixel(v, e, wx, wy, size, i, (tx << shift) + (k & (side - 1)), (ty << shift) + (k >> shift),
+                                    key);
+            }
+    }
+    const unsigned mine = (unsigned)__popc(passed);
+    unsigned sum = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned o = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += o;
+    }
+    if (lane == 31) s_sum[warp] = sum;
+    __syncthreads();
+    if (t == 0) {
+        unsigned all = 0;
+        for (int w = 0; w < 8; ++w) {
+            const unsigned c = s_sum[w];
+            s_sum[w] = all;
+            all += c;
+        }
+        s_base = all ? atomicAdd(count, all) : 0u;
+    }
+    __syncthreads();
+    unsigned at = s_base + s_sum[warp] + sum - mine;
+    for (; passed; passed &= passed - 1u, ++at) {
+        const int q = __ffs((int)passed) - 1, tx = tx0 + q % nx, ty = ty0 + q / nx;
+        if (at < cap) list[at] = make_int2(i, ty * tw + tx);
+        else
+            for (int k = 0; k < side * side; ++k)
+                splat_pixel(v, e, wx, wy, size, i, (tx << shift) + (k & (side - 1)), (ty << shift) + (k >> shift), key);
+    }
+}
+
+/* The listed pairs, 16 lanes each. */
+__global__ void __launch_bounds__(256) k_splat_pairs(View v, const float4* __restrict__ pos, int shift, int tw,
+                                                     unsigned long long* __restrict__ key,
+                                                     const int2* __restrict__ list, unsigned cap,
+                                                     const unsigned* __restrict__ count) {
+    const unsigned m = min(*count, cap);
+    const int side = 1 << shift;
+    for (unsigned k = (blockIdx.x * 256 + threadIdx.x) >> 4; k < m; k += gridDim.x * 16) {
+        const int2 w = __ldg(&list[k]);
+        float e[4], wx, wy, size;
+        if (!sprite(v, __ldg(&pos[w.x]), e, wx, wy, size)) continue;
+        const int ty = w.y / tw, tx = w.y - ty * tw;
+        for (int q = threadIdx.x & 15; q < side * side; q += 16)
+            splat_pixel(v, e, wx, wy, size, w.x, (tx << shift) + (q & (side - 1)), (ty << shift) + (q >> shift), key);
     }
 }
 
@@ -239,9 +404,12 @@ __global__ void k_particle_shade(View v, const float4* __restrict__ pos, const u
     out[k] = col;
 }
 
-__global__ void k_splat_clear(size_t npix, unsigned long long* __restrict__ key) {
+__global__ void k_splat_clear(size_t npix, unsigned long long* __restrict__ key, size_t ntiles,
+                              unsigned* __restrict__ tile) {
     const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k < npix) key[k] = ~0ull;
+    if (k < ntiles) tile[k] = ~0u;   /* no bound */
+    if (k == 0) tile[ntiles] = 0u;   /* the pairs listed */
 }
 
 __device__ __forceinline__ float texel(const float* img, int w, int h, int x, int y) {
@@ -250,21 +418,44 @@ __device__ __forceinline__ float texel(const float* img, int w, int h, int x, in
     return img[(size_t)y * w + x];
 }
 
-/* kernels/bilateral.cl */
-__global__ void k_bilateral(const float* __restrict__ in, float* __restrict__ out, int w, int h) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const float depth = texel(in, w, h, x, y);
+/* kernels/bilateral.cl.  The 64 weights depend on the offset alone, so a block forms them once
+ * (by the same arithmetic), and its pixels and their window come from shared memory.  A pass
+ * over 1920 x 1080 pixels, the fluid on about a tenth of them: 11 us, against 24 with an
+ * exponential per pixel and offset and the window from global memory. */
+constexpr int kBilW = 32, kBilH = 8;
+__global__ void __launch_bounds__(kBilW* kBilH) k_bilateral(const float* __restrict__ in, float* __restrict__ out,
+                                                            int w, int h) {
+    __shared__ float s_in[kBilH + 7][kBilW + 7];
+    __shared__ float s_wt[64];
+    const int bx = blockIdx.x * kBilW, by = blockIdx.y * kBilH;
+    const int x = bx + threadIdx.x, y = by + threadIdx.y, t = threadIdx.y * kBilW + threadIdx.x;
+    const bool inside = x < w && y < h;
+    const float depth = inside ? in[(size_t)y * w + x] : 0.0f;
+    if (!__syncthreads_or(depth > 0.0f)) {   /* no fluid in the block's pixels */
+        if (inside) out[(size_t)y * w + x] = 0.0f;
+        return;
+    }
+    if (t < 64) {
+        const float fx = (float)(t / 8 - 4), fy = (float)(t % 8 - 4);
+        const float r = sqrtf(fx * fx + fy * fy) * 0.0001f;
+        s_wt[t] = expf(-r * r);
+    }
+    for (int k = t; k < (kBilH + 7) * (kBilW + 7); k += kBilW * kBilH) {
+        const int ly = k / (kBilW + 7), lx = k % (kBilW + 7);
+        s_in[ly][lx] = texel(in, w, h, bx + lx - 4, by + ly - 4);
+    }
+    __syncthreads();
+    if (!inside) return;
     float o = 0.0f;
     if (depth > 0.0f) {
         float sum = 0.0f, wsum = 0.0f;
-        for (int dx = -4; dx < 4; ++dx)
-            for (int dy = -4; dy < 4; ++dy) {
-                const float s = texel(in, w, h, x + dx, y + dy);
+#pragma unroll
+        for (int dx = 0; dx < 8; ++dx)
+#pragma unroll
+            for (int dy = 0; dy < 8; ++dy) {
+                const float s = s_in[threadIdx.y + dy][threadIdx.x + dx];
                 if (fabsf(s - depth) < 0.015f) {
-                    const float fx = (float)dx, fy = (float)dy;
-                    const float r = sqrtf(fx * fx + fy * fy) * 0.0001f;
-                    const float wt = expf(-r * r);
+                    const float wt = s_wt[dx * 8 + dy];
                     sum += s * wt;
                     wsum += wt;
                 }
@@ -484,16 +675,61 @@ inline bool image_ok(int w, int h) {
 
 extern "C" {
 
-/* Checks the view, allocates the depth-test keys and the particle-order buffers, clears the
- * keys and sorts the particles front to back; the caller splats and resolves. */
-static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigned long long*& key,
-                         const int32_t*& sorted) {
+/* The tiles of k_cover for a view: their side's shift, or -1 when the sprites, at the distance
+ * of the scene's origin, are too small to cover tiles (below 6 pixels) or the projection is
+ * not a symmetric one.  4 pixels to a side below 24-pixel sprites, 8 below 48, else 16. */
+static int tile_shift(const sph_view* view) {
+    const float *m = view->projection, *t = view->modelview + 12;
+    if (m[8] != 0.f || m[9] != 0.f || m[12] != 0.f || m[13] != 0.f) return -1;
+    const float dist = std::sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+    const float size = view->point_radius * (view->point_scale / dist);
+    if (!(size >= 6.0f)) return -1;
+    return size < 24.0f ? 2 : (size < 48.0f ? 3 : 4);
+}
+
+/* Entries of the list of (particle, tile) pairs to splat. */
+static size_t splat_list_cap(int n) { return (size_t)n + 65536; }
+
+/* Checks the view, allocates the depth-test keys, the list of pairs, the tile bounds and the
+ * pair count (behind the ntiles bounds, before the coarse ones), and clears keys, bounds and
+ * count. */
+static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigned long long*& key, unsigned*& tile,
+                         int2*& list, size_t& ntiles) {
     if (!sph::image_ok(view->width, view->height))
         return sph_ctx_fail(x, SPH_E_INVALID, "render: width and height must be 1..65536 (at most 2^28 pixels)");
     if (!(view->point_radius > 0.f) || !(view->point_scale > 0.f))
         return sph_ctx_fail(x, SPH_E_INVALID, "render: point_radius and point_scale must be > 0");
     if (!x->has_state || x->N <= 0) return sph_ctx_fail(x, SPH_E_STATE, "render: no particles added");
     const size_t npix = (size_t)view->width * view->height;
+    ntiles = (size_t)((view->width + 3) / 4) * ((view->height + 3) / 4);   /* the most there are */
+    const size_t ncoarse = (size_t)((view->width + 15) / 16) * ((view->height + 15) / 16);
+    const size_t need = 8 * npix + 4 * (ntiles + 2 + ncoarse) + 8 * splat_list_cap(x->N);
+    if (x->render_bytes < need) {
+        cudaStreamSynchronize(x->stream);
+        cudaFree(x->render_buf);
+        x->render_buf = nullptr;
+        x->render_bytes = 0;
+        if (cudaMalloc(&x->render_buf, need) != cudaSuccess) {
+            cudaGetLastError();
+            return sph_ctx_fail(x, SPH_E_NOMEM, "render: depth-test buffers");
+        }
+        x->render_bytes = need;
+    }
+    std::memcpy(v.mv, view->modelview, sizeof v.mv);
+    std::memcpy(v.pr, view->projection, sizeof v.pr);
+    v.radius = view->point_radius;
+    v.scale = view->point_scale;
+    v.w = view->width;
+    v.h = view->height;
+    key = reinterpret_cast<unsigned long long*>(x->render_buf);
+    list = reinterpret_cast<int2*>(key + npix);
+    tile = reinterpret_cast<unsigned*>(list + splat_list_cap(x->N));
+    sph::k_splat_clear<<<(unsigned)((npix + 255) / 256), 256, 0, x->stream>>>(npix, key, ntiles, tile);
+    return SPH_OK;
+}
+
+/* The particles front to back (16 bits of the eye distance). */
+static int splat_order(sph_ctx* x, const sph::View& v, const int32_t*& sorted) {
     /* keys, order, their sort ping-pong copies and the sort's workspace, all the context's own */
     const size_t nsort = 16 * (size_t)x->N + sph::sort_workspace_bytes(x->N, 16);
     if (x->render_sort_bytes < nsort) {
@@ -509,27 +745,8 @@ static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigne
         /* the sort workspace starts at zero */
         cudaMemsetAsync(x->render_sort, 0, sph::sort_workspace_bytes(x->N, 16), x->stream);
     }
-    if (x->render_pixels < npix) {
-        cudaStreamSynchronize(x->stream);
-        cudaFree(x->render_buf);
-        x->render_buf = nullptr;
-        x->render_pixels = 0;
-        if (cudaMalloc(&x->render_buf, 8 * npix) != cudaSuccess) {
-            cudaGetLastError();
-            return sph_ctx_fail(x, SPH_E_NOMEM, "render: depth-test buffers");
-        }
-        x->render_pixels = npix;
-    }
-    std::memcpy(v.mv, view->modelview, sizeof v.mv);
-    std::memcpy(v.pr, view->projection, sizeof v.pr);
-    v.radius = view->point_radius;
-    v.scale = view->point_scale;
-    v.w = view->width;
-    v.h = view->height;
-    key = reinterpret_cast<unsigned long long*>(x->render_buf);
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
-    sph::k_splat_clear<<<(unsigned)((npix + bs - 1) / bs), bs, 0, s>>>(npix, key);
     void* ws = x->render_sort;   /* first, so that it stays in place when the particle count changes */
     uint32_t* okeys = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + sph::sort_workspace_bytes(n, 16));
     int32_t* order = reinterpret_cast<int32_t*>(okeys + n);
@@ -547,13 +764,30 @@ int sph_render_depth(sph_ctx* x, const sph_view* view, float* d_depth) {
     if (!x || !view || !d_depth) return SPH_E_INVALID;
     sph::View v;
     unsigned long long* key;
-    const int32_t* sorted;
-    const int rc = splat_prepare(x, view, v, key, sorted);
+    unsigned* tile;
+    int2* list;
+    size_t ntiles;
+    int rc = splat_prepare(x, view, v, key, tile, list, ntiles);
     if (rc != SPH_OK) return rc;
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
     const dim3 b2(16, 16);
-    sph::k_splat_keys<<<(n + bs - 1) / bs, bs, 0, s>>>(v, n, x->b.pos, sorted, key);
+    const int shift = tile_shift(view);
+    if (shift > 0) {
+        const int tw = (v.w + (1 << shift) - 1) >> shift, th = (v.h + (1 << shift) - 1) >> shift;
+        const int cw = (tw + 3) / 4, ch = (th + 3) / 4;
+        unsigned* const coarse = tile + ntiles + 2;
+        sph::k_cover<<<(n + bs - 1) / bs, bs, 0, s>>>(v, n, x->b.pos, shift, tw, tile);
+        const unsigned cap = (unsigned)splat_list_cap(n);
+        sph::k_tile_max<<<(cw * ch + bs - 1) / bs, bs, 0, s>>>(tw, th, tile, cw, ch, coarse);
+        sph::k_splat_cull<<<(n + bs - 1) / bs, bs, 0, s>>>(v, n, x->b.pos, shift, tw, tile, cw, coarse, key, list, cap,
+                                                           tile + ntiles);
+        sph::k_splat_pairs<<<4 * x->num_sms, bs, 0, s>>>(v, x->b.pos, shift, tw, key, list, cap, tile + ntiles);
+    } else {
+        const int32_t* sorted;
+        if ((rc = splat_order(x, v, sorted)) != SPH_OK) return rc;
+        sph::k_splat_keys<<<(n + bs - 1) / bs, bs, 0, s>>>(v, n, x->b.pos, sorted, key);
+    }
     sph::k_splat_resolve<<<sph::grid2(v.w, v.h, b2), b2, 0, s>>>(v, x->b.pos, key, d_depth);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return sph_ctx_fail(x, SPH_E_CUDA, std::string("render launch: ") + cudaGetErrorString(e));
@@ -570,8 +804,12 @@ int sph_render_particles(sph_ctx* x, const sph_view* view, const sph_light* ligh
     }
     sph::View v;
     unsigned long long* key;
+    unsigned* tile;
+    int2* list;
+    size_t ntiles;
     const int32_t* sorted;
-    const int rc = splat_prepare(x, view, v, key, sorted);
+    int rc = splat_prepare(x, view, v, key, tile, list, ntiles);
+    if (rc == SPH_OK) rc = splat_order(x, v, sorted);
     if (rc != SPH_OK) return rc;
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
@@ -586,7 +824,7 @@ int sph_render_particles(sph_ctx* x, const sph_view* view, const sph_light* ligh
 
 int sph_filter_bilateral(const float* d_in, float* d_out, int width, int height, void* stream) {
     if (!d_in || !d_out || !sph::image_ok(width, height) || d_in == d_out) return SPH_E_INVALID;
-    const dim3 b(16, 16);
+    const dim3 b(sph::kBilW, sph::kBilH);
     sph::k_bilateral<<<sph::grid2(width, height, b), b, 0, (cudaStream_t)stream>>>(d_in, d_out, width, height);
     return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_E_CUDA;
 }
@@ -594,7 +832,7 @@ int sph_filter_bilateral(const float* d_in, float* d_out, int width, int height,
 int sph_render_smooth(float* d_depth, float* d_tmp, int width, int height, int iterations, void* stream) {
     if (!d_depth || !d_tmp || !sph::image_ok(width, height) || iterations < 0 || d_depth == d_tmp)
         return SPH_E_INVALID;
-    const dim3 b(16, 16);
+    const dim3 b(sph::kBilW, sph::kBilH);
     const cudaStream_t s = (cudaStream_t)stream;
     for (int it = 0; it < iterations; ++it) {
         sph::k_bilateral<<<sph::grid2(width, height, b), b, 0, s>>>(d_depth, d_tmp, width, height);
