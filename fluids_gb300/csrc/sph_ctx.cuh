@@ -87,8 +87,8 @@ struct sph_ctx {
     double* d_scene_stats = nullptr;
     int inject = 0;   /* one-shot fault for the next step (sph_inject_fault) */
     bool inject_alloc = false;   /* the next arena allocation fails (sph_inject_fault) */
-    /* depth-test scratch of sph_render_depth: 8 bytes per pixel, 4 per tile of 4 x 4 pixels, 8
-     * per particle and 65,536 more for the list of pairs to splat */
+    /* depth-test scratch of sph_render_depth: 8 bytes per pixel, 4 per tile of 4 x 4 pixels,
+     * and the list of pairs to splat: 16 per particle and up to 4 MB more */
     void* render_buf = nullptr;
     size_t render_bytes = 0;
     void* render_sort = nullptr;   /* sph_render_depth: 16-bit depth keys and particle order */

@@ -24,6 +24,7 @@
  * Images are row-major, row 0 at the bottom (window coordinates), single-channel float
  * (depth) or float4 (normals); reads outside the image clamp to the edge.
  */
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <utility>
@@ -176,9 +177,11 @@ __global__ void __launch_bounds__(256) k_cover(View v, int n, const float4* __re
         if (pole >= e[2] - 1e-3f * v.radius && pole <= hi) return;
     }
     const float lin_hi = lin(hi);
-    /* the tiles inside the middle of the disc (0.6 of its radius), where the bound is tight */
+    /* the tiles inside the middle of the disc (0.6 of its radius), where the bound is tight; of a
+     * small disc, as much of it as holds a tile wherever it lies */
     const int side = 1 << shift;
-    const float inv = 2.0f / size, half = 0.3f * size, scale = 1.0f / (float)side;
+    const float inv = 2.0f / size, scale = 1.0f / (float)side;
+    const float half = fmaxf(0.3f * size, fminf(0.45f * size, 0.9f * (float)side));
     const int tx0 = max(0, (int)ceilf((wx - half) * scale)), tx1 = min(tw, (int)floorf((wx + half) * scale));
     const int ty0 = max(0, (int)ceilf((wy - half) * scale)),
               ty1 = min((v.h + side - 1) >> shift, (int)floorf((wy + half) * scale));
@@ -687,8 +690,9 @@ static int tile_shift(const sph_view* view) {
     return size < 24.0f ? 2 : (size < 48.0f ? 3 : 4);
 }
 
-/* Entries of the list of (particle, tile) pairs to splat. */
-static size_t splat_list_cap(int n) { return (size_t)n + 65536; }
+/* Entries of the list of (particle, tile) pairs to splat: a sprite of a few particles may show in
+ * all of its tiles, in a crowd one in a hundred pairs does. */
+static size_t splat_list_cap(int n) { return std::min(32 * (size_t)n, 2 * (size_t)n + 524288); }
 
 /* Checks the view, allocates the depth-test keys, the list of pairs, the tile bounds and the
  * pair count (behind the ntiles bounds, before the coarse ones), and clears keys, bounds and

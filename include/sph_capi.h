@@ -381,7 +381,7 @@ typedef struct sph_view {
  * pixel the NDC depth of the nearest sprite fragment (GL_LESS on the normalised depth, the
  * lower particle index winning a tie) and 0 where no sprite covers it.  No background
  * depth texture: fragments beyond the far plane are dropped.  Runs on the context stream;
- * holds about 8.3 bytes per pixel and 8 bytes per particle of scratch in the context. */
+ * holds about 8.3 bytes per pixel, 16 per particle and up to 4 MB more of scratch in the context. */
 int sph_render_depth(sph_ctx* ctx, const sph_view* view, float* d_depth);
 /* One pass of kernels/bilateral.cl (BilateralFilter::filter, filters/bilateralfilter.cpp:
  * 28-41): d_in and d_out must differ. */
