@@ -399,9 +399,9 @@ void backward_pairs(sph_adj* a, int k, const float4* xk, const int32_t* lk, cons
     const cudaStream_t s = a->ctx->stream;
     const size_t sn = (size_t)a->N;
     const int g = sph::blocks(a->N * W, 256);
-    sph::launch_chained(s, sph::k_adj_forces_bwd<W>, g, 256, 0, a->c, a->N, xk, a->tv + k * sn, a->taux + k * sn, a->la,
+    sph::launch_early(true, s, sph::k_adj_forces_bwd<W>, g, 256, 0, a->c, a->N, xk, a->tv + k * sn, a->taux + k * sn, a->la,
                         lk, nk, a->lrho, a->lxf, a->lv[nx], a->gmu, a->gk);
-    sph::launch_chained(s, sph::k_adj_density_bwd<W>, g, 256, 0, a->c, a->N, xk, a->lrho, lk, nk, a->lx[cur], a->lxf,
+    sph::launch_early(true, s, sph::k_adj_density_bwd<W>, g, 256, 0, a->c, a->N, xk, a->lrho, lk, nk, a->lx[cur], a->lxf,
                         a->lx[nx]);
 }
 
@@ -549,7 +549,7 @@ int sph_adj_backward(sph_adj* a, const float* gxT_4, const float* gvT_4, float* 
             const float4* xk = a->tx + k * sn;
             const int32_t* lk = a->tlist + (size_t)k * a->cap * sn;
             const int32_t* nk = a->tlen + k * sn;
-            sph::launch_chained(s, sph::k_adj_integrate_bwd, sph::blocks(n, bs), bs, 0, a->c, n, xk, a->tu + k * sn,
+            sph::launch_early(true, s, sph::k_adj_integrate_bwd, sph::blocks(n, bs), bs, 0, a->c, n, xk, a->tu + k * sn,
                                 a->ta + k * sn, a->lx[cur], a->lv[cur], a->lu[cur], a->la, a->lu[nx], a->flags);
             switch (sph::walk_lanes(n, a->ctx->num_sms)) {
             case 8: backward_pairs<8>(a, k, xk, lk, nk, cur, nx); break;

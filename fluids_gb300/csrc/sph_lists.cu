@@ -105,7 +105,9 @@ constexpr int kMaxCap = 128;
 
 template <bool BATCH, bool REMAP, bool PCI>
 static void split_launch(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap) {
-    launch_chained(s, k_lists_split<BATCH, REMAP, PCI>, (c.n + kPer - 1) / kPer, kSplitThreads,
+    /* the adjoint's steps are not captured, and early launches save more there */
+    const int grid = (c.n + kPer - 1) / kPer;
+    launch_early(REMAP || grid <= kEarlyBlocks, s, k_lists_split<BATCH, REMAP, PCI>, grid, kSplitThreads,
                    sizeof(float2) * kPer * (size_t)(c.cap | 1), c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist,
                    b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes, b.scene_of, remap, b.flags,
                    b.bnear, b.prho);
