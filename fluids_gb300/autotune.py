@@ -2,7 +2,7 @@
 
 The threads per block of the step's kernels (sph_set_block_size) are chosen by timing a
 few steps of the live context at each candidate and keeping the fastest; for a batched
-context the candidates are the shapes of its persistent tile launches -- threads per block
+context the candidates are the shapes of its tiled launches -- threads per block
 and CTAs per SM (sph_set_tile_shape) of the grid whose warps take the 32-particle scene
 tiles.  The choice is
 stored in a JSON file keyed by GPU name, method, mode, batched or not, and the particle
@@ -20,7 +20,7 @@ import os
 import time
 
 CANDIDATES = (64, 128, 256)
-# CTAs per SM of a batched context's persistent tile launches (0: 2048 / block size)
+# CTAs per SM of a batched context's tiled launches (0: as many as give each tile a warp)
 TILE_CTAS = (0, 2, 4)
 
 

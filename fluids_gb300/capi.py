@@ -526,11 +526,11 @@ class BatchContext(Context):
         return np.array(out[:], dtype=np.float64).reshape(self.nscenes, 8)
 
     def set_tile_shape(self, ctas_per_sm):
-        """CTAs per SM of the persistent per-scene tile launches (0: 2048 / block size)."""
+        """CTAs per SM of the per-scene tiled launches (0: a warp for each tile)."""
         self._c(self._lib.sph_set_tile_shape(self.h, int(ctas_per_sm)))
 
     def tile_shape(self):
-        """{tile_particles, ctas_per_sm, tiles, blocks} of the persistent tile launches."""
+        """{tile_particles, ctas_per_sm, tiles, blocks} of the tiled launches."""
         v = [C.c_int() for _ in range(4)]
         self._c(self._lib.sph_get_tile_shape(self.h, *[C.byref(x) for x in v]))
         return dict(zip(("tile_particles", "ctas_per_sm", "tiles", "blocks"), [x.value for x in v]))

@@ -194,6 +194,7 @@ int derive(sph_ctx* x) {
             sd.ox = o[0]; sd.oy = o[1]; sd.oz = o[2];
             sd.nx = n[0]; sd.ny = n[1]; sd.nz = n[2];
             sd.ncells = (long long)n[0] * n[1] * n[2];
+            sph::neigh_linear_offsets(n[0], n[1], sd.noff);
             sd.cell_base = base;
             base += sd.ncells;
             sd.lim_x = in.lim[0]; sd.lim_y = in.lim[1]; sd.lim_z = in.lim[2];
@@ -284,14 +285,13 @@ void carve(sph_ctx* x, Carver& cv) {
         x->d_scene_of = cv.take<int32_t>(n);
         x->d_scene_stats = cv.take<double>(8 * x->scene_in.size());
     }
-    /* persistent scene tiles: at most one per 32 particles of a scene plus one per scene */
+    /* scene tiles: at most one per 32 particles of a scene plus one per scene */
     b.tiles = cv.take<sph::SceneTile>(x->scene_in.empty() ? 1 : n / sph::kTileParticles + x->scene_in.size() + 1);
-    b.tile_next = cv.take<unsigned>(4);
 }
 
 /* The scene tile table of a batched context: each scene's particle range cut into tiles of
- * at most 32 particles (one warp), in scene order; and the grid of the persistent launches
- * whose CTAs take chunks of tiles from a counter.  Uploaded synchronously (a host vector). */
+ * at most 32 particles (one warp), in scene order; and the grid of the tiled launches: a warp
+ * per tile, or the CTAs per SM that were set.  Uploaded synchronously (a host vector). */
 int upload_tiles(sph_ctx* x) {
     x->c.ntiles = 0;
     x->c.tile_blocks = 0;
@@ -304,11 +304,10 @@ int upload_tiles(sph_ctx* x) {
             x->h_tiles.push_back(sph::SceneTile{(int)sc, first + a, count - a < T ? count - a : T, 0});
     }
     if (x->h_tiles.empty()) return SPH_OK;
-    const int per_sm = x->tile_ctas > 0 ? x->tile_ctas : (2048 / x->bs > 0 ? 2048 / x->bs : 1);
-    const long long blocks = (long long)x->num_sms * per_sm;
     x->c.ntiles = (int)x->h_tiles.size();
     const long long warps_needed = (x->c.ntiles + x->bs / 32 - 1) / (x->bs / 32);
-    x->c.tile_blocks = (int)(blocks < warps_needed ? blocks : warps_needed);
+    const long long set = (long long)x->num_sms * x->tile_ctas;
+    x->c.tile_blocks = (int)(0 < set && set < warps_needed ? set : warps_needed);
     SPH_CUDA(x, cudaStreamSynchronize(x->stream));
     SPH_CUDA(x, cudaMemcpy(const_cast<sph::SceneTile*>(x->b.tiles), x->h_tiles.data(),
                            sizeof(sph::SceneTile) * x->h_tiles.size(), cudaMemcpyHostToDevice));
@@ -757,6 +756,7 @@ int rebuild(sph_ctx* x, bool keep) {
         sd.ncells = c.ncells;
         sd.lim_x = c.lim_x; sd.lim_y = c.lim_y; sd.lim_z = c.lim_z;
         sd.mu = c.mu; sd.kgas = c.kgas;
+        sph::neigh_linear_offsets(c.nx, c.ny, sd.noff);
         sd.first = 0; sd.count = x->N; sd.first_b = 0; sd.count_b = x->NB;
         x->h_scenes.assign(1, sd);
     } else {

@@ -63,7 +63,7 @@ struct sph_ctx {
     int max_iter_slots = 1;
     int coop_blocks = 0;
     int bs = 256;
-    int tile_ctas = 0;   /* batched: CTAs per SM of the persistent tile launches (0: 2048 / bs) */
+    int tile_ctas = 0;   /* batched: CTAs per SM of the tiled launches (0: a warp per tile) */
     std::vector<sph::SceneTile> h_tiles;
     bool graph_ok = true;
     cudaGraphExec_t gexec = nullptr;

@@ -40,7 +40,7 @@ struct Const {
     int scene_shift;     /* Morton bits below the scene id in the sort key */
     int monaghan;        /* COMPAT with the Monaghan kernels (sph_params::kernels) */
     int ntiles;          /* batched: entries of the scene tile table (SceneTile) */
-    int tile_blocks;     /* batched: CTAs of a persistent launch over the tiles */
+    int tile_blocks;     /* batched: CTAs of a launch over the tiles */
     int block0, blocks;  /* single-scene passes launched in parts: blocks [block0, block0 + blocks)
                             of the whole pass (0, 0: the whole pass in one launch) */
     int first, last;     /* the particles [first, last) of a launch with several lanes a particle */
@@ -54,15 +54,22 @@ struct SceneDev {
     long long cell_base, ncells;
     float lim_y, lim_z, mu, kgas;
     int count, first_b, count_b, pad;
+    int32_t noff[28];   /* the 27 linear neighbour-cell offsets of its grid (neigh_linear_offsets) */
 };
 
 /* The constants of the scene a particle belongs to: grid, viscosity, stiffness, container. */
-__device__ __forceinline__ void apply_scene(Const& c, const SceneDev& s) {
+__device__ __forceinline__ void apply_scene_grid(Const& c, const SceneDev& s) {
     c.ox = s.ox; c.oy = s.oy; c.oz = s.oz;
     c.nx = s.nx; c.ny = s.ny; c.nz = s.nz;
     c.ncells = s.ncells;
+}
+__device__ __forceinline__ void apply_scene_state(Const& c, const SceneDev& s) {
     c.mu = s.mu; c.kgas = s.kgas;
     c.lim_x = s.lim_x; c.lim_y = s.lim_y; c.lim_z = s.lim_z;
+}
+__device__ __forceinline__ void apply_scene(Const& c, const SceneDev& s) {
+    apply_scene_grid(c, s);
+    apply_scene_state(c, s);
 }
 /* Switches c to particle i's scene and returns that scene's offset in the cell tables.
  * Every context has a scene table (one entry for a single scene, scene_of null), and the
@@ -82,48 +89,52 @@ struct SceneTile {
     int scene, first, count, pad;
 };
 
-/* Runs f(c, cell_base, i) for the particles of a launch.  Single scene (BATCH = false): one
- * particle per thread of a flat grid, the parameter's constants.  Batched: a persistent
- * grid of tile_blocks CTAs takes the scene tiles from a counter (*next, zero before the
- * launch), one contiguous chunk of blockDim / 32 tiles per CTA at a time, one tile per
- * warp, so the work balances dynamically however uneven the tiles are and the warps of a
- * CTA work on adjacent particles (whose neighbour cells they share in L1); a tile's scene
- * constants are read once, at a warp-uniform address, for its 32 particles (one per lane),
- * instead of being looked up per particle.  f must not use warp-collective operations (a
- * tile's lanes beyond its count are idle). */
-/* W > 1 (single scene): W adjacent threads per particle, all of them running f(c, 0, i) to its
- * end (it sums over them); threads past the last particle run it for the last one, which f
- * tells by lane_of_particle. */
+/* Runs f(c, cell_base, i, scene) for the particles of a launch.  Single scene (BATCH = false):
+ * one particle per thread of a flat grid, the parameter's constants, no scene.  Batched: one
+ * scene tile per warp (its particles one per lane; the lanes beyond its count are idle, so f
+ * must not use warp-collective operations), with the grid constants of the tile's scene; f
+ * takes the other constants of the scene by late_scene where it needs them, so that they are
+ * not held in registers along its neighbour walk.  The grid is one warp per tile, or the
+ * CTAs per SM that the caller set, which then stride over the tiles.  Measured on GB300 (40
+ * scenes, 662,935 particles; one CTA chunk of tiles at a time from a counter before): list
+ * pass 200 -> 186 us, forces 116 -> 108, normals 54 -> 51, a step 457 -> 420, also through
+ * the three memsets of the counters. */
+/* W > 1: W adjacent threads per particle, all of them running f to its end (it sums over
+ * them); threads past the last particle run it for the last one, which f tells by
+ * lane_of_particle.  The scene is the particle's by scene_of, and f, which walks the lists
+ * only, gets neither its grid nor its place in the cell tables. */
 template <bool BATCH, int W = 1, class F>
 __device__ __forceinline__ void for_each_particle(const Const& c0, const SceneTile* __restrict__ tiles,
-                                                  const SceneDev* __restrict__ scenes, unsigned* next, F&& f) {
+                                                  const SceneDev* __restrict__ scenes, F&& f,
+                                                  const int32_t* __restrict__ scene_of = nullptr) {
     if constexpr (W > 1) {
         const int i = c0.first + ((int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x) / W;
-        f(c0, 0LL, i < c0.last ? i : c0.last - 1);
+        const int q = i < c0.last ? i : c0.last - 1;
+        f(c0, 0LL, q, BATCH && scene_of ? scenes + __ldg(&scene_of[q]) : scenes);
     } else if constexpr (BATCH) {
-        __shared__ int s_chunk;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+        const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
 #pragma unroll 1
-        for (;;) {
-            if (threadIdx.x == 0) s_chunk = (int)atomicAdd(next, (unsigned)warps);
-            __syncthreads();
-            const int t = s_chunk + warp;
-            __syncthreads();   /* every thread has read s_chunk before it is written again */
-            if (t - warp >= c0.ntiles) break;
-            if (t < c0.ntiles) {
-                const SceneTile tl = tiles[t];
-                if (lane < tl.count) {
-                    Const c = c0;
-                    const SceneDev& sd = scenes[tl.scene];
-                    apply_scene(c, sd);
-                    f(c, sd.cell_base, tl.first + lane);
-                }
+        for (int t = blockIdx.x * warps + (threadIdx.x >> 5); t < c0.ntiles; t += gridDim.x * warps) {
+            const SceneTile tl = tiles[t];
+            if (lane < tl.count) {
+                Const c = c0;
+                const SceneDev& sd = scenes[tl.scene];
+                apply_scene_grid(c, sd);
+                f(c, sd.cell_base, tl.first + lane, &sd);
             }
         }
     } else {
         const int i = (c0.block0 + (int)blockIdx.x) * (int)blockDim.x + (int)threadIdx.x;
-        if (i < c0.n) f(c0, 0LL, i);
+        if (i < c0.n) f(c0, 0LL, i, scenes);
     }
+}
+
+/* c with the remaining constants of the scene (batched; a single scene's are the parameter's). */
+template <bool BATCH>
+__device__ __forceinline__ Const late_scene(const Const& c, const SceneDev* sd) {
+    Const r = c;
+    if constexpr (BATCH) apply_scene_state(r, *sd);
+    return r;
 }
 
 /* This thread's place among the W of its particle, W for a thread past the last particle. */
@@ -731,18 +742,7 @@ __device__ __forceinline__ float pown7(float x) {
 }
 /* kernels/surface_tension.h:23-50 */
 __device__ __forceinline__ float st_corr(float rho0, float di, float dj) { return 2.0f * rho0 / (di + dj); }
-__device__ __forceinline__ float st_kernel(float r, float h, float c) {
-    if (r <= 0.5f * h) {
-        float t1 = h - r;
-        float t2 = (t1 * t1 * t1) * (r * r * r);
-        return 2.0f * t2 - c;
-    } else if (r <= h) {
-        float t1 = h - r;
-        return (t1 * t1 * t1) * (r * r * r);
-    }
-    return 0.0f;
-}
-/* st_kernel with selects instead of branches (same arithmetic, same values). */
+/* the surface tension kernel with selects instead of its branches (same arithmetic, same values) */
 __device__ __forceinline__ float st_kernel_sel(float r, float h, float c) {
     const float t1 = h - r;
     const float t2 = (t1 * t1 * t1) * (r * r * r);

@@ -58,7 +58,6 @@ struct Bufs {
     const SceneDev* scenes;
     const int32_t* scene_of;
     const SceneTile* tiles;                /* batched: per-scene tiles of 32 particles (Const::ntiles) */
-    unsigned* tile_next;                   /* batched: the tile counters of the four tiled passes */
     /* status */
     unsigned* flags;
     int32_t* pci_iters;

@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(256) k_wc_density(Const c0, Neigh<LIST, COMPAT
                                                     const float* __restrict__ bphi_s, float* __restrict__ dens,
                                                     float* __restrict__ pres, float4* __restrict__ aux,
                                                     const SceneDev* __restrict__ scenes,
-                                                    const SceneTile* __restrict__ tiles, unsigned* next) {
-  for_each_particle<BATCH>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
+                                                    const SceneTile* __restrict__ tiles) {
+  for_each_particle<BATCH>(c0, tiles, scenes, [&](const Const& c, long long base, int i, const SceneDev* sd) {
     Neigh<LIST, COMPAT> fl = fl0, bl = bl0;
     fl.tab += base;
     bl.tab += base;
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) k_wc_density(Const c0, Neigh<LIST, COMPAT
     }
     di += c.poly6_eval * bdi;
     dens[i] = di;
-    const float pv = c.kgas * (pown7(di / c.rho0) - 1.0f);
+    const float pv = late_scene<BATCH>(c, sd).kgas * (pown7(di / c.rho0) - 1.0f);
     const float p = (0.f < pv) ? pv : 0.f;
     pres[i] = p;
     aux[i] = make_aux(di, p);
@@ -98,14 +98,14 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
                                                        int* __restrict__ sblen, float* __restrict__ dens,
                                                        float* __restrict__ pres, float4* __restrict__ aux,
                                                        const SceneDev* __restrict__ scenes,
-                                                       const SceneTile* __restrict__ tiles, unsigned* next,
+                                                       const SceneTile* __restrict__ tiles,
                                                        const int32_t* __restrict__ remap = nullptr,
                                                        unsigned* __restrict__ flags = nullptr,
                                                        const uint8_t* __restrict__ bnear = nullptr,
                                                        const int32_t* __restrict__ noff = nullptr,
                                                        float4* __restrict__ prho = nullptr) {
   chain_next();
-  for_each_particle<BATCH>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
+  for_each_particle<BATCH>(c0, tiles, scenes, [&](const Const& c, long long base, int i, const SceneDev* sd) {
     const int2* __restrict__ ftab = tab0 + base;
     const int2* __restrict__ fbtab = btab0 + base;
     const float4 pi = spos[i];
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
     float di = 0.f;
     char* const lrow = reinterpret_cast<char*>(nlist + row);
     const unsigned n4 = 4u * (unsigned)c.n;
-    const int k = build_scan(c, pi.x, pi.y, pi.z, cx, cy, cz, ftab, spos, BATCH ? nullptr : noff,
+    const int k = build_scan(c, pi.x, pi.y, pi.z, cx, cy, cz, ftab, spos, BATCH ? sd->noff : noff,
                              [&](bool hit, int j, float r2, int slot) {
         if (hit) *list_slot(lrow, slot, n4) = REMAP ? __ldg(&remap[j]) : j;
         if (COMPAT && c.monaghan) {
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
     const bool scan_b = c.wrap || bnear == nullptr || bnear[base + cell_lin(c, cx, cy, cz)] != 0;
     if (c.nb > 0 && !REMAP && scan_b) {
         char* const brow = reinterpret_cast<char*>(sblist + i);
-        kb = build_scan(c, pi.x, pi.y, pi.z, cx, cy, cz, fbtab, bpos_s, BATCH ? nullptr : noff,
+        kb = build_scan(c, pi.x, pi.y, pi.z, cx, cy, cz, fbtab, bpos_s, BATCH ? sd->noff : noff,
                         [&](bool hit, int j, float r2, int slot) {
             if (hit) *list_slot(brow, slot, n4) = j;
             float w = 0.f;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
     di += c.poly6_eval * bdi;
     dens[row] = di;
     if (prho) prho[row] = make_float4(pi.x, pi.y, pi.z, di);   /* the normal pass's neighbour records */
-    const float pv = c.kgas * (pown7(di / c.rho0) - 1.0f);
+    const float pv = late_scene<BATCH>(c, sd).kgas * (pown7(di / c.rho0) - 1.0f);
     const float p = (0.f < pv) ? pv : 0.f;
     pres[row] = p;
     aux[row] = make_aux(di, p);
@@ -191,11 +191,11 @@ template <bool LIST, bool EXACT, bool BATCH, bool MON = false, bool PRHO = false
 __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl0, const float4* __restrict__ aux,
                                                  const float* __restrict__ dens, float4* __restrict__ normal,
                                                  const SceneDev* __restrict__ scenes,
-                                                 const SceneTile* __restrict__ tiles, unsigned* next,
+                                                 const SceneTile* __restrict__ tiles,
                                                  const float4* __restrict__ vel_s = nullptr,
                                                  float4* __restrict__ nrec = nullptr) {
   chain_next();
-  for_each_particle<BATCH, W>(c0, tiles, scenes, next, [&](const Const& c, long long base, int i) {
+  for_each_particle<BATCH, W>(c0, tiles, scenes, [&](const Const& c, long long base, int i, const SceneDev*) {
     Neigh<LIST, EXACT> fl = fl0;
     fl.tab += base;
     const float4 pi = __ldg(&fl.npos[i]);
@@ -294,7 +294,7 @@ __device__ __forceinline__ void wc_integrate_one(const Const& c, float4 p, float
 template <bool COMPAT, bool LIST, bool FUSE, bool WRITE_ACC, bool ST, bool BATCH, bool PACK = false, int W = 1>
 __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const c0, Neigh<LIST, COMPAT> fl0, Neigh<LIST, COMPAT> bl0, Bufs b) {
   chain_next();
-  for_each_particle<BATCH, W>(c0, b.tiles, b.scenes, b.tile_next + 3, [&](const Const& c, long long base, int i) {
+  for_each_particle<BATCH, W>(c0, b.tiles, b.scenes, [&](const Const& c, long long base, int i, const SceneDev* sd) {
     const int w = W > 1 ? lane_of_particle<W>(c) : 0;
     Neigh<LIST, COMPAT> fl = fl0, bl = bl0;
     fl.tab += base;
@@ -328,7 +328,6 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
             bl.visit(c, i, pi.x, pi.y, pi.z, pair);
         }
     };
-    if (BATCH) boundary_pairs();
     float4 ni = make_float4(0.f, 0.f, 0.f, 0.f);
     if (ST) ni = __ldg(&b.normal[i]);
     float pax = 0.f, pay = 0.f, paz = 0.f, vax = 0.f, vay = 0.f, vaz = 0.f;
@@ -364,8 +363,8 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
                 cux += (ni.x - nj.x) * K;
                 cuy += (ni.y - nj.y) * K;
                 cuz += (ni.z - nj.z) * K;
-                /* selects in the single-scene kernel (0.666 -> 0.636 ms), branches in the batched one */
-                const float ck = (BATCH ? st_kernel(rn, h, c.st_term) : st_kernel_sel(rn, h, c.st_term)) * K * irn;
+                /* selects, not branches: 0.666 -> 0.636 ms at 4M */
+                const float ck = st_kernel_sel(rn, h, c.st_term) * K * irn;
                 cox += dx * ck;
                 coy += dy * ck;
                 coz += dz * ck;
@@ -376,16 +375,15 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
         list_neighbors_split<W>(i, c.n, fl.list, w < W ? __ldg(&fl.len[i]) : 0, w, i, fl.npos, pi.x, pi.y, pi.z, pair);
     else
         /* the list walk SPH_FORCES_WALK (four) entries deep with the next entries loaded during
-         * the visits and a predicated last batch, single-scene; the batched kernel walks two
-         * deep with a serial tail (measured faster there) */
-        fl.template visit<true, BATCH ? 2 : SPH_FORCES_WALK, !BATCH>(c, i, pi.x, pi.y, pi.z, pair);
-    /* single scene: the boundary pairs after the fluid pairs, so that their sums are not live
-     * during the fluid walk (each term keeps its own accumulator, so the result is the same);
-     * the batched kernel measured faster with them first (2.46 vs 2.59 ms per batched step) */
-    if (!BATCH) boundary_pairs();
+         * the visits and a predicated last batch */
+        fl.template visit<true, SPH_FORCES_WALK, true>(c, i, pi.x, pi.y, pi.z, pair);
+    /* the boundary pairs after the fluid pairs, so that their sums are not live during the
+     * fluid walk (each term keeps its own accumulator) */
+    boundary_pairs();
+    const Const cl = late_scene<BATCH>(c, sd);
     const float m = c.mass;
     pax *= -m; pay *= -m; paz *= -m;
-    const float vs = COMPAT ? (c.visc_lapl * c.mu) : (c.visc_lapl * c.mu) * (m * ai.y);
+    const float vs = COMPAT ? (c.visc_lapl * cl.mu) : (c.visc_lapl * cl.mu) * (m * ai.y);
     vax *= vs; vay *= vs; vaz *= vs;
     float ax = pax + vax + bax, ay = c.g + pay + vay + bay, az = paz + vaz + baz;
     if constexpr (W > 1) {
@@ -406,14 +404,14 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
     if (FUSE) {
         float4 po, vo, vho;
         bool bad;
-        wc_integrate_one(c, pi, __ldg(&b.vhalf_s[i]), ax, ay, az, po, vo, vho, bad);
+        wc_integrate_one(cl, pi, __ldg(&b.vhalf_s[i]), ax, ay, az, po, vo, vho, bad);
         b.pos[i] = po;
         b.vel[i] = vo;
         b.vhalf[i] = vho;
         b.ids[i] = __ldg(&b.ids_s[i]);
         if (bad) atomicOr(b.flags, kFlagNan);
     }
-  });
+  }, b.scene_of);
 }
 
 __global__ void __launch_bounds__(256) k_wc_integrate(Const c0, Bufs b) {
@@ -433,18 +431,11 @@ __global__ void __launch_bounds__(256) k_wc_integrate(Const c0, Bufs b) {
 }
 
 static inline int nblk(int n, int bs) { return (n + bs - 1) / bs; }
-/* grid of a launch: one particle per thread, or the persistent tile grid of a batched context */
+/* grid of a launch: one particle per thread, or the tile grid of a batched context */
 template <bool BATCH>
 static inline int grid_for(const Const& c, int bs) {
     if constexpr (BATCH) return c.tile_blocks > 0 ? c.tile_blocks : 1;
     return c.blocks > 0 ? c.blocks : nblk(c.n, bs);
-}
-/* a batched pass's tile counter, zeroed on the stream before its launch (slot: 0 density,
- * 1 list build, 2 normals, 3 forces) */
-static unsigned* tile_counter(cudaStream_t s, const Bufs& b, int slot, bool batched) {
-    if (!batched) return nullptr;
-    cudaMemsetAsync(b.tile_next + slot, 0, sizeof(unsigned), s);
-    return b.tile_next + slot;
 }
 
 template <bool LIST, bool EXACT>
@@ -458,10 +449,9 @@ static Neigh<LIST, EXACT> bnd_src(const Bufs& b) {
 
 template <bool COMPAT, bool LIST, bool BATCH>
 static void density_launch(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
-    unsigned* next = tile_counter(s, b, 0, BATCH);
     k_wc_density<COMPAT, LIST, BATCH><<<grid_for<BATCH>(c, bs), bs, 0, s>>>(c, fluid_src<LIST, COMPAT>(b),
                                                                    bnd_src<LIST, COMPAT>(b), b.bphi_s, b.density,
-                                                                   b.pressure, b.aux, b.scenes, b.tiles, next);
+                                                                   b.pressure, b.aux, b.scenes, b.tiles);
 }
 
 /* Batched contexts exist only in PHYSICS mode, so the scene lookup is compiled for that mode alone. */
@@ -486,10 +476,9 @@ void launch_wc_density(cudaStream_t s, const Const& c, const Bufs& b, bool lists
 
 template <bool COMPAT, bool BATCH>
 static void lists_density_launch(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
-    unsigned* next = tile_counter(s, b, 1, BATCH);
     launch_chained(s, k_lists_density<COMPAT, BATCH>, grid_for<BATCH>(c, bs), bs, 0, c, b.pos_s, b.tab, b.bpos_s,
                    b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes,
-                   b.tiles, next, nullptr, nullptr, b.bnear, b.noff, b.prho);
+                   b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho);
 }
 
 void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
@@ -497,7 +486,7 @@ void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int
     if (launch_lists_split(s, c, b, true, nullptr, num_sms)) return;
     k_lists_density<false, false, false, true><<<nblk(c.n, bs), bs, 0, s>>>(
         c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
-        b.aux, b.scenes, b.tiles, nullptr, nullptr, nullptr, b.bnear, b.noff, b.prho);
+        b.aux, b.scenes, b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho);
 }
 void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap, int bs,
                                 int num_sms) {
@@ -505,7 +494,7 @@ void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, c
     if (launch_lists_split(s, c, b, false, remap, num_sms)) return;
     k_lists_density<false, false, true><<<nblk(c.n, bs), bs, 0, s>>>(
         c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
-        b.aux, b.scenes, b.tiles, nullptr, remap, b.flags);
+        b.aux, b.scenes, b.tiles, remap, b.flags);
 }
 
 void launch_lists_density(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
@@ -521,9 +510,10 @@ void launch_aux(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
     k_aux<<<nblk(c.n, bs), bs, 0, s>>>(c.n, b.density, b.pressure, b.aux);
 }
 
-/* The walks of the fused step of a single scene take several lanes a particle in small scenes
- * (walk_lanes); their sums then add by lane instead of in list order. */
-static int split_walk(const Const& c, int num_sms) { return c.batched || c.compat ? 1 : walk_lanes(c.n, num_sms); }
+/* The walks of the fused step take several lanes a particle in small contexts, of one scene or
+ * of many (walk_lanes); their sums then add by lane instead of in list order.  A batch of 3
+ * scenes with 14,332 particles: 387 -> 195 us for three steps, with the lists' lanes. */
+static int split_walk(const Const& c, int num_sms) { return c.compat ? 1 : walk_lanes(c.n, num_sms); }
 
 template <int W>
 static void normals_split(cudaStream_t s, const Const& c0, const Bufs& b, float4* nrec) {
@@ -532,8 +522,9 @@ static void normals_split(cudaStream_t s, const Const& c0, const Bufs& b, float4
     c.last = c.n;
     auto fl = fluid_src<true, true>(b);
     fl.npos = b.prho;
+    /* the lists hold a batch's pairs, so the pass is the same for it */
     launch_chained(s, k_normals<true, true, false, false, true, W>, nblk(c.n * W, 256), 256, 0, c, fl, b.aux,
-                   b.density, b.normal, b.scenes, b.tiles, nullptr, b.vel_s, nrec);
+                   b.density, b.normal, b.scenes, b.tiles, b.vel_s, nrec);
 }
 
 void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack, bool prho) {
@@ -548,14 +539,13 @@ void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, i
     }
     const int g = nblk(c.n, bs), gt = grid_for<true>(c, bs);
     float4* nrec = pack ? b.nrec : nullptr;
-    unsigned* next = tile_counter(s, b, 2, c.batched != 0);
     if (c.monaghan) {   /* COMPAT only */
         if (lists)
             k_normals<true, true, false, true><<<g, bs, 0, s>>>(c, fluid_src<true, true>(b), b.aux, b.density,
-                                                                b.normal, b.scenes, b.tiles, next, b.vel_s, nrec);
+                                                                b.normal, b.scenes, b.tiles, b.vel_s, nrec);
         else
             k_normals<false, true, false, true><<<g, bs, 0, s>>>(c, fluid_src<false, true>(b), b.aux, b.density,
-                                                                 b.normal, b.scenes, b.tiles, next);
+                                                                 b.normal, b.scenes, b.tiles);
         return;
     }
     if (lists) {
@@ -564,31 +554,31 @@ void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, i
         if (c.batched) {
             if (prho)
                 k_normals<true, true, true, false, true><<<gt, bs, 0, s>>>(c, fl, b.aux, b.density, b.normal,
-                                                                         b.scenes, b.tiles, next, b.vel_s, nrec);
+                                                                         b.scenes, b.tiles, b.vel_s, nrec);
             else
                 k_normals<true, true, true><<<gt, bs, 0, s>>>(c, fl, b.aux, b.density, b.normal, b.scenes, b.tiles,
-                                                              next, b.vel_s, nrec);
+                                                              b.vel_s, nrec);
         } else {
             if (prho)
                 launch_chained(s, k_normals<true, true, false, false, true>, g, bs, 0, c, fl, b.aux, b.density,
-                               b.normal, b.scenes, b.tiles, next, b.vel_s, nrec);
+                               b.normal, b.scenes, b.tiles, b.vel_s, nrec);
             else
                 k_normals<true, true, false><<<g, bs, 0, s>>>(c, fl, b.aux, b.density, b.normal, b.scenes, b.tiles,
-                                                              next, b.vel_s, nrec);
+                                                              b.vel_s, nrec);
         }
     } else if (c.compat) {
         k_normals<false, true, false><<<g, bs, 0, s>>>(c, fluid_src<false, true>(b), b.aux, b.density, b.normal,
-                                                       b.scenes, b.tiles, next);
+                                                       b.scenes, b.tiles);
     } else if (c.batched) {
         k_normals<false, false, true><<<gt, bs, 0, s>>>(c, fluid_src<false, false>(b), b.aux, b.density, b.normal,
-                                                        b.scenes, b.tiles, next);
+                                                        b.scenes, b.tiles);
     } else {
         k_normals<false, false, false><<<g, bs, 0, s>>>(c, fluid_src<false, false>(b), b.aux, b.density, b.normal,
-                                                        b.scenes, b.tiles, next);
+                                                        b.scenes, b.tiles);
     }
 }
 
-template <int W>
+template <bool BATCH, int W>
 static void forces_split(cudaStream_t s, const Const& c0, const Bufs& b, int bs, bool st) {
     Const c = c0;
     c.first = c0.block0 * bs;   /* a part of the pass covers the particles of its blocks of bs */
@@ -596,25 +586,24 @@ static void forces_split(cudaStream_t s, const Const& c0, const Bufs& b, int bs,
     auto fs = fluid_src<true, false>(b);
     auto bsrc = bnd_src<true, false>(b);
     const int g = nblk((c.last - c.first) * W, 256);
-    if (st) launch_chained(s, k_wc_forces<false, true, true, false, true, false, true, W>, g, 256, 0, c, fs, bsrc, b);
-    else launch_chained(s, k_wc_forces<false, true, true, false, false, false, false, W>, g, 256, 0, c, fs, bsrc, b);
+    if (st) launch_chained(s, k_wc_forces<false, true, true, false, true, BATCH, true, W>, g, 256, 0, c, fs, bsrc, b);
+    else launch_chained(s, k_wc_forces<false, true, true, false, false, BATCH, false, W>, g, 256, 0, c, fs, bsrc, b);
 }
 
 template <bool COMPAT, bool LIST, bool BATCH>
 static void forces_launch(cudaStream_t s, const Const& c, const Bufs& b, bool fuse, bool write_acc, int bs,
                           int num_sms, bool pack) {
     const int g = grid_for<BATCH>(c, bs);
-    tile_counter(s, b, 3, BATCH);
     const bool st = c.sigma != 0.f;
     auto fs = fluid_src<LIST, COMPAT>(b);
     auto bsrc = bnd_src<LIST, COMPAT>(b);
-    if constexpr (LIST && !COMPAT && !BATCH) {
+    if constexpr (LIST && !COMPAT) {
         /* the fused step's pass, without the acceleration field */
         if (fuse && !write_acc && pack == st) {
             switch (split_walk(c, num_sms)) {
-            case 8: forces_split<8>(s, c, b, bs, st); return;
-            case 4: forces_split<4>(s, c, b, bs, st); return;
-            case 2: forces_split<2>(s, c, b, bs, st); return;
+            case 8: forces_split<BATCH, 8>(s, c, b, bs, st); return;
+            case 4: forces_split<BATCH, 4>(s, c, b, bs, st); return;
+            case 2: forces_split<BATCH, 2>(s, c, b, bs, st); return;
             }
         }
     }

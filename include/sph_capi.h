@@ -306,15 +306,15 @@ int sph_set_block_size(sph_ctx* ctx, int block_size);
 
 /* Batched contexts (no counterpart in the reference, which steps one scene): the neighbour
  * passes of a batched step (list build + density, normals, forces + integration) run as
- * persistent launches over per-scene tiles -- each scene's particle range cut into tiles of
- * 32 particles, a tile never straddling two scenes -- whose CTAs take the next chunk of
- * tiles (one per warp) from a counter; a warp reads its tile's scene constants once.  The shape of the persistent grid is
- * block_size threads (sph_set_block_size) times SMs x ctas_per_sm CTAs (0 = 2048 /
- * block_size).  The shape never changes results; fluids_gb300/autotune.py picks it.
+ * launches over per-scene tiles -- each scene's particle range cut into tiles of 32
+ * particles, a tile never straddling two scenes -- with one tile per warp, which reads the
+ * scene's constants once.  The shape of the grid is block_size threads (sph_set_block_size)
+ * times SMs x ctas_per_sm CTAs, whose warps stride over the tiles (0 = as many CTAs as give
+ * every tile its warp).  The shape never changes results; fluids_gb300/autotune.py picks it.
  * SPH_E_INVALID on a single-scene context. */
 int sph_set_tile_shape(sph_ctx* ctx, int ctas_per_sm);
 /* The current tile shape: particles per tile, CTAs per SM (0 = automatic), tile count and
- * CTAs of the persistent launches. */
+ * CTAs of the tiled launches. */
 int sph_get_tile_shape(const sph_ctx* ctx, int* tile_particles, int* ctas_per_sm, int* ntiles, int* blocks);
 
 /* ---- differentiable WCSPH (adjoint) ----------------------------------------------------
