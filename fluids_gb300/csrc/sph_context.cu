@@ -241,7 +241,6 @@ void carve(sph_ctx* x, Carver& cv) {
     b.normal = cv.take<float4>(n); b.accel = cv.take<float4>(n); b.pos_pred = cv.take<float4>(n);
     b.f_other = cv.take<float4>(n); b.f_press = cv.take<float4>(n);
     b.density = cv.take<float>(n); b.pressure = cv.take<float>(n); b.dens_var = cv.take<float>(n);
-    b.pci_c = cv.take<float>(n);
     b.pci_pc = cv.take<float4>(n);
     b.aux = cv.take<float4>(n);
     b.nrec = cv.take<float4>(2 * n);
@@ -274,8 +273,9 @@ void carve(sph_ctx* x, Carver& cv) {
     b.body_dyn = cv.take<float>(8 * nbod);
     b.flags = cv.take<unsigned>(4);
     b.pci_iters = cv.take<int32_t>(4);
-    b.pci_maxerr = cv.take<float>((size_t)x->max_iter_slots);
-    b.barrier = cv.take<unsigned>(4);
+    /* the loop's barrier and the largest errors of its iterations, cleared together */
+    b.barrier = cv.take<unsigned>(4 + (size_t)x->max_iter_slots);
+    b.pci_maxerr = b.barrier ? reinterpret_cast<float*>(b.barrier + 4) : nullptr;
     b.stats = cv.take<double>(8);
     /* every context has a scene table; a single-scene context has one entry */
     x->d_scenes = cv.take<sph::SceneDev>(x->scene_in.empty() ? 1 : x->scene_in.size());
@@ -427,8 +427,7 @@ int run_stage_impl(sph_ctx* x, int stage) {
         sph::launch_pci_init_forces(s, c, b, bs, x->num_sms);
         break;
     case SPH_S_PCI_LOOP: {
-        cudaMemsetAsync(b.pci_maxerr, 0, sizeof(float) * x->max_iter_slots, s);
-        cudaMemsetAsync(b.barrier, 0, 4 * sizeof(unsigned), s);
+        cudaMemsetAsync(b.barrier, 0, sizeof(unsigned) * (4 + x->max_iter_slots), s);
         cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, c.pci_max_iter, x->coop_blocks, x->num_sms, false);
         if (e != cudaSuccess) return cuda_fail(x, e, "cooperative launch of the PCISPH loop");
         break;
@@ -594,8 +593,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
         }
         sph::launch_pci_init_forces(s, c, b, bs, x->num_sms, pack);
         mark(x, "k_pci_init_forces");
-        cudaMemsetAsync(b.pci_maxerr, 0, sizeof(float) * x->max_iter_slots, s);
-        cudaMemsetAsync(b.barrier, 0, 4 * sizeof(unsigned), s);
+        cudaMemsetAsync(b.barrier, 0, sizeof(unsigned) * (4 + x->max_iter_slots), s);
         if (x->any_massive) {
             cudaError_t e = sph::launch_pci_loop(s, c, b, c.pci_min_iter, pci_max_iter, x->coop_blocks, x->num_sms, false);
             if (e != cudaSuccess) return cuda_fail(x, e, "cooperative launch of the PCISPH loop");
@@ -838,7 +836,7 @@ int rebuild(sph_ctx* x, bool keep) {
         sph::launch_bnd_phi(s, x->c, b, x->p.boundary_phi_coeff > 0.f ? x->p.boundary_phi_coeff : 1.0f, x->bs);
         SPH_CUDA(x, cudaGetLastError());
     }
-    x->coop_blocks = sph::pci_loop_blocks(x->num_sms, x->bs);
+    x->coop_blocks = sph::pci_loop_blocks(x->num_sms);
     int trc = upload_tiles(x);
     if (trc != SPH_OK) return trc;
     x->has_state = true;
@@ -1267,7 +1265,6 @@ int sph_set_block_size(sph_ctx* x, int block_size) {
     cudaStreamSynchronize(x->stream);
     x->p.block_size = block_size;
     x->bs = block_size;
-    x->coop_blocks = sph::pci_loop_blocks(x->num_sms, x->bs);
     drop_graph(x);
     return upload_tiles(x);
 }

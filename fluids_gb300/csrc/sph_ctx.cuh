@@ -61,7 +61,7 @@ struct sph_ctx {
     char* arena = nullptr;
     size_t arena_bytes = 0;
     int max_iter_slots = 1;
-    int coop_blocks = 0;
+    sph::LoopBlocks coop_blocks{1, 1};
     int bs = 256;
     int tile_ctas = 0;   /* batched: CTAs per SM of the tiled launches (0: a warp per tile) */
     std::vector<sph::SceneTile> h_tiles;

@@ -18,8 +18,7 @@ struct Bufs {
     float4 *pos_s, *vel_s, *vhalf_s;       /* this step's sorted copies */
     float4 *normal, *accel, *pos_pred, *f_other, *f_press;
     float *density, *pressure, *dens_var;
-    float* pci_c;                          /* PCISPH loop: p / rho^2 of each particle this iteration */
-    float4* pci_pc;                        /* PCISPH loop: (x, y, z, p / rho^2), the force phase's neighbour record */
+    float4* pci_pc;                        /* PCISPH loop: (x, y, z, p / rho^2), the force phase's record */
     float4* aux;                           /* per particle (p/rho^2, 1/rho, rho, p) */
     float4* nrec;                          /* 2 per particle: (v, p/rho^2), (normal, 1/rho) for the force pass */
     float4* prho;                          /* per particle (x, y, z, rho), written by the list + density pass of
@@ -204,9 +203,13 @@ bool launch_lists_split(cudaStream_t s, const Const& c, const Bufs& b, bool pci,
 /* sph_pcisph.cu */
 void launch_pci_init_density(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms, bool pack = false);
-int pci_loop_blocks(int num_sms, int bs);
-cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter, int blocks,
-                            int num_sms, bool fuse_integrate);
+/* CTAs of the loop's kernels that run at once: of the plain and of the denser variant */
+struct LoopBlocks {
+    int plain, dense;
+};
+LoopBlocks pci_loop_blocks(int num_sms);
+cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter,
+                            const LoopBlocks& fit, int num_sms, bool fuse_integrate);
 void launch_pci_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_pci_predict(cudaStream_t s, const Const& c, const Bufs& b, int bs);
 void launch_pci_update_pressure(cudaStream_t s, const Const& c, const Bufs& b, int bs);

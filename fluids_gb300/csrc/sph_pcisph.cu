@@ -57,18 +57,20 @@ __device__ __forceinline__ void pci_advance(const Const& c, float4 p, float4 v, 
     d = len3(cx - px, cy - py, cz - pz);
 }
 
-__device__ __forceinline__ void pci_predict_one(const Const& c, const Bufs& b, int i) {
+/* with the particle's (sorted) position p and pressure force fp */
+__device__ __forceinline__ void pci_predict_one(const Const& c, const Bufs& b, int i, float4 p, float4 fp) {
     float px, py, pz, vx, vy, vz, cx, cy, cz, d, vn;
-    pci_advance(c, __ldg(&b.pos_s[i]), __ldg(&b.vel_s[i]), b.f_other[i], b.f_press[i], px, py, pz, vx, vy, vz, cx,
-                cy, cz, d, vn);
+    pci_advance(c, p, __ldg(&b.vel_s[i]), __ldg(&b.f_other[i]), fp, px, py, pz, vx, vy, vz, cx, cy, cz, d, vn);
     if (d > 0.f && vn > 0.f) { px = cx; py = cy; pz = cz; }
     b.pos_pred[i] = make_float4(px, py, pz, 1.f);
 }
+__device__ __forceinline__ void pci_predict_one(const Const& c, const Bufs& b, int i) {
+    pci_predict_one(c, b, i, __ldg(&b.pos_s[i]), b.f_press[i]);
+}
 
-__device__ __forceinline__ void pci_integrate_one(const Const& c, const Bufs& b, int i) {
+__device__ __forceinline__ void pci_integrate_one(const Const& c, const Bufs& b, int i, float4 p, float4 fp) {
     float px, py, pz, vx, vy, vz, cx, cy, cz, d, vn;
-    pci_advance(c, __ldg(&b.pos_s[i]), __ldg(&b.vel_s[i]), b.f_other[i], b.f_press[i], px, py, pz, vx, vy, vz, cx,
-                cy, cz, d, vn);
+    pci_advance(c, p, __ldg(&b.vel_s[i]), __ldg(&b.f_other[i]), fp, px, py, pz, vx, vy, vz, cx, cy, cz, d, vn);
     if (d > 0.f && vn > 0.f) {
         float sx = signf(cx - px), sy = signf(cy - py), sz = signf(cz - pz);
         const float sl = len3(sx, sy, sz);
@@ -84,13 +86,16 @@ __device__ __forceinline__ void pci_integrate_one(const Const& c, const Bufs& b,
     const bool bad = !(isfinite(px) && isfinite(py) && isfinite(pz) && isfinite(vx) && isfinite(vy) && isfinite(vz));
     if (bad) atomicOr(b.flags, kFlagNan);
 }
+__device__ __forceinline__ void pci_integrate_one(const Const& c, const Bufs& b, int i) {
+    pci_integrate_one(c, b, i, __ldg(&b.pos_s[i]), b.f_press[i]);
+}
 
 /* update_pressure for one particle: predicted density from the fixed lists at x*.  The
  * list is walked two entries deep with the next two entries loaded during the current two
  * visits (the sum keeps list order).  x* is written by this kernel, so it is read with plain loads.
  * The updated pressure's p / rho^2 (the initial density, as compute_pressure_force uses it)
- * goes to pci_c for the force phase: the same IEEE quotient the force phase would form per
- * pair, formed once per particle. */
+ * goes to pci_pc, beside the position, for the force phase: the same IEEE quotient the force
+ * phase would form per pair, formed once per particle. */
 /* Visits list entries [0, len) of row e (stride n) in list order, loading the data of D
  * entries (load(j)) before their D visits and the next D entries' indices during them: the
  * walks of the loop are bound by the latency of these dependent loads.  Four deep, measured
@@ -120,11 +125,21 @@ __device__ __forceinline__ void walk_list(const int* __restrict__ e, size_t n, i
             if (k + u < len) visit(q[u]);
     }
 }
+/* A boundary particle's position and Psi. */
+struct BndRec {
+    float4 p;
+    float phi;
+};
+__device__ __forceinline__ BndRec load_bnd(const Bufs& b, int j) { return {__ldg(&b.bpos_s[j]), __ldg(&b.bphi_s[j])}; }
+/* the boundary walks: four entries deep with one lane, three with several.  A near-wall
+ * particle's twenty-odd entries, walked one after the other behind its fluid pairs, were the
+ * tail of every phase: 103,823 particles 28.8 -> 23.0 us an iteration, 19,683 31.2 -> 28.7. */
+constexpr int kBndDepth = 4, kBndSplit = 3;
 /* W > 1: W lanes of a particle (small scenes, PHYSICS): each forms the terms of entries w, w +
  * W, ..., and all add them in list order, so the sum is that of one thread.  w >= W: a lane
  * without a particle, which only takes part in the exchange. */
 template <bool COMPAT, int W = 1>
-__device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, int i, int w = 0) {
+__device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, int i, int w = 0, bool full = true) {
     const float4 pi = b.pos_pred[i];
     const float H = c.h_def, HH = H * H;
     const size_t n = (size_t)c.n;
@@ -169,33 +184,42 @@ __device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, i
                 for (int v = 0; v < W; ++v) pd = __fadd_rn(pd, __shfl_sync(0xffffffffu, term[u], v, W));
         }
         const int bmost = __reduce_max_sync(0xffffffffu, w < W ? blen : 0);
-        for (int k0 = 0; k0 < bmost; k0 += W) {
-            const int k = k0 + w;
-            float term = 0.f;
-            if (w < W && k < blen) {
-                const int j = __ldg(&b.sblist[k * n + i]);
-                term = __fmul_rn(cube(__ldg(&b.bpos_s[j])), __ldg(&b.bphi_s[j]));
+        for (int k0 = 0; k0 < bmost; k0 += kBndSplit * W) {
+            float term[kBndSplit];
+            int j[kBndSplit];
+#pragma unroll
+            for (int u = 0; u < kBndSplit; ++u) {
+                const int k = k0 + u * W + w;
+                j[u] = w < W && k < blen ? __ldg(&b.sblist[k * n + i]) : -1;
             }
 #pragma unroll
-            for (int v = 0; v < W; ++v) pdb = __fadd_rn(pdb, __shfl_sync(0xffffffffu, term, v, W));
+            for (int u = 0; u < kBndSplit; ++u) {
+                term[u] = 0.f;
+                if (j[u] >= 0) {
+                    const BndRec r = load_bnd(b, j[u]);
+                    term[u] = __fmul_rn(cube(r.p), r.phi);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kBndSplit; ++u)
+#pragma unroll
+                for (int v = 0; v < W; ++v) pdb = __fadd_rn(pdb, __shfl_sync(0xffffffffu, term[u], v, W));
         }
         if (w != 0) return 0.f;
     } else {
         walk_list<SPH_PCI_WALK_DEPTH>(e, n, len, i, [&](int j) { return b.pos_pred[j]; }, visit);
     }
     pd *= c.default_eval * c.mass_def;
-    for (int k = 0; k < (W > 1 ? 0 : blen); ++k) {
-        const int j = __ldg(&b.sblist[k * n + i]);
-        const float4 pj = __ldg(&b.bpos_s[j]);
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        const float r2 = r2_exact(dx, dy, dz);
+    walk_list<kBndDepth>(b.sblist + i, n, W > 1 ? 0 : blen, 0, [&](int j) { return load_bnd(b, j); },
+                                 [&](const BndRec& q) {
+        const float r2 = r2_exact(pi.x - q.p.x, pi.y - q.p.y, pi.z - q.p.z);
         if (COMPAT && c.monaghan) {
-            pdb += w_monaghan(r2, H, H) * __ldg(&b.bphi_s[j]);
+            pdb += w_monaghan(r2, H, H) * q.phi;
         } else if (COMPAT || r2 < HH) {
             const float t = HH - r2;
-            pdb = __fadd_rn(pdb, __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), __ldg(&b.bphi_s[j])));
+            pdb = __fadd_rn(pdb, __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), q.phi));
         }
-    }
+    });
     pdb *= c.default_eval;
     const float e0 = pd + pdb - c.rho0_def;
     const float dv = (0.f < e0) ? e0 : 0.f;
@@ -204,23 +228,26 @@ __device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, i
     b.pressure[i] = p;
     const float di = __ldg(&b.density[i]);
     const float q = p / (di * di);
-    b.pci_c[i] = q;
+    if (!full) {   /* the record has the position already */
+        b.pci_pc[i].w = q;
+        return dv;
+    }
     const float4 ps = __ldg(&b.pos_s[i]);
     b.pci_pc[i] = make_float4(ps.x, ps.y, ps.z, q);   /* one record per neighbour for the force phase */
     return dv;
 }
 
 /* compute_pressure_force for one particle (initial density, updated pressure):
- * (p_i / rho_i^2 + p_j / rho_j^2) per pair with the quotients of pci_c; each neighbour's
- * position and quotient come as one record from pci_pc (both written by the update phase
- * of this kernel, so plain loads). */
+ * (p_i / rho_i^2 + p_j / rho_j^2) per pair; the particle's and each neighbour's position and
+ * quotient come as one record from pci_pc (written by the update phase of this kernel, so
+ * plain loads).  Gives done(record, force) to the particle's (first) lane. */
 /* W > 1: W lanes of a particle, their sums added (w >= W as in pci_update_one). */
-template <bool MON = false, int W = 1>
-__device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Bufs& b, int i, int w = 0) {
-    const float4 pi = __ldg(&b.pos_s[i]);
+template <bool MON = false, int W = 1, class F>
+__device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Bufs& b, int i, int w, F&& done) {
+    const float4 pi = b.pci_pc[i];
     const float H = c.h_def;
     const size_t n = (size_t)c.n;
-    const float C = b.pci_c[i];
+    const float C = pi.w;
     float fx = 0.f, fy = 0.f, fz = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
     const int len = __ldg(&b.nlen[i]);
     const int* __restrict__ e = b.nlist + i;
@@ -267,34 +294,47 @@ __device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Buf
     const float sf = (-(c.mass_def * c.mass_def)) * c.spiky_grad;
     fx *= sf; fy *= sf; fz *= sf;
     const int blen = __ldg(&b.sblen[i]);
-    for (int k = w; k < (w < W ? blen : 0); k += W) {
-        const int j = __ldg(&b.sblist[k * n + i]);
-        const float4 pj = __ldg(&b.bpos_s[j]);
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+    auto wall = [&](const BndRec& r) {
+        const float dx = pi.x - r.p.x, dy = pi.y - r.p.y, dz = pi.z - r.p.z;
         const float l = sqrtf(dx * dx + dy * dy + dz * dz);
-        const float q = __ldg(&b.bphi_s[j]) * (2.0f * C);
+        const float q = r.phi * (2.0f * C);
         if constexpr (MON) {
             float wx, wy, wz;
             grad_w_monaghan(dx, dy, dz, l, H, H, wx, wy, wz);
             gx += q * wx;
             gy += q * wy;
             gz += q * wz;
-            continue;
+            return;
         }
         const float il = 1.0f / l, t = (H - l) * (H - l);
         gx += q * ((dx * il) * t);
         gy += q * ((dy * il) * t);
         gz += q * ((dz * il) * t);
+    };
+    if constexpr (W > 1) {
+        for (int k0 = w; k0 < (w < W ? blen : 0); k0 += kBndSplit * W) {
+            int j[kBndSplit];
+            BndRec r[kBndSplit];
+#pragma unroll
+            for (int u = 0; u < kBndSplit; ++u) j[u] = k0 + u * W < blen ? __ldg(&b.sblist[(k0 + u * W) * n + i]) : -1;
+#pragma unroll
+            for (int u = 0; u < kBndSplit; ++u) r[u] = load_bnd(b, j[u] < 0 ? 0 : j[u]);
+#pragma unroll
+            for (int u = 0; u < kBndSplit; ++u)
+                if (j[u] >= 0) wall(r[u]);
+        }
+    } else {
+        walk_list<kBndDepth>(b.sblist + i, n, blen, 0, [&](int j) { return load_bnd(b, j); }, wall);
     }
     const float sb = (-c.mass_def) * c.spiky_grad;
     if constexpr (W > 1) {
         fx = sum_lanes<W>(fx + gx * sb);
         fy = sum_lanes<W>(fy + gy * sb);
         fz = sum_lanes<W>(fz + gz * sb);
-        if (w == 0) b.f_press[i] = make_float4(fx, fy, fz, 0.f);
+        if (w == 0) done(pi, make_float4(fx, fy, fz, 0.f));
         return;
     }
-    b.f_press[i] = make_float4(fx + gx * sb, fy + gy * sb, fz + gz * sb, 0.f);
+    done(pi, make_float4(fx + gx * sb, fy + gy * sb, fz + gz * sb, 0.f));
 }
 }  // namespace
 
@@ -414,22 +454,22 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
     b.f_other[i] = make_float4(fx, fy, fz, 0.f);
 }
 
-/* 5 blocks/SM (at most 51 registers, a few bytes of spill): 6.7 ms per 4M-particle step vs
- * 7.2 ms at the unbounded 60 registers (4 blocks/SM), measured on GB300. */
-#ifndef SPH_PCI_LOOP_MIN_BLOCKS
-#define SPH_PCI_LOOP_MIN_BLOCKS 5
-#endif
-/* the loop's own block size, whatever the context's: measured on GB300, 256 threads at 5
- * blocks/SM 0.623 ms per 358k step and 6.35 ms per 4M step, against 0.651 / 6.79 ms with
- * 512 x 2, 0.648 / 6.77 ms with 1024 x 1 and 0.659 / 6.80 ms with 256 x 4 */
-#ifndef SPH_PCI_LOOP_THREADS
-#define SPH_PCI_LOOP_THREADS 256
-#endif
-constexpr int kLoopThreads = SPH_PCI_LOOP_THREADS;
+/* The loop's own block size and blocks per SM, whatever the context's; bound by the L1 data
+ * pipe once enough walks are in flight, by their latency before.  Scenes of more than three
+ * rounds of 5 blocks/SM (583,680 particles) take 6 blocks/SM (40 registers, some spills).
+ * Measured on GB300, us a step, 5 and 6 blocks: 357,911 particles 545 / 560; 512,000 769 / 793;
+ * 592,704 972 / 945; 778,688 1268 / 1220; 4,194,304 5678 / 5503.  An iteration at 4M takes 7 and
+ * 8 blocks/SM 10 to 30 % longer, 128 threads x 12 7 %; 512 threads x 3 gain 1 % there and lose
+ * 7 % at 358k. */
+constexpr int kLoopThreads = 256, kLoopBlocks = 5, kLoopDense = 6;
+constexpr long long kLoopDenseFrom = 3LL * kLoopBlocks * kLoopThreads;   /* particles per SM */
 /* W lanes a particle in small scenes (walk_lanes): with one, a loop of 9,177 particles ran on 36
  * SMs; measured on GB300, its three iterations 79 -> 45 us. */
-template <bool COMPAT, bool FUSE_INTEGRATE, int W = 1>
-__global__ void __launch_bounds__(kLoopThreads, SPH_PCI_LOOP_MIN_BLOCKS) k_pci_loop(Const c, Bufs b, int min_iter, int max_iter) {
+/* An iteration's prediction is the epilogue of the force pass before it (as a pass of its own it
+ * read and wrote 80 bytes a particle): 4M 538 -> 511 us an iteration, and 503 with the records'
+ * positions written in the first iteration only. */
+template <bool COMPAT, bool FUSE_INTEGRATE, int W = 1, int BLOCKS = kLoopBlocks>
+__global__ void __launch_bounds__(kLoopThreads, BLOCKS) k_pci_loop(Const c, Bufs b, int min_iter, int max_iter) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
     const int n = c.n;
@@ -438,28 +478,41 @@ __global__ void __launch_bounds__(kLoopThreads, SPH_PCI_LOOP_MIN_BLOCKS) k_pci_l
     auto lane_of = [&](int t) { return W > 1 ? (t / W < n ? t & (W - 1) : W) : 0; };
     auto particle = [&](int t) { return W > 1 ? min(t / W, n - 1) : t; };
     int it = 1;
-    for (; it <= max_iter; ++it) {
-        /* a particle's lane 0 predicts it: the force it reads is its own write */
+    if (max_iter >= 1)
         for (int t = tid; t < walks; t += stride)
             if (lane_of(t) == 0) pci_predict_one(c, b, particle(t));
+    for (; it <= max_iter; ++it) {
         if (!grid_barrier(b.barrier, b.flags, (unsigned)c.barrier_extra)) return;
         float lmax = 0.f;
         for (int t = tid; t < walks; t += stride)
-            lmax = fmaxf(lmax, pci_update_one<COMPAT, W>(c, b, particle(t), lane_of(t)));
+            lmax = fmaxf(lmax, pci_update_one<COMPAT, W>(c, b, particle(t), lane_of(t), it == 1));
         lmax = block_max(lmax);
         if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned*>(&b.pci_maxerr[it - 1]), __float_as_uint(lmax));
         if (!grid_barrier(b.barrier, b.flags, (unsigned)c.barrier_extra)) return;
         const float mx = *reinterpret_cast<volatile float*>(&b.pci_maxerr[it - 1]);
-        if (COMPAT && c.monaghan) {
-            for (int i = tid; i < n; i += stride) pci_pressure_force_one<true>(c, b, i);
-        } else {
-            for (int t = tid; t < walks; t += stride)
-                pci_pressure_force_one<false, W>(c, b, particle(t), lane_of(t));
-        }
         bool stop = false;
         if (it >= min_iter) {
             const float crit = COMPAT ? (mx - c.rho0) / c.rho0 : mx / c.rho0;
             stop = crit < c.pci_eta;
+        }
+        /* the force goes straight into the next prediction, or the step's integration */
+        const bool last = stop || it == max_iter;
+        auto apply = [&](int i, float4 p, float4 f) {
+            if (!last) {
+                pci_predict_one(c, b, i, p, f);
+            } else {
+                b.f_press[i] = f;
+                if (FUSE_INTEGRATE) pci_integrate_one(c, b, i, p, f);
+            }
+        };
+        if (COMPAT && c.monaghan) {
+            for (int i = tid; i < n; i += stride)
+                pci_pressure_force_one<true>(c, b, i, 0, [&](float4 p, float4 f) { apply(i, p, f); });
+        } else {
+            for (int t = tid; t < walks; t += stride) {
+                const int i = particle(t);
+                pci_pressure_force_one<false, W>(c, b, i, lane_of(t), [&](float4 p, float4 f) { apply(i, p, f); });
+            }
         }
         if (stop) break;
     }
@@ -467,7 +520,7 @@ __global__ void __launch_bounds__(kLoopThreads, SPH_PCI_LOOP_MIN_BLOCKS) k_pci_l
         b.pci_iters[0] = it > max_iter ? max_iter : it;
         if (it > max_iter && !COMPAT) atomicOr(b.flags, kFlagNonconverged);
     }
-    if (FUSE_INTEGRATE) {
+    if (FUSE_INTEGRATE && max_iter < 1) {
         for (int t = tid; t < walks; t += stride)
             if (lane_of(t) == 0) pci_integrate_one(c, b, particle(t));
     }
@@ -499,7 +552,6 @@ __global__ void __launch_bounds__(256) k_pci_quotient(Const c, Bufs b) {
     if (i >= c.n) return;
     const float di = b.density[i];
     const float q = b.pressure[i] / (di * di);
-    b.pci_c[i] = q;
     const float4 ps = __ldg(&b.pos_s[i]);
     b.pci_pc[i] = make_float4(ps.x, ps.y, ps.z, q);
 }
@@ -507,8 +559,9 @@ __global__ void __launch_bounds__(256) k_pci_quotient(Const c, Bufs b) {
 __global__ void __launch_bounds__(256) k_pci_pressure_force(Const c, Bufs b) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    if (c.monaghan) pci_pressure_force_one<true>(c, b, i);
-    else pci_pressure_force_one(c, b, i);
+    auto store = [&](float4, float4 f) { b.f_press[i] = f; };
+    if (c.monaghan) pci_pressure_force_one<true>(c, b, i, 0, store);
+    else pci_pressure_force_one(c, b, i, 0, store);
 }
 
 static inline int nblk(int n, int bs) { return (n + bs - 1) / bs; }
@@ -551,40 +604,44 @@ void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int b
     else k_pci_init_forces<false><<<nblk(c.n, bs), bs, 0, s>>>(c, b);
 }
 
-static void* loop_fn(bool compat, bool fuse, int w) {
-    if (compat) w = 1;
+static void* loop_fn(bool compat, bool fuse, int w, bool dense) {
+    if (compat) return fuse ? (void*)k_pci_loop<true, true> : (void*)k_pci_loop<true, false>;
+    if (dense)
+        return fuse ? (void*)k_pci_loop<false, true, 1, kLoopDense> : (void*)k_pci_loop<false, false, 1, kLoopDense>;
     if (w == 8) return fuse ? (void*)k_pci_loop<false, true, 8> : (void*)k_pci_loop<false, false, 8>;
     if (w == 4) return fuse ? (void*)k_pci_loop<false, true, 4> : (void*)k_pci_loop<false, false, 4>;
     if (w == 2) return fuse ? (void*)k_pci_loop<false, true, 2> : (void*)k_pci_loop<false, false, 2>;
-    if (compat) return fuse ? (void*)k_pci_loop<true, true> : (void*)k_pci_loop<true, false>;
     return fuse ? (void*)k_pci_loop<false, true> : (void*)k_pci_loop<false, false>;
 }
 
-int pci_loop_blocks(int num_sms, int bs) {
-    (void)bs;   /* the loop runs with its own block size */
-    int per_sm = 0;
-    for (int w = 1; w <= 8; w *= 2)
-        for (int k = 0; k < 4; ++k) {
-            int v = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, loop_fn((k & 1) != 0, (k & 2) != 0, w), kLoopThreads, 0);
-            per_sm = per_sm == 0 || v < per_sm ? v : per_sm;
-        }
-    if (per_sm < 1) per_sm = 1;
-    return per_sm * num_sms;
+LoopBlocks pci_loop_blocks(int num_sms) {
+    int most[2] = {kLoopBlocks, kLoopDense};
+    for (int dense = 0; dense < 2; ++dense)
+        for (int w = 1; w <= 8; w *= 2)
+            for (int k = 0; k < 4; ++k) {
+                int v = 0;
+                void* f = loop_fn((k & 1) != 0, (k & 2) != 0, w, dense != 0);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, f, kLoopThreads, 0);
+                if (v < most[dense]) most[dense] = v;
+            }
+    return {num_sms * (most[0] < 1 ? 1 : most[0]), num_sms * (most[1] < 1 ? 1 : most[1])};
 }
 
-cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter, int blocks,
-                            int num_sms, bool fuse) {
+cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter,
+                            const LoopBlocks& fit, int num_sms, bool fuse) {
     if (c.n <= 0) return cudaSuccess;
     const int w = c.compat ? 1 : walk_lanes(c.n, num_sms);
-    int need = nblk(c.n * w, kLoopThreads);
-    if (blocks > need) blocks = need;
-    if (blocks < 1) blocks = 1;
+    const bool dense = !c.compat && c.n > kLoopDenseFrom * num_sms;
+    /* the fewest blocks that need no more rounds over the particles, so that no round is nearly
+     * empty: 216,000 particles (1.1 rounds of 760 blocks) 54 -> 37 us an iteration */
+    const int need = nblk(c.n * w, kLoopThreads), rounds = nblk(need, dense ? fit.dense : fit.plain);
+    const int blocks = nblk(need, rounds);
     Const cc = c;
     Bufs bb = b;
     int mi = min_iter, ma = max_iter;
     void* args[] = {&cc, &bb, &mi, &ma};
-    return cudaLaunchCooperativeKernel(loop_fn(c.compat != 0, fuse, w), dim3(blocks), dim3(kLoopThreads), args, 0, s);
+    return cudaLaunchCooperativeKernel(loop_fn(c.compat != 0, fuse, w, dense), dim3(blocks), dim3(kLoopThreads), args, 0,
+                                       s);
 }
 
 void launch_pci_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
