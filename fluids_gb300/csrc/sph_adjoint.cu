@@ -284,7 +284,7 @@ struct sph_adj {
     float4 *tx = nullptr, *tv = nullptr, *tu = nullptr, *taux = nullptr, *ta = nullptr;
     int32_t *tlist = nullptr, *tlen = nullptr;
     /* binning scratch */
-    float4* pos_s = nullptr;
+    float4 *pos_s = nullptr, *rec = nullptr;   /* rec: store_rec, of the step in flight */
     float *dens = nullptr, *pres = nullptr;
     uint32_t *keys = nullptr, *keys_alt = nullptr;
     int32_t *mask = nullptr, *mask_alt = nullptr, *cell_prev = nullptr, *iota = nullptr, *ids = nullptr;
@@ -333,6 +333,7 @@ void carve(sph_adj* a, ACarver& cv) {
     a->keys = cv.take<uint32_t>(n); a->keys_alt = cv.take<uint32_t>(n);
     a->mask = cv.take<int32_t>(n); a->mask_alt = cv.take<int32_t>(n);
     a->cell_prev = cv.take<int32_t>(n);
+    a->rec = cv.take<float4>(2 * n);
     a->iota = cv.take<int32_t>(n); a->ids = cv.take<int32_t>(n);
     a->tab = cv.take<int2>((size_t)a->c.ncells);
     a->sort_ws = cv.take<char>(sph::sort_workspace_bytes((int)n, a->c.key_bits));
@@ -370,12 +371,15 @@ int adj_step(sph_adj* a, const float4* x, const float4* v, const float4* u, floa
     lb.aux = aux;
     lb.scenes = ctx->b.scenes;
     lb.flags = a->flags;
+    lb.vel_s = const_cast<float4*>(v);
+    lb.nrec = a->rec;
     sph::launch_lists_density_remap(s, c, lb, ms, bs, ctx->num_sms);
     Bufs fb{};
     fb.pos_s = const_cast<float4*>(x);
     fb.vel_s = const_cast<float4*>(v);
     fb.vhalf_s = const_cast<float4*>(u);
     fb.aux = aux;
+    fb.nrec = a->rec;
     fb.nlist = list;
     fb.nlen = len;
     fb.tab = a->tab;
@@ -387,7 +391,7 @@ int adj_step(sph_adj* a, const float4* x, const float4* v, const float4* u, floa
     fb.ids = a->ids;
     fb.scenes = ctx->b.scenes;
     fb.flags = a->flags;
-    sph::launch_wc_forces(s, c, fb, true, true, true, bs, ctx->num_sms);
+    sph::launch_wc_forces(s, c, fb, true, true, true, bs, ctx->num_sms, true);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return afail(a, SPH_E_CUDA, std::string("adjoint forward launch: ") + cudaGetErrorString(e));
     return SPH_OK;

@@ -557,6 +557,28 @@ inline int walk_lanes(int n, int num_sms) {
         if ((long long)n * w <= 1024LL * num_sms) return w;
     return 1;
 }
+/* Visits list entries [0, len) of row e (stride n) in list order, loading the data of D entries
+ * (load(j)) before their D visits and the next D entries' indices during them.  A last, partial
+ * batch loads its missing entries as entry `self` (a valid index) and does not visit them. */
+template <int D, class L, class V>
+__device__ __forceinline__ void walk_list(const int* __restrict__ e, size_t n, int len, int self, L&& load,
+                                          V&& visit) {
+    int jn[D];
+#pragma unroll
+    for (int u = 0; u < D; ++u) jn[u] = u < len ? __ldg(e + u * n) : self;
+#pragma unroll 1
+    for (int k = 0; k < len; k += D) {
+        decltype(load(0)) q[D];
+#pragma unroll
+        for (int u = 0; u < D; ++u) q[u] = load(jn[u]);
+        e += D * n;
+#pragma unroll
+        for (int u = 0; u < D; ++u) jn[u] = k + D + u < len ? __ldg(e + u * n) : self;
+#pragma unroll
+        for (int u = 0; u < D; ++u)
+            if (k + u < len) visit(q[u]);
+    }
+}
 /* The list of particle i shared by W lanes (small scenes, where one thread's walk is all
  * latency): lane w visits entries w, w + W, ...; four entries and their positions are loaded
  * before their visits.  A lane's last batch may visit the particle itself (distance 0) in
@@ -761,6 +783,12 @@ __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf(
 /* aux record of a particle: (p/rho^2, 1/rho, rho, p) */
 __device__ __forceinline__ float4 make_aux(float d, float p) {
     return make_float4(p / (d * d), 1.0f / d, d, p);
+}
+/* A particle's record for the force pass of the adjoint's steps: position, velocity, p / rho^2
+ * and 1 / rho (of its aux) in 32 bytes. */
+__device__ __forceinline__ void store_rec(float4* __restrict__ rec, int i, float4 p, float4 v, float4 aux) {
+    rec[2 * (size_t)i] = make_float4(p.x, p.y, p.z, aux.x);
+    rec[2 * (size_t)i + 1] = make_float4(v.x, v.y, v.z, aux.y);
 }
 
 

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kSplitThreads)
                   float* __restrict__ dens, float* __restrict__ pres, float4* __restrict__ aux,
                   const SceneDev* __restrict__ scenes, const int32_t* __restrict__ scene_of,
                   const int32_t* __restrict__ remap, unsigned* __restrict__ flags, const uint8_t* __restrict__ bnear,
-                  float4* __restrict__ prho) {
+                  float4* __restrict__ prho, const float4* __restrict__ vel, float4* __restrict__ rec) {
     extern __shared__ float2 s_term[];   /* per particle: cap entries, padded to an odd number */
     __shared__ int2 s_rng[kPer][27];
     chain_next();
@@ -93,7 +93,9 @@ __global__ void __launch_bounds__(kSplitThreads)
     dens[row] = d;
     if (prho) prho[row] = make_float4(p.x, p.y, p.z, d);
     pres[row] = pr;
-    aux[row] = PCI ? make_float4(0.f, 1.0f / d, d, 0.f) : make_aux(d, pr);
+    const float4 ax = PCI ? make_float4(0.f, 1.0f / d, d, 0.f) : make_aux(d, pr);
+    aux[row] = ax;
+    if (REMAP) store_rec(rec, row, p, __ldg(&vel[row]), ax);
 }
 
 /* The pass takes scenes of up to two waves of lanes (77,824 particles on 152 SMs): measured on
@@ -110,7 +112,7 @@ static void split_launch(cudaStream_t s, const Const& c, const Bufs& b, const in
     launch_early(REMAP || grid <= kEarlyBlocks, s, k_lists_split<BATCH, REMAP, PCI>, grid, kSplitThreads,
                    sizeof(float2) * kPer * (size_t)(c.cap | 1), c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist,
                    b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes, b.scene_of, remap, b.flags,
-                   b.bnear, b.prho);
+                   b.bnear, b.prho, b.vel_s, b.nrec);
 }
 
 bool launch_lists_split(cudaStream_t s, const Const& c, const Bufs& b, bool pci, const int32_t* remap, int num_sms) {

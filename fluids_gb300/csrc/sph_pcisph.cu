@@ -96,35 +96,12 @@ __device__ __forceinline__ void pci_integrate_one(const Const& c, const Bufs& b,
  * The updated pressure's p / rho^2 (the initial density, as compute_pressure_force uses it)
  * goes to pci_pc, beside the position, for the force phase: the same IEEE quotient the force
  * phase would form per pair, formed once per particle. */
-/* Visits list entries [0, len) of row e (stride n) in list order, loading the data of D
- * entries (load(j)) before their D visits and the next D entries' indices during them: the
- * walks of the loop are bound by the latency of these dependent loads.  Four deep, measured
- * on GB300: the 4M PCISPH step 6.35 ms against 7.20 ms two deep (the 358k step 0.620 against
- * 0.618 ms); three deep 6.58 ms. */
+/* The loop's list walks (walk_list) are bound by the latency of their dependent loads.  Four
+ * deep, measured on GB300: the 4M PCISPH step 6.35 ms against 7.20 ms two deep (the 358k step
+ * 0.620 against 0.618 ms); three deep 6.58 ms. */
 #ifndef SPH_PCI_WALK_DEPTH
 #define SPH_PCI_WALK_DEPTH 4
 #endif
-template <int D, class L, class V>
-__device__ __forceinline__ void walk_list(const int* __restrict__ e, size_t n, int len, int self, L&& load,
-                                          V&& visit) {
-    /* batches of D entries; a last, partial batch loads its missing entries as the particle
-     * itself (a valid index) and does not visit them */
-    int jn[D];
-#pragma unroll
-    for (int u = 0; u < D; ++u) jn[u] = u < len ? __ldg(e + u * n) : self;
-#pragma unroll 1
-    for (int k = 0; k < len; k += D) {
-        decltype(load(0)) q[D];
-#pragma unroll
-        for (int u = 0; u < D; ++u) q[u] = load(jn[u]);
-        e += D * n;
-#pragma unroll
-        for (int u = 0; u < D; ++u) jn[u] = k + D + u < len ? __ldg(e + u * n) : self;
-#pragma unroll
-        for (int u = 0; u < D; ++u)
-            if (k + u < len) visit(q[u]);
-    }
-}
 /* A boundary particle's position and Psi. */
 struct BndRec {
     float4 p;

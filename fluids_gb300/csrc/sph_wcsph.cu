@@ -103,7 +103,9 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
                                                        unsigned* __restrict__ flags = nullptr,
                                                        const uint8_t* __restrict__ bnear = nullptr,
                                                        const int32_t* __restrict__ noff = nullptr,
-                                                       float4* __restrict__ prho = nullptr) {
+                                                       float4* __restrict__ prho = nullptr,
+                                                       const float4* __restrict__ vel = nullptr,
+                                                       float4* __restrict__ rec = nullptr) {
   chain_next();
   for_each_particle<BATCH>(c0, tiles, scenes, [&](const Const& c, long long base, int i, const SceneDev* sd) {
     const int2* __restrict__ ftab = tab0 + base;
@@ -164,7 +166,9 @@ __global__ void __launch_bounds__(256, SPH_LISTS_MIN_BLOCKS) k_lists_density(Con
     const float pv = late_scene<BATCH>(c, sd).kgas * (pown7(di / c.rho0) - 1.0f);
     const float p = (0.f < pv) ? pv : 0.f;
     pres[row] = p;
-    aux[row] = make_aux(di, p);
+    const float4 ax = make_aux(di, p);
+    aux[row] = ax;
+    if (REMAP) store_rec(rec, row, pi, __ldg(&vel[row]), ax);
   });
 }
 
@@ -295,6 +299,7 @@ template <bool COMPAT, bool LIST, bool FUSE, bool WRITE_ACC, bool ST, bool BATCH
 __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const c0, Neigh<LIST, COMPAT> fl0, Neigh<LIST, COMPAT> bl0, Bufs b) {
   chain_next();
   for_each_particle<BATCH, W>(c0, b.tiles, b.scenes, [&](const Const& c, long long base, int i, const SceneDev* sd) {
+    constexpr bool REC = PACK && !ST;   /* nrec holds store_rec's records, position included */
     const int w = W > 1 ? lane_of_particle<W>(c) : 0;
     Neigh<LIST, COMPAT> fl = fl0, bl = bl0;
     fl.tab += base;
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
             bay += dy * k;
             baz += dz * k;
         };
-        if constexpr (W > 1) {
+        if constexpr (W > 1 && !WRITE_ACC) {
             const int len = w < W ? __ldg(&bl.len[i]) : 0;
             for (int k = w; k < len; k += W) {
                 const int j = __ldg(&bl.list[i + (size_t)k * c.n]);
@@ -333,18 +338,8 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
     float pax = 0.f, pay = 0.f, paz = 0.f, vax = 0.f, vay = 0.f, vaz = 0.f;
     float cux = 0.f, cuy = 0.f, cuz = 0.f, cox = 0.f, coy = 0.f, coz = 0.f;
     const float rmin2 = c.rmin2_wc, two_rho0 = 2.0f * c.rho0;
-    auto pair = [&](int j, float4, float dx, float dy, float dz) {
+    auto terms = [&](float4 aj, float4 vj, float4 nj, float dx, float dy, float dz) {
         const float r2 = dx * dx + dy * dy + dz * dz;
-        /* loaded ahead of the guard so that the list loop can issue them early */
-        float4 aj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
-        if constexpr (PACK) {
-            load_pair(&b.nrec[2 * (size_t)j], vj, nj);
-            aj = make_float4(vj.w, nj.w, 1.0f, 0.f);   /* (C_j, R_j, -, -); the guard uses R_j > 0 */
-        } else {
-            aj = __ldg(&b.aux[j]);
-            vj = __ldg(&b.vel_s[j]);
-            if (ST) nj = __ldg(&b.normal[j]);
-        }
         const bool pos_j = PACK ? aj.y > 0.f : aj.z > 0.f;
         if (di > 0.f && pos_j && r2 > rmin2) {
             const float irn = rsqrtf(r2);
@@ -371,7 +366,81 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
             }
         }
     };
-    if constexpr (W > 1)
+    auto pair = [&](int j, float4, float dx, float dy, float dz) {
+        /* loaded ahead of the guard so that the list loop can issue them early */
+        float4 aj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (PACK) {
+            load_pair(&b.nrec[2 * (size_t)j], vj, nj);
+            aj = make_float4(vj.w, nj.w, 1.0f, 0.f);   /* (C_j, R_j, -, -); the guard uses R_j > 0 */
+        } else {
+            aj = __ldg(&b.aux[j]);
+            vj = __ldg(&b.vel_s[j]);
+            if (ST) nj = __ldg(&b.normal[j]);
+        }
+        terms(aj, vj, nj, dx, dy, dz);
+    };
+    struct Rec {
+        float4 p, v;   /* (x, y, z, C), (v, R) */
+    };
+    auto load_rec = [&](int j) {
+        Rec r;
+        load_pair(&b.nrec[2 * (size_t)j], r.p, r.v);
+        return r;
+    };
+    if constexpr (W > 1 && WRITE_ACC) {
+        /* the sums in list order, so that the state has the bits of one lane's walk (a last bit can
+         * turn the clamp of the pressure, and with it the gradient): W entries a round, whose
+         * factors go through shared memory to the lane of each component */
+        static_assert(W == 8 && REC, "six sums, one a lane");
+        __shared__ float4 s_fac[256 / W][28];   /* a group's 8 x 3, padded by a half-warp's banks */
+        float4* const fac = s_fac[threadIdx.x / W];
+        const int len = w < W ? __ldg(&fl.len[i]) : 0, lane = threadIdx.x & (W - 1);
+        const int most = __reduce_max_sync(0xffffffffu, len);
+        const int* const e = fl.list + i;
+        const size_t n = (size_t)c.n;
+        const float2* const mine = reinterpret_cast<const float2*>(fac) + (lane < 6 ? lane : 0);
+        float sum = 0.f;
+        auto index = [&](int k) { return k < len ? __ldg(e + k * n) : -1; };
+        int j = index(lane), jn = index(lane + W);
+        Rec q = load_rec(j < 0 ? i : j);
+        for (int k0 = 0; k0 < most; k0 += W) {
+            const int jnn = index(k0 + 2 * W + lane);
+            const Rec qn = load_rec(jn < 0 ? i : jn);
+            const float dx = __fsub_rn(pi.x, q.p.x), dy = __fsub_rn(pi.y, q.p.y), dz = __fsub_rn(pi.z, q.p.z);
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            const bool ok = j >= 0 && di > 0.f && q.v.w > 0.f && r2 > rmin2;
+            const float irn = rsqrtf(r2);
+            const float rn = r2 * irn;
+            const float t = h - rn;
+            const float f = (sg * irn) * (t * t) * (C + q.p.w);
+            const float vw = t * q.v.w;
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            fac[3 * lane] = ok ? make_float4(dx, f, dy, f) : zero;
+            fac[3 * lane + 1] = ok ? make_float4(dz, f, q.v.x - vi.x, vw) : zero;
+            fac[3 * lane + 2] = ok ? make_float4(q.v.y - vi.y, vw, q.v.z - vi.z, vw) : zero;
+            __syncwarp();
+#pragma unroll
+            for (int v = 0; v < W; ++v) {
+                const float2 a = mine[6 * v];
+                sum = __fmaf_rn(a.x, a.y, sum);
+            }
+            __syncwarp();
+            j = jn; jn = jnn;
+            q = qn;
+        }
+        pax = __shfl_sync(0xffffffffu, sum, 0, W);
+        pay = __shfl_sync(0xffffffffu, sum, 1, W);
+        paz = __shfl_sync(0xffffffffu, sum, 2, W);
+        vax = __shfl_sync(0xffffffffu, sum, 3, W);
+        vay = __shfl_sync(0xffffffffu, sum, 4, W);
+        vaz = __shfl_sync(0xffffffffu, sum, 5, W);
+        if (w != 0) return;
+    } else if constexpr (REC) {
+        walk_list<SPH_FORCES_WALK>(fl.list + i, (size_t)c.n, __ldg(&fl.len[i]), i, load_rec, [&](const Rec& q) {
+            terms(make_float4(q.p.w, q.v.w, 1.0f, 0.f), q.v, make_float4(0.f, 0.f, 0.f, 0.f), __fsub_rn(pi.x, q.p.x),
+                  __fsub_rn(pi.y, q.p.y), __fsub_rn(pi.z, q.p.z));
+        });
+    } else if constexpr (W > 1)
         list_neighbors_split<W>(i, c.n, fl.list, w < W ? __ldg(&fl.len[i]) : 0, w, i, fl.npos, pi.x, pi.y, pi.z, pair);
     else
         /* the list walk SPH_FORCES_WALK (four) entries deep with the next entries loaded during
@@ -386,7 +455,7 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const 
     const float vs = COMPAT ? (c.visc_lapl * cl.mu) : (c.visc_lapl * cl.mu) * (m * ai.y);
     vax *= vs; vay *= vs; vaz *= vs;
     float ax = pax + vax + bax, ay = c.g + pay + vay + bay, az = paz + vaz + baz;
-    if constexpr (W > 1) {
+    if constexpr (W > 1 && !WRITE_ACC) {
         /* each lane's share of every term, then their sum */
         const float cs = COMPAT ? c.st_main : c.st_main * m, ns = ST ? -c.sigma : 0.f;
         ax = sum_lanes<W>(((ns * (cux + cox * cs) + pax) + vax) + bax);
@@ -478,7 +547,7 @@ template <bool COMPAT, bool BATCH>
 static void lists_density_launch(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
     launch_chained(s, k_lists_density<COMPAT, BATCH>, grid_for<BATCH>(c, bs), bs, 0, c, b.pos_s, b.tab, b.bpos_s,
                    b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes,
-                   b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho);
+                   b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho, nullptr, nullptr);
 }
 
 void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
@@ -486,7 +555,7 @@ void launch_lists_density_pci(cudaStream_t s, const Const& c, const Bufs& b, int
     if (launch_lists_split(s, c, b, true, nullptr, num_sms)) return;
     k_lists_density<false, false, false, true><<<nblk(c.n, bs), bs, 0, s>>>(
         c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
-        b.aux, b.scenes, b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho);
+        b.aux, b.scenes, b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho, nullptr, nullptr);
 }
 void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, const int32_t* remap, int bs,
                                 int num_sms) {
@@ -494,7 +563,7 @@ void launch_lists_density_remap(cudaStream_t s, const Const& c, const Bufs& b, c
     if (launch_lists_split(s, c, b, false, remap, num_sms)) return;
     k_lists_density<false, false, true><<<nblk(c.n, bs), bs, 0, s>>>(
         c, b.pos_s, b.tab, b.bpos_s, b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure,
-        b.aux, b.scenes, b.tiles, remap, b.flags);
+        b.aux, b.scenes, b.tiles, remap, b.flags, nullptr, nullptr, nullptr, b.vel_s, b.nrec);
 }
 
 void launch_lists_density(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms) {
@@ -605,6 +674,24 @@ static void forces_launch(cudaStream_t s, const Const& c, const Bufs& b, bool fu
             case 4: forces_split<BATCH, 4>(s, c, b, bs, st); return;
             case 2: forces_split<BATCH, 2>(s, c, b, bs, st); return;
             }
+        }
+    }
+    if constexpr (LIST && !COMPAT && !BATCH) {
+        /* the adjoint's steps (nrec by store_rec): eight lanes a particle, their sums in list
+         * order, up to 160 particles an SM.  An optimisation step of 8 + 8 time steps on GB300,
+         * us, with the three gathers a pair before, with the records, and with the lanes: 343
+         * particles 872, 831, 776; 8,000 1216, 1154, 1120; 19,683 1513, 1381, 1303; 32,768 1618,
+         * 1508, 1531; 262,144 4147, 3954, 4676. */
+        if (fuse && write_acc && !st && pack) {
+            Const cw = c;
+            cw.first = 0;
+            cw.last = c.n;
+            if (c.n <= 160 * num_sms)
+                launch_early(true, s, k_wc_forces<false, true, true, true, false, false, true, 8>, nblk(8 * c.n, 256),
+                             256, 0, cw, fs, bsrc, b);
+            else
+                launch_early(true, s, k_wc_forces<false, true, true, true, false, false, true>, g, bs, 0, c, fs, bsrc, b);
+            return;
         }
     }
     if constexpr (LIST) {
