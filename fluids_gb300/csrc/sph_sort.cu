@@ -261,12 +261,17 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restric
     }
 }
 
-/* The whole sort of up to kOneTiles tiles of 2,048 pairs (4,096 in a single CTA) in one
- * cooperative launch, a tile per CTA: for a small sort the launches of the memset, the
+/* Barrier of the cluster's CTAs; what its threads wrote before is seen by all of them after. */
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+/* The whole sort of up to kOneTiles tiles of 2,048 pairs (4,096 in a single CTA) in one launch,
+ * cooperative or (CLUSTER) one cluster, a tile per CTA: for a small sort the launches of the memset, the
  * histogram and the passes are its time.  Measured on GB300 against those launches (24-bit
  * keys, us): 2,387 pairs 20 / 41, 40,000 32 / 45, 150,000 38 / 49, 300,000 44 / 52, 500,000
  * 56 / 59, 600,000 (32-bit keys) 76 / 75.  Per
- * pass each CTA ranks its tile, publishes its digit counts, and after a grid barrier adds the
+ * pass each CTA ranks its tile, publishes its digit counts, and after a barrier of all CTAs adds the
  * counts of the tiles before it (and of all tiles, for the buckets), which it reads row by
  * row, so there is no separate histogram and no look-back; a second barrier ends the pass. */
 constexpr int kOneThreads = 512;
@@ -274,7 +279,7 @@ constexpr int kOneWarps = kOneThreads / 32;
 constexpr int kOneTile = kOneThreads * 4;
 constexpr int kOneTiles = 256;
 constexpr int kOneSolo = kOneThreads * 8;   /* the largest sort of a single CTA */
-template <int ITEMS>
+template <int ITEMS, bool CLUSTER = false>
 __global__ void __launch_bounds__(kOneThreads) k_sort_one(SortBufs b, int n, int passes, uint32_t* __restrict__ counts,
                                                           unsigned* bar, unsigned* __restrict__ flags,
                                                           const unsigned* __restrict__ gate) {
@@ -284,6 +289,7 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_one(SortBufs b, int n, int
     __shared__ uint32_t s_part[2][2][256];
     __shared__ uint32_t s_tprefix[256], s_dbase[256];
     __shared__ uint32_t s_scan[kWarps];
+    chain_next();
     if (gate && *gate == 0u) return;   /* the whole grid leaves together */
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tile = blockIdx.x, tiles = gridDim.x, base = tile * (kOneThreads * ITEMS), wbase = base + warp * (32 * ITEMS);
@@ -325,7 +331,9 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_one(SortBufs b, int n, int
             }
             __stcg(&counts[(size_t)tile * 256 + d], cnt);
         }
-        if (tiles > 1) {
+        if (CLUSTER) {
+            cluster_barrier();
+        } else if (tiles > 1) {
             if (!grid_barrier(bar, flags, 0u)) return;
         } else {
             __syncthreads();
@@ -369,13 +377,45 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_one(SortBufs b, int n, int
             __stcg(&vout[dest], s_vals[s]);
         }
         if (p + 1 < passes) {
-            if (tiles > 1) {
+            if (CLUSTER) {
+                cluster_barrier();
+            } else if (tiles > 1) {
                 if (!grid_barrier(bar, flags, 0u)) return;
             } else {
                 __syncthreads();
             }
         }
     }
+}
+
+/* Up to kClusterMost tiles of 2,048 pairs, else of 4,096, run as one cluster: its barrier takes a
+ * fraction of a grid's (five of them for 24 bits), and the launch need not be cooperative, so it
+ * can be set up early.  Measured on GB300: an optimisation step of the adjoint with 32 sorts of
+ * 32,768 pairs (21 bits) 2713 us with grid barriers, 2421 as 16 tiles, 2584 as 8 of 4,096; 65,536 pairs of 24 bits through the entry point 33.0 -> 29.2 us.  A gated sort
+ * takes tiles of 2,048 only: set up beside the step's kernels, the larger ones cost a step of
+ * 64,000 particles 5 us, where four steps of 32,768 went from 292 to 285. */
+constexpr int kClusterMost = 16;
+static bool launch_cluster(cudaStream_t s, void* kernel, int ctas, void** args) {
+    /* more than 8 CTAs are beyond what every GPU takes; refused here, the caller's other path runs */
+    if (ctas > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kOneThreads);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    if (cudaLaunchKernelExC(&cfg, kernel, args) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
 }
 
 int sort_passes(int key_bits) { return key_bits <= 0 ? 0 : (key_bits + 7) / 8; }
@@ -423,6 +463,14 @@ void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned*
         uint32_t* counts = status;
         int nn = n, np = passes;
         void* args[] = {&bb, &nn, &np, &counts, &bar, &flags, &gate};
+        if (n <= kOneSolo) {
+            if (launch_cluster(s, (void*)k_sort_one<8>, 1, args)) return;
+        } else if (n <= (gate ? 4 : 8) * kOneThreads * kClusterMost) {
+            const bool four = n <= 4 * kOneThreads * kClusterMost;
+            if (launch_cluster(s, four ? (void*)k_sort_one<4, true> : (void*)k_sort_one<8, true>,
+                               (n + (four ? 4 : 8) * kOneThreads - 1) / ((four ? 4 : 8) * kOneThreads), args))
+                return;
+        }
         void* fn = n <= kOneSolo ? (void*)k_sort_one<8> : (void*)k_sort_one<4>;
         if (cudaLaunchCooperativeKernel(fn, dim3(one), dim3(kOneThreads), args, 0, s) == cudaSuccess) return;
         cudaGetLastError();   /* then by several launches */
