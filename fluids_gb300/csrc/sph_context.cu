@@ -588,7 +588,7 @@ int enqueue_step(sph_ctx* x, int pci_max_iter, cudaEvent_t vel_ready, const Host
          * (velocity, normal, 1/rho) that the force pass reads */
         const bool pack = c.sigma != 0.f;
         if (pack) {
-            sph::launch_normals(s, c, b, true, bs, x->num_sms, true, !c.compat && !c.batched);   /* after k_lists_density_pci */
+            sph::launch_normals(s, c, b, true, bs, x->num_sms, true, !c.compat && !c.batched, true);   /* after k_lists_density_pci */
             mark(x, "k_normals");
         }
         sph::launch_pci_init_forces(s, c, b, bs, x->num_sms, pack);

@@ -579,6 +579,13 @@ __device__ __forceinline__ void walk_list(const int* __restrict__ e, size_t n, i
             if (k + u < len) visit(q[u]);
     }
 }
+/* Lanes per particle of ordered_walk: 8 up to 64 particles an SM (9,728), 4 up to 256 (38,912),
+ * else 1.  Measured on GB300 (three PCISPH steps, us; 1, 2, 4 and 8 lanes): 2,197 particles 550,
+ * 495, 409, 388; 8,000 664, 571, 475, 464; 13,824 662, 572, 492, 517; 35,937 739, 677, 665, 786;
+ * 46,656 765, 762, 776, 929. */
+inline int ordered_lanes(int n, int num_sms) {
+    return n <= 64LL * num_sms ? 8 : (n <= 256LL * num_sms ? 4 : 1);
+}
 /* The list of particle i shared by W lanes (small scenes, where one thread's walk is all
  * latency): lane w visits entries w, w + W, ...; four entries and their positions are loaded
  * before their visits.  A lane's last batch may visit the particle itself (distance 0) in
@@ -600,6 +607,53 @@ __device__ __forceinline__ void list_neighbors_split(int i, int n, const int* __
         for (int u = 0; u < U; ++u)
             f(j[u], q[u], __fsub_rn(px, q[u].x), __fsub_rn(py, q[u].y), __fsub_rn(pz, q[u].z));
     }
+}
+/* The C sums over particle i's list of products a b, in list order, by W lanes: each lane forms
+ * the factors of its entry of a round (terms(record, whether there is one, f), zeros where not;
+ * record by load(j), loaded a round ahead), which go through shared memory (s_fac: C a thread) to
+ * the lane of each sum.  The sums have the bits of one thread's walk: a last bit of PCISPH's
+ * forces can turn its stop test, and with it the number of iterations. */
+template <int W, int C, class L, class T>
+__device__ __forceinline__ void ordered_walk(int i, int n, const int* __restrict__ list, int len, int self,
+                                             float2* s_fac, float (&total)[C], L&& load, T&& terms) {
+    constexpr int M = (C + W - 1) / W;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & (W - 1);
+    float2* const fac = s_fac + (threadIdx.x / W) * (W * C);
+    const int* const e = list + i;
+    const int most = __reduce_max_sync(kAll, len);
+    float sum[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) sum[m] = 0.f;
+    if (most > 0) {
+        auto index = [&](int k) { return k < len ? __ldg(e + (size_t)k * n) : -1; };
+        int j = index(lane), jn = index(lane + W);
+        auto q = load(j < 0 ? self : j);
+#pragma unroll 1
+        for (int k0 = 0; k0 < most; k0 += W) {
+            const int jnn = index(k0 + 2 * W + lane);
+            const auto qn = load(jn < 0 ? self : jn);
+            float2 f[C];
+            terms(q, j >= 0, f);
+#pragma unroll
+            for (int c = 0; c < C; ++c) fac[lane * C + c] = f[c];
+            __syncwarp();
+#pragma unroll
+            for (int v = 0; v < W; ++v)
+#pragma unroll
+                for (int m = 0; m < M; ++m)
+                    if (lane + W * m < C) {
+                        const float2 a = fac[v * C + lane + W * m];
+                        sum[m] = __fmaf_rn(a.x, a.y, sum[m]);
+                    }
+            __syncwarp();
+            j = jn;
+            jn = jnn;
+            q = qn;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) total[c] = __shfl_sync(kAll, sum[c / W], c % W, W);
 }
 /* The sum of v over the W lanes of a particle, in all of them. */
 template <int W>

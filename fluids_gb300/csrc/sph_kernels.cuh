@@ -182,9 +182,9 @@ void launch_wc_density(cudaStream_t s, const Const& c, const Bufs& b, bool lists
 /* pack: also write nrec (the force pass then reads 2 adjacent float4 per neighbour instead of
  * velocity, aux and normal); only the fused step uses it */
 /* prho: the step's list + density pass wrote b.prho, which the walk then reads for both the
- * neighbour's position and its density */
+ * neighbour's position and its density.  ordered: several lanes' sums in list order */
 void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack = false,
-                    bool prho = false);
+                    bool prho = false, bool ordered = false);
 void launch_wc_forces(cudaStream_t s, const Const& c, const Bufs& b, bool lists, bool fuse_integrate,
                       bool write_acc, int bs, int num_sms, bool pack = false);
 void launch_wc_integrate(cudaStream_t s, const Const& c, const Bufs& b, int bs);

@@ -108,9 +108,9 @@ struct BndRec {
     float phi;
 };
 __device__ __forceinline__ BndRec load_bnd(const Bufs& b, int j) { return {__ldg(&b.bpos_s[j]), __ldg(&b.bphi_s[j])}; }
-/* the boundary walks: four entries deep with one lane, three with several.  A near-wall
+/* the boundary walks: four entries deep with one lane, the update's three with several.  A near-wall
  * particle's twenty-odd entries, walked one after the other behind its fluid pairs, were the
- * tail of every phase: 103,823 particles 28.8 -> 23.0 us an iteration, 19,683 31.2 -> 28.7. */
+ * tail of every phase: 103,823 particles 28.8 -> 23.0 us an iteration. */
 constexpr int kBndDepth = 4, kBndSplit = 3;
 /* W > 1: W lanes of a particle (small scenes, PHYSICS): each forms the terms of entries w, w +
  * W, ..., and all add them in list order, so the sum is that of one thread.  w >= W: a lane
@@ -218,9 +218,10 @@ __device__ __forceinline__ float pci_update_one(const Const& c, const Bufs& b, i
  * (p_i / rho_i^2 + p_j / rho_j^2) per pair; the particle's and each neighbour's position and
  * quotient come as one record from pci_pc (written by the update phase of this kernel, so
  * plain loads).  Gives done(record, force) to the particle's (first) lane. */
-/* W > 1: W lanes of a particle, their sums added (w >= W as in pci_update_one). */
+/* W > 1: W lanes of a particle, their sums in list order (w >= W as in pci_update_one; s_fac as
+ * in ordered_walk, three a thread). */
 template <bool MON = false, int W = 1, class F>
-__device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Bufs& b, int i, int w, F&& done) {
+__device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Bufs& b, int i, int w, float2* s_fac, F&& done) {
     const float4 pi = b.pci_pc[i];
     const float H = c.h_def;
     const size_t n = (size_t)c.n;
@@ -254,16 +255,23 @@ __device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Buf
         fz += q * ((dz * il) * t);
     };
     if constexpr (W > 1) {
-        for (int k0 = w; k0 < (w < W ? len : 0); k0 += 4 * W) {
-            int j[4];
-            float4 q[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) j[u] = k0 + u * W < len ? __ldg(e + (k0 + u * W) * n) : i;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) q[u] = b.pci_pc[j[u]];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) visit(q[u], q[u].w);   /* the particle itself adds zeros */
-        }
+        float total[3];
+        ordered_walk<W>(i, c.n, b.nlist, w < W ? len : 0, i, s_fac, total, [&](int j) { return b.pci_pc[j]; },
+                        [&](float4 pj, bool in, float2 (&f)[3]) {
+            const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            const float il0 = rsqrtf(r2), l0 = r2 * il0;
+            const bool ok = l0 >= 1e-5f;
+            const float il = ok ? il0 : 0.f, l = ok ? l0 : H;
+            const float q = in ? C + pj.w : 0.f;
+            const float t = (H - l) * (H - l);
+            f[0] = make_float2(q, (dx * il) * t);
+            f[1] = make_float2(q, (dy * il) * t);
+            f[2] = make_float2(q, (dz * il) * t);
+        });
+        fx = total[0];
+        fy = total[1];
+        fz = total[2];
     } else {
         walk_list<SPH_PCI_WALK_DEPTH>(e, n, len, i, [&](int j) { return b.pci_pc[j]; },
                                       [&](const float4& v) { visit(v, v.w); });
@@ -289,29 +297,25 @@ __device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Buf
         gz += q * ((dz * il) * t);
     };
     if constexpr (W > 1) {
-        for (int k0 = w; k0 < (w < W ? blen : 0); k0 += kBndSplit * W) {
-            int j[kBndSplit];
-            BndRec r[kBndSplit];
-#pragma unroll
-            for (int u = 0; u < kBndSplit; ++u) j[u] = k0 + u * W < blen ? __ldg(&b.sblist[(k0 + u * W) * n + i]) : -1;
-#pragma unroll
-            for (int u = 0; u < kBndSplit; ++u) r[u] = load_bnd(b, j[u] < 0 ? 0 : j[u]);
-#pragma unroll
-            for (int u = 0; u < kBndSplit; ++u)
-                if (j[u] >= 0) wall(r[u]);
-        }
+        float total[3];
+        ordered_walk<W>(i, c.n, b.sblist, w < W ? blen : 0, 0, s_fac, total, [&](int j) { return load_bnd(b, j); },
+                        [&](const BndRec& r, bool in, float2 (&f)[3]) {
+            const float dx = pi.x - r.p.x, dy = pi.y - r.p.y, dz = pi.z - r.p.z;
+            const float l = sqrtf(dx * dx + dy * dy + dz * dz);
+            const float q = r.phi * (2.0f * C);
+            const float il = 1.0f / l, t = (H - l) * (H - l);
+            f[0] = in ? make_float2(q, (dx * il) * t) : make_float2(0.f, 0.f);
+            f[1] = in ? make_float2(q, (dy * il) * t) : make_float2(0.f, 0.f);
+            f[2] = in ? make_float2(q, (dz * il) * t) : make_float2(0.f, 0.f);
+        });
+        gx = total[0];
+        gy = total[1];
+        gz = total[2];
     } else {
         walk_list<kBndDepth>(b.sblist + i, n, blen, 0, [&](int j) { return load_bnd(b, j); }, wall);
     }
     const float sb = (-c.mass_def) * c.spiky_grad;
-    if constexpr (W > 1) {
-        fx = sum_lanes<W>(fx + gx * sb);
-        fy = sum_lanes<W>(fy + gy * sb);
-        fz = sum_lanes<W>(fz + gz * sb);
-        if (w == 0) done(pi, make_float4(fx, fy, fz, 0.f));
-        return;
-    }
-    done(pi, make_float4(fx + gx * sb, fy + gy * sb, fz + gz * sb, 0.f));
+    if (w == 0) done(pi, make_float4(fx + gx * sb, fy + gy * sb, fz + gz * sb, 0.f));
 }
 }  // namespace
 
@@ -363,7 +367,7 @@ __global__ void __launch_bounds__(256) k_pci_init_density(Const c, Bufs b) {
 #ifndef SPH_PCI_INIT_PIPE
 #define SPH_PCI_INIT_PIPE 1
 #endif
-/* W > 1 (small scenes, PACK): W lanes a particle (list_neighbors_split), their sums added. */
+/* W > 1 (small scenes, PACK): W lanes a particle, their sums in list order (ordered_walk). */
 template <bool PACK, bool MON = false, int W = 1>
 __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
     chain_next();
@@ -410,8 +414,39 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
                        oz += ((dz * inv) * sk) * K;
                    };
     if constexpr (W > 1) {
-        /* a lane's last batch may visit the particle itself, whose every term is zero */
-        list_neighbors_split<W>(i, c.n, b.nlist, w < W ? __ldg(&b.nlen[i]) : 0, w, i, b.pos_s, pi.x, pi.y, pi.z, pair);
+        struct Rec {
+            float4 p, v, n;
+        };
+        __shared__ float2 s_fac[256 * 9];
+        float total[9];
+        ordered_walk<W>(i, c.n, b.nlist, w < W ? __ldg(&b.nlen[i]) : 0, i, s_fac, total, [&](int j) {
+            Rec r;
+            r.p = __ldg(&b.pos_s[j]);
+            load_pair(&b.nrec[2 * (size_t)j], r.v, r.n);
+            return r;
+        }, [&](const Rec& q, bool in, float2 (&f)[9]) {
+            const float dx = __fsub_rn(pi.x, q.p.x), dy = __fsub_rn(pi.y, q.p.y), dz = __fsub_rn(pi.z, q.p.z);
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            const float Rj = q.n.w;
+            const float inv = r2 > 0.f ? rsqrtf(r2) : 0.f;
+            const float rn = r2 * inv;
+            const float w = in ? (H - rn) * Rj : 0.f;
+            const float K = in ? __fdividef(two_rho0 * Rj, di * Rj + 1.0f) : 0.f;
+            const float sk = st_kernel_sel(rn, H, c.st_term);
+            f[0] = make_float2(q.v.x - vi.x, w);
+            f[1] = make_float2(q.v.y - vi.y, w);
+            f[2] = make_float2(q.v.z - vi.z, w);
+            f[3] = make_float2(ni.x - q.n.x, K);
+            f[4] = make_float2(ni.y - q.n.y, K);
+            f[5] = make_float2(ni.z - q.n.z, K);
+            f[6] = make_float2((dx * inv) * sk, K);
+            f[7] = make_float2((dy * inv) * sk, K);
+            f[8] = make_float2((dz * inv) * sk, K);
+        });
+        if (w != 0) return;
+        vx = total[0], vy = total[1], vz = total[2];
+        ux = total[3], uy = total[4], uz = total[5];
+        ox = total[6], oy = total[7], oz = total[8];
     } else {
         list_neighbors<SPH_PCI_INIT_U, SPH_PCI_INIT_PIPE, SPH_PCI_INIT_PIPE>(i, c.n, b.nlist, __ldg(&b.nlen[i]),
                                                                            b.pos_s, pi.x, pi.y, pi.z, pair);
@@ -422,12 +457,6 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
     const float tsc = (-c.sigma) * md;
     float fx = vx * vsc + tsc * (ux + ox * csc), fy = vy * vsc + tsc * (uy + oy * csc),
           fz = vz * vsc + tsc * (uz + oz * csc);
-    if constexpr (W > 1) {
-        fx = sum_lanes<W>(fx);
-        fy = sum_lanes<W>(fy);
-        fz = sum_lanes<W>(fz);
-        if (w != 0) return;
-    }
     b.f_other[i] = make_float4(fx, fy, fz, 0.f);
 }
 
@@ -440,8 +469,8 @@ __global__ void __launch_bounds__(256) k_pci_init_forces(Const c, Bufs b) {
  * 7 % at 358k. */
 constexpr int kLoopThreads = 256, kLoopBlocks = 5, kLoopDense = 6;
 constexpr long long kLoopDenseFrom = 3LL * kLoopBlocks * kLoopThreads;   /* particles per SM */
-/* W lanes a particle in small scenes (walk_lanes): with one, a loop of 9,177 particles ran on 36
- * SMs; measured on GB300, its three iterations 79 -> 45 us. */
+/* W lanes a particle in small scenes (ordered_lanes): with one, a loop of 9,177 particles ran on
+ * 36 SMs; measured on GB300, its three iterations 79 -> 47 us. */
 /* An iteration's prediction is the epilogue of the force pass before it (as a pass of its own it
  * read and wrote 80 bytes a particle): 4M 538 -> 511 us an iteration, and 503 with the records'
  * positions written in the first iteration only. */
@@ -454,6 +483,7 @@ __global__ void __launch_bounds__(kLoopThreads, BLOCKS) k_pci_loop(Const c, Bufs
     const int walks = W > 1 ? (n * W + 31) & ~31 : n;
     auto lane_of = [&](int t) { return W > 1 ? (t / W < n ? t & (W - 1) : W) : 0; };
     auto particle = [&](int t) { return W > 1 ? min(t / W, n - 1) : t; };
+    __shared__ float2 s_fac[W > 1 ? 3 * kLoopThreads : 1];
     int it = 1;
     if (max_iter >= 1)
         for (int t = tid; t < walks; t += stride)
@@ -484,11 +514,11 @@ __global__ void __launch_bounds__(kLoopThreads, BLOCKS) k_pci_loop(Const c, Bufs
         };
         if (COMPAT && c.monaghan) {
             for (int i = tid; i < n; i += stride)
-                pci_pressure_force_one<true>(c, b, i, 0, [&](float4 p, float4 f) { apply(i, p, f); });
+                pci_pressure_force_one<true>(c, b, i, 0, nullptr, [&](float4 p, float4 f) { apply(i, p, f); });
         } else {
             for (int t = tid; t < walks; t += stride) {
                 const int i = particle(t);
-                pci_pressure_force_one<false, W>(c, b, i, lane_of(t), [&](float4 p, float4 f) { apply(i, p, f); });
+                pci_pressure_force_one<false, W>(c, b, i, lane_of(t), s_fac, [&](float4 p, float4 f) { apply(i, p, f); });
             }
         }
         if (stop) break;
@@ -537,8 +567,8 @@ __global__ void __launch_bounds__(256) k_pci_pressure_force(Const c, Bufs b) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     auto store = [&](float4, float4 f) { b.f_press[i] = f; };
-    if (c.monaghan) pci_pressure_force_one<true>(c, b, i, 0, store);
-    else pci_pressure_force_one(c, b, i, 0, store);
+    if (c.monaghan) pci_pressure_force_one<true>(c, b, i, 0, nullptr, store);
+    else pci_pressure_force_one(c, b, i, 0, nullptr, store);
 }
 
 static inline int nblk(int n, int bs) { return (n + bs - 1) / bs; }
@@ -566,10 +596,9 @@ void launch_pci_init_density(cudaStream_t s, const Const& c, const Bufs& b, int 
 void launch_pci_init_forces(cudaStream_t s, const Const& c, const Bufs& b, int bs, int num_sms, bool pack) {
     if (c.n <= 0) return;
     if (pack && !c.compat) {
-        switch (walk_lanes(c.n, num_sms)) {
+        switch (ordered_lanes(c.n, num_sms)) {
         case 8: launch_chained(s, k_pci_init_forces<true, false, 8>, nblk(8 * c.n, 256), 256, 0, c, b); return;
         case 4: launch_chained(s, k_pci_init_forces<true, false, 4>, nblk(4 * c.n, 256), 256, 0, c, b); return;
-        case 2: launch_chained(s, k_pci_init_forces<true, false, 2>, nblk(2 * c.n, 256), 256, 0, c, b); return;
         }
     }
     if (c.monaghan) {
@@ -587,14 +616,13 @@ static void* loop_fn(bool compat, bool fuse, int w, bool dense) {
         return fuse ? (void*)k_pci_loop<false, true, 1, kLoopDense> : (void*)k_pci_loop<false, false, 1, kLoopDense>;
     if (w == 8) return fuse ? (void*)k_pci_loop<false, true, 8> : (void*)k_pci_loop<false, false, 8>;
     if (w == 4) return fuse ? (void*)k_pci_loop<false, true, 4> : (void*)k_pci_loop<false, false, 4>;
-    if (w == 2) return fuse ? (void*)k_pci_loop<false, true, 2> : (void*)k_pci_loop<false, false, 2>;
     return fuse ? (void*)k_pci_loop<false, true> : (void*)k_pci_loop<false, false>;
 }
 
 LoopBlocks pci_loop_blocks(int num_sms) {
     int most[2] = {kLoopBlocks, kLoopDense};
     for (int dense = 0; dense < 2; ++dense)
-        for (int w = 1; w <= 8; w *= 2)
+        for (int w : {1, 4, 8})
             for (int k = 0; k < 4; ++k) {
                 int v = 0;
                 void* f = loop_fn((k & 1) != 0, (k & 2) != 0, w, dense != 0);
@@ -607,7 +635,7 @@ LoopBlocks pci_loop_blocks(int num_sms) {
 cudaError_t launch_pci_loop(cudaStream_t s, const Const& c, const Bufs& b, int min_iter, int max_iter,
                             const LoopBlocks& fit, int num_sms, bool fuse) {
     if (c.n <= 0) return cudaSuccess;
-    const int w = c.compat ? 1 : walk_lanes(c.n, num_sms);
+    const int w = c.compat ? 1 : ordered_lanes(c.n, num_sms);
     const bool dense = !c.compat && c.n > kLoopDenseFrom * num_sms;
     /* the fewest blocks that need no more rounds over the particles, so that no round is nearly
      * empty: 216,000 particles (1.1 rounds of 760 blocks) 54 -> 37 us an iteration */

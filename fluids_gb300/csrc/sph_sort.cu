@@ -1,5 +1,6 @@
 /*
- * sph_sort.cu -- stable LSD onesweep radix sort of (uint32 key, int32 value) pairs.
+ * sph_sort.cu -- stable LSD radix sort of (uint32 key, int32 value) pairs: onesweep, and up to
+ * 524,288 pairs k_sort_one, all passes in one launch.
  *
  * Replaces clsort<cl_uint, cl_int> (opencl/algorithms/clsort.h:13-35), which calls the
  * external clogs 1.5.1 Radixsort (a stable LSD radix sort).  The permutation of a stable
@@ -267,11 +268,10 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 /* The whole sort of up to kOneTiles tiles of 2,048 pairs (4,096 in a single CTA) in one launch,
- * cooperative or (CLUSTER) one cluster, a tile per CTA: for a small sort the launches of the memset, the
- * histogram and the passes are its time.  Measured on GB300 against those launches (24-bit
- * keys, us): 2,387 pairs 20 / 41, 40,000 32 / 45, 150,000 38 / 49, 300,000 44 / 52, 500,000
- * 56 / 59, 600,000 (32-bit keys) 76 / 75.  Per
- * pass each CTA ranks its tile, publishes its digit counts, and after a barrier of all CTAs adds the
+ * cooperative or (CLUSTER) one cluster, a tile per CTA: for a small sort the launches of the
+ * memset, the histogram and the passes are its time.  Measured on GB300, cooperative, against
+ * those launches (24-bit keys, us): 2,387 pairs 20 / 41, 40,000 32 / 45, 150,000 38 / 49, 300,000
+ * 44 / 52, 500,000 56 / 59, 600,000 (32-bit keys) 76 / 75.  Per pass each CTA ranks its tile, publishes its digit counts, and after a barrier of all CTAs adds the
  * counts of the tiles before it (and of all tiles, for the buckets), which it reads row by
  * row, so there is no separate histogram and no look-back; a second barrier ends the pass. */
 constexpr int kOneThreads = 512;
@@ -391,9 +391,10 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_one(SortBufs b, int n, int
 /* Up to kClusterMost tiles of 2,048 pairs, else of 4,096, run as one cluster: its barrier takes a
  * fraction of a grid's (five of them for 24 bits), and the launch need not be cooperative, so it
  * can be set up early.  Measured on GB300: an optimisation step of the adjoint with 32 sorts of
- * 32,768 pairs (21 bits) 2713 us with grid barriers, 2421 as 16 tiles, 2584 as 8 of 4,096; 65,536 pairs of 24 bits through the entry point 33.0 -> 29.2 us.  A gated sort
- * takes tiles of 2,048 only: set up beside the step's kernels, the larger ones cost a step of
- * 64,000 particles 5 us, where four steps of 32,768 went from 292 to 285. */
+ * 32,768 pairs (21 bits) 2713 us with grid barriers, 2421 as 16 tiles, 2584 as 8 of 4,096;
+ * 65,536 pairs of 24 bits through the entry point 33.0 -> 29.2 us.  A gated sort takes tiles of
+ * 2,048 only: set up beside the step's kernels, the larger ones cost a step of 64,000 particles
+ * 5 us, where four steps of 32,768 went from 292 to 285. */
 constexpr int kClusterMost = 16;
 static bool launch_cluster(cudaStream_t s, void* kernel, int ctas, void** args) {
     /* more than 8 CTAs are beyond what every GPU takes; refused here, the caller's other path runs */

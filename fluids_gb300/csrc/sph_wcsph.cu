@@ -12,7 +12,7 @@
  *                 the mass factors of kernels/pcisph.cl:216-219 (P3).  With FUSE the
  *                 leapfrog integration of predict_vel_n_pos (kernels/wcsph.cl:176-224) runs
  *                 as the epilogue, so the acceleration never round-trips through HBM.
- * One thread per particle in Morton order: the 32 particles of a warp share most of their
+ * One thread per particle in Morton order (a few lanes in small contexts): the 32 particles of a warp share most of their
  * 27 neighbour cells, so neighbour data comes from L1/L2 rather than HBM.  Inside the
  * neighbour loops 1/r comes from rsqrtf and 1/rho_j from aux or the correctly rounded
  * reciprocal of the density (FP32 results differ from the
@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(256) k_aux(int n, const float* __restrict__ de
 #endif
 /* MON: compute_normals with the Monaghan kernels, GRAD_W_DEFAULT(r, r.r, h) / rho_j
  * (normals.cl:66; the kernel text passes r^2 where the function takes |r|). */
-template <bool LIST, bool EXACT, bool BATCH, bool MON = false, bool PRHO = false, int W = 1>
+/* W > 1: ORD adds in list order (PCISPH), else by lane. */
+template <bool LIST, bool EXACT, bool BATCH, bool MON = false, bool PRHO = false, int W = 1, bool ORD = false>
 __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl0, const float4* __restrict__ aux,
                                                  const float* __restrict__ dens, float4* __restrict__ normal,
                                                  const SceneDev* __restrict__ scenes,
@@ -226,7 +227,24 @@ __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl
             nz += dz * k;
         }
     };
-    if constexpr (W > 1) {
+    if constexpr (W > 1 && ORD) {
+        __shared__ float2 s_fac[256 * 3];
+        const int w = lane_of_particle<W>(c);
+        float total[3];
+        ordered_walk<W>(i, c.n, fl.list, w < W ? __ldg(&fl.len[i]) : 0, i, s_fac, total,
+                        [&](int j) { return __ldg(&fl.npos[j]); }, [&](float4 q, bool in, float2 (&f)[3]) {
+            const float dx = __fsub_rn(pi.x, q.x), dy = __fsub_rn(pi.y, q.y), dz = __fsub_rn(pi.z, q.z);
+            const float t = HH - (dx * dx + dy * dy + dz * dz);
+            const float k = in ? (t * t) * __frcp_rn(q.w) : 0.f;
+            f[0] = make_float2(dx, k);
+            f[1] = make_float2(dy, k);
+            f[2] = make_float2(dz, k);
+        });
+        if (w != 0) return;
+        nx = total[0];
+        ny = total[1];
+        nz = total[2];
+    } else if constexpr (W > 1) {
         const int w = lane_of_particle<W>(c);
         list_neighbors_split<W>(i, c.n, fl.list, w < W ? __ldg(&fl.len[i]) : 0, w, i, fl.npos, pi.x, pi.y, pi.z, pair);
         nx = sum_lanes<W>(nx);
@@ -296,7 +314,8 @@ __device__ __forceinline__ void wc_integrate_one(const Const& c, float4 p, float
  * three separate loads; rho_j = 1/(1/rho_j) enters only the symmetrised surface-tension
  * factor 2 rho0 / (rho_i + rho_j) = 2 rho0 R_j / (rho_i R_j + 1). */
 template <bool COMPAT, bool LIST, bool FUSE, bool WRITE_ACC, bool ST, bool BATCH, bool PACK = false, int W = 1>
-__global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS) k_wc_forces(Const c0, Neigh<LIST, COMPAT> fl0, Neigh<LIST, COMPAT> bl0, Bufs b) {
+__global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS)
+    k_wc_forces(Const c0, Neigh<LIST, COMPAT> fl0, Neigh<LIST, COMPAT> bl0, Bufs b) {
   chain_next();
   for_each_particle<BATCH, W>(c0, b.tiles, b.scenes, [&](const Const& c, long long base, int i, const SceneDev* sd) {
     constexpr bool REC = PACK && !ST;   /* nrec holds store_rec's records, position included */
@@ -585,25 +604,29 @@ void launch_aux(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
 static int split_walk(const Const& c, int num_sms) { return c.compat ? 1 : walk_lanes(c.n, num_sms); }
 
 template <int W>
-static void normals_split(cudaStream_t s, const Const& c0, const Bufs& b, float4* nrec) {
+static void normals_split(cudaStream_t s, const Const& c0, const Bufs& b, float4* nrec, bool ordered) {
     Const c = c0;
     c.first = 0;
     c.last = c.n;
     auto fl = fluid_src<true, true>(b);
     fl.npos = b.prho;
     /* the lists hold a batch's pairs, so the pass is the same for it */
-    launch_chained(s, k_normals<true, true, false, false, true, W>, nblk(c.n * W, 256), 256, 0, c, fl, b.aux,
-                   b.density, b.normal, b.scenes, b.tiles, b.vel_s, nrec);
+    auto kernel = k_normals<true, true, false, false, true, W>;
+    if constexpr (W != 2)
+        if (ordered) kernel = k_normals<true, true, false, false, true, W, true>;
+    launch_chained(s, kernel, nblk(c.n * W, 256), 256, 0, c, fl, b.aux, b.density, b.normal, b.scenes, b.tiles,
+                   b.vel_s, nrec);
 }
 
-void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack, bool prho) {
+void launch_normals(cudaStream_t s, const Const& c, const Bufs& b, bool lists, int bs, int num_sms, bool pack,
+                    bool prho, bool ordered) {
     if (c.n <= 0) return;
     if (prho && lists) {
         float4* rec = pack ? b.nrec : nullptr;
-        switch (split_walk(c, num_sms)) {
-        case 8: normals_split<8>(s, c, b, rec); return;
-        case 4: normals_split<4>(s, c, b, rec); return;
-        case 2: normals_split<2>(s, c, b, rec); return;
+        switch (ordered ? ordered_lanes(c.n, num_sms) : split_walk(c, num_sms)) {
+        case 8: normals_split<8>(s, c, b, rec, ordered); return;
+        case 4: normals_split<4>(s, c, b, rec, ordered); return;
+        case 2: normals_split<2>(s, c, b, rec, ordered); return;
         }
     }
     const int g = nblk(c.n, bs), gt = grid_for<true>(c, bs);
