@@ -1723,6 +1723,7 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
     std::lock_guard<std::mutex> lk(g_sort.mu);
     int dev = 0;
     cudaGetDevice(&dev);
+    cudaStream_t s = (cudaStream_t)stream;
     const size_t need = sph::sort_workspace_bytes(n, key_bits);
     if (g_sort.device != dev || g_sort.n_cap < (size_t)n || g_sort.ws_bytes < need) {
         if (g_sort.ws && g_sort.device == dev) {
@@ -1740,8 +1741,10 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
             cudaGetLastError();
             return fail(nullptr, SPH_E_NOMEM, "sph_sort_pairs: scratch allocation failed");
         }
-        cudaMemset(g_sort.flags, 0, 16);
-        cudaMemset(g_sort.ws, 0, wsb);   /* the sort's grid barrier starts at zero */
+        /* the sort's grid barrier starts at zero; on the caller's stream, which need not wait for
+         * the default stream's work */
+        cudaMemsetAsync(g_sort.flags, 0, 16, s);
+        cudaMemsetAsync(g_sort.ws, 0, wsb, s);
         if (cudaEventCreateWithFlags(&g_sort.done, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
             g_sort.done = nullptr;
@@ -1751,7 +1754,6 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
     }
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaStream_t s = (cudaStream_t)stream;
     /* calls on different streams share the scratch: each waits on the GPU for the previous
        one (outside stream capture, where an outside event cannot be waited on) */
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
