@@ -457,7 +457,6 @@ int sph_adj_create(sph_ctx* ctx, int steps, int checkpoint_every, sph_adj** out)
     cudaMemsetAsync(a->tab, 0, sizeof(int2) * (size_t)a->c.ncells, s);
     cudaMemsetAsync(a->cell_prev, 0xff, 4 * (size_t)a->N, s);
     cudaMemsetAsync(a->flags, 0, 16, s);
-    cudaMemsetAsync(a->sort_ws, 0, sph::sort_workspace_bytes(a->N, a->c.key_bits), s);
     sph::k_adj_iota<<<sph::blocks(a->N, 256), 256, 0, s>>>(a->N, a->iota);
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {

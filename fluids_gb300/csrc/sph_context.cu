@@ -1741,10 +1741,8 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
             cudaGetLastError();
             return fail(nullptr, SPH_E_NOMEM, "sph_sort_pairs: scratch allocation failed");
         }
-        /* the sort's grid barrier starts at zero; on the caller's stream, which need not wait for
-         * the default stream's work */
+        /* on the caller's stream, which need not wait for the default stream's work */
         cudaMemsetAsync(g_sort.flags, 0, 16, s);
-        cudaMemsetAsync(g_sort.ws, 0, wsb, s);
         if (cudaEventCreateWithFlags(&g_sort.done, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
             g_sort.done = nullptr;

@@ -746,12 +746,10 @@ static int splat_order(sph_ctx* x, const sph::View& v, const int32_t*& sorted) {
             return sph_ctx_fail(x, SPH_E_NOMEM, "render: particle order buffers");
         }
         x->render_sort_bytes = nsort;
-        /* the sort workspace starts at zero */
-        cudaMemsetAsync(x->render_sort, 0, sph::sort_workspace_bytes(x->N, 16), x->stream);
     }
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
-    void* ws = x->render_sort;   /* first, so that it stays in place when the particle count changes */
+    void* ws = x->render_sort;
     uint32_t* okeys = reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + sph::sort_workspace_bytes(n, 16));
     int32_t* order = reinterpret_cast<int32_t*>(okeys + n);
     uint32_t* okeys_alt = reinterpret_cast<uint32_t*>(order + n);

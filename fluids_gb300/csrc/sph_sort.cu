@@ -447,8 +447,8 @@ void sort_launches(cudaStream_t s, const SortBufs& b, int n, int passes, uint32_
     }
 }
 
-/* The sort of (b.kin, b.vin) by passes whose outputs b names.  ws: sort_workspace_bytes, zero
- * before the first call.  gate: null, or a flag word an earlier kernel of the stream wrote;
+/* The sort of (b.kin, b.vin) by passes whose outputs b names.  ws: sort_workspace_bytes, of any
+ * content.  gate: null, or a flag word an earlier kernel of the stream wrote;
  * every kernel of the sort leaves at once while it is 0. */
 void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned* gate, int key_bits, void* ws,
                        unsigned* flags, int num_sms) {
@@ -460,7 +460,7 @@ void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned*
     const int one = n <= kOneSolo ? 1 : (n + kOneTile - 1) / kOneTile;
     if (one <= kOneTiles && one <= 2 * num_sms) {
         SortBufs bb = b;
-        unsigned* bar = counters + 32;   /* zero between sorts */
+        unsigned* bar = counters + 32;
         uint32_t* counts = status;
         int nn = n, np = passes;
         void* args[] = {&bb, &nn, &np, &counts, &bar, &flags, &gate};
@@ -473,6 +473,9 @@ void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned*
                 return;
         }
         void* fn = n <= kOneSolo ? (void*)k_sort_one<8> : (void*)k_sort_one<4>;
+        /* a barrier whose wait ran out leaves arrivals behind, and the next launch's barriers
+         * would open too early: its words start at zero in each launch */
+        cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s);
         if (cudaLaunchCooperativeKernel(fn, dim3(one), dim3(kOneThreads), args, 0, s) == cudaSuccess) return;
         cudaGetLastError();   /* then by several launches */
     }

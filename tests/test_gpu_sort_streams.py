@@ -1,11 +1,15 @@
 """sph_sort_pairs on non-blocking streams: its scratch is the process's, and nothing of a call
 may depend on, or run beside, what other streams have queued."""
+import ctypes as C
 import os
 import subprocess
 import sys
 
 import numpy as np
 import pytest
+import torch
+
+from fluids_gb300 import capi
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +49,27 @@ def _run(code):
 
 def test_growing_scratch_beside_a_busy_default_stream(gpu_lib):
     assert "sorted" in _run(BUSY_DEFAULT)
+
+
+@pytest.mark.parametrize("n", [65_537, 300_001, 524_288])
+def test_barrier_words_left_by_a_timed_out_sort(gpu_lib, n):
+    """A cooperative sort whose wait ran out leaves arrivals in its barrier: the next sort on the
+    workspace (sph::sort_pairs, as the context's sorts call it) is right all the same."""
+    f = getattr(capi.lib(), "_ZN3sph10sort_pairsEP11CUstream_stPjPiS2_S3_iiPvS2_iPS2_PS3_")
+    f.restype = None
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 1 << 24, size=n, dtype=np.int64).astype(np.uint32)
+    k0 = torch.from_numpy(keys.view(np.int32)).cuda()
+    v0 = torch.arange(n, dtype=torch.int32, device="cuda")
+    k1, v1 = torch.empty_like(k0), torch.empty_like(v0)
+    ws = torch.full((4 * 256 + 64 + 1024 * 256,), 37, dtype=torch.int32, device="cuda")   # barrier words included
+    flags = torch.zeros(4, dtype=torch.int32, device="cuda")
+    kr, vr = C.c_void_p(), C.c_void_p()
+    torch.cuda.synchronize()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    f(C.c_void_p(0), *[C.c_void_p(t.data_ptr()) for t in (k0, v0, k1, v1)], C.c_int(n), C.c_int(24),
+      C.c_void_p(ws.data_ptr()), C.c_void_p(flags.data_ptr()), C.c_int(sms), C.byref(kr), C.byref(vr))
+    torch.cuda.synchronize()
+    assert flags[0].item() == 0
+    got = {t.data_ptr(): t for t in (v0, v1)}[vr.value]
+    assert np.array_equal(got.cpu().numpy(), np.argsort(keys, kind="stable").astype(np.int32))
