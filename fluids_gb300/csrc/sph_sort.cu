@@ -68,6 +68,19 @@ __device__ __forceinline__ unsigned same_digit(uint32_t d) {
     }
     return peers;
 }
+/* same_digit for a warp whose digits may be few (nearly sorted keys of any caller): by match_any
+ * where an earlier round of the warp's keys, told by `few`, held at most kFewDigits of them.
+ * Measured on GB300 (us; ballots alone, then with the choice at 4, 8 and 12 digits): 4,194,304 nearly
+ * sorted pairs of 16 bits 115, 99, 96, 96; of seven keys 112, 112, 94, 94; random ones 139 in all. */
+constexpr int kFewDigits = 8;
+template <bool FEW>
+__device__ __forceinline__ unsigned same_digit(uint32_t d, bool few) {
+    return FEW || few ? __match_any_sync(0xffffffffu, d) : same_digit<false>(d);
+}
+/* Whether the warp's round with these peers had few digits. */
+__device__ __forceinline__ bool few_digits(unsigned peers, unsigned lt_mask) {
+    return __popc(__ballot_sync(0xffffffffu, (peers & lt_mask) == 0u)) <= kFewDigits;
+}
 
 /* Exclusive prefix sum over the 256 values held one per thread by the first 256 threads
  * (every thread of the block calls it). */
@@ -109,6 +122,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
     for (int t = threadIdx.x; t < 4 * 256; t += kThreads) (&s_hist[0][0])[t] = 0u;
     __syncthreads();
     const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
     const long long step = (long long)gridDim.x * kThreads * kHistItems;
     for (long long base = (long long)blockIdx.x * kThreads * kHistItems; base < n; base += step) {
         uint32_t k[kHistItems];
@@ -117,6 +131,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
             const long long i = base + (long long)u * kThreads + threadIdx.x;
             k[u] = i < n ? __ldg(&keys[i]) : 0u;
         }
+        unsigned few = 0u;   /* the passes of few digits */
 #pragma unroll
         for (int u = 0; u < kHistItems; ++u) {
             const long long i = base + (long long)u * kThreads + threadIdx.x;
@@ -124,7 +139,8 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
             const unsigned active = __ballot_sync(0xffffffffu, valid);
             for (int p = 0; p < passes; ++p) {
                 const uint32_t d = (k[u] >> (8 * p)) & 255u;
-                const unsigned peers = same_digit<FEW>(d) & active;
+                const unsigned all = same_digit<FEW>(d, (few >> p) & 1u), peers = all & active;
+                if (!FEW && u == 0 && few_digits(all, lt_mask)) few |= 1u << p;
                 if (valid && lane == __ffs(peers) - 1) atomicAdd(&s_hist[p][d], (uint32_t)__popc(peers));
             }
         }
@@ -136,8 +152,12 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
     }
 }
 
+/* Three blocks an SM (80 registers, no spills): the look-back's words in flight took it to 128
+ * registers and two blocks, and sorts of 16,000,000 nearly sorted pairs (16 bits) from 284 us to
+ * 304 against 265 now; 1,062,234 random pairs (32 bits) 104 us either way.  Four blocks gain another
+ * 5 % there and lose 3 to 8 % below 1,500,000 pairs. */
 template <bool FEW>
-__global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
+__global__ void __launch_bounds__(kThreads, 3) k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                                                        uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int n,
                                                        int shift, int pass, int tiles,
                                                        const uint32_t* __restrict__ hist,
@@ -175,10 +195,12 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint32_t* __restric
         key[k] = valid ? __ldg(&kin[idx]) : 0xffffffffu;   /* tail keys sort last and are not written */
         val[k] = valid ? (vin ? __ldg(&vin[idx]) : (int32_t)idx) : 0;   /* no vin: the identity */
     }
+    bool few = false;
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
         const uint32_t d = (key[k] >> shift) & 255u;
-        const unsigned peers = same_digit<FEW>(d);
+        const unsigned peers = same_digit<FEW>(d, few);
+        if (!FEW && k == 0) few = few_digits(peers, lt_mask);
         const uint32_t before = s_whist[warp][d];
         __syncwarp();
         if ((peers & lt_mask) == 0u) s_whist[warp][d] = before + (uint32_t)__popc(peers);
