@@ -140,7 +140,7 @@ __global__ void k_bnd_forces(Const c, int nb, const float4* __restrict__ bpos, c
 
 /* k_bnd_forces on the clamped (PHYSICS) grid with kSplitLanes lanes a boundary particle, for the
  * particles of bodies with mass (idx): one thread's scan of 27 cells took 85 us on GB300 for
- * any number of particles.  The pairs are those within the list test's r^2 < h^2, at most cap
+ * any number of particles up to what the GPU holds at once.  The pairs are those within the list test's r^2 < h^2, at most cap
  * of them in list order; a lane adds the pairs it finds and the lanes' sums are added. */
 __global__ void __launch_bounds__(256) k_bnd_forces_split(Const c, int count, const int32_t* __restrict__ idx,
                                                           const float4* __restrict__ bpos,
@@ -408,9 +408,14 @@ __device__ void body_step(float* t, const float* d, float4 F, float4 T, float g,
     }
 }
 
-void launch_bnd_forces(cudaStream_t s, const Const& c, const Bufs& b, int nbodies, int nmass, bool dynamic, int bs) {
+/* Lanes for up to 512 particles an SM (77,824 on 152), where the GPU holds two waves of them; a thread
+ * a particle beyond.  Measured on GB300 (WCSPH step, us, lanes and threads): a body of 40,000
+ * particles inside 8,000 of fluid 391 / 452, mostly outside 105 / 95; of 100,000 929 / 934 and
+ * 187 / 154; of 800,000 6997 / 6775 and 1017 / 738. */
+void launch_bnd_forces(cudaStream_t s, const Const& c, const Bufs& b, int nbodies, int nmass, bool dynamic, int bs,
+                       int num_sms) {
     if (c.nb <= 0 || nbodies <= 0) return;
-    if (!c.compat && !c.wrap && nmass > 0) {
+    if (!c.compat && !c.wrap && nmass > 0 && nmass <= 512LL * num_sms) {
         const int per = 256 / kSplitLanes;
         k_bnd_forces_split<<<nblk(nmass, per), 256, 0, s>>>(c, nmass, b.bmass, b.bpos, b.bphi, b.bbody, b.body_xf,
                                                             b.pos_s, b.density, b.pressure, b.tab, b.bft);

@@ -223,7 +223,8 @@ void launch_bnd_phi(cudaStream_t s, const Const& c, const Bufs& b, float phi_coe
 void launch_bnd_near(cudaStream_t s, const Const& c, const Bufs& b, int nb, int bs);
 /* the fluid's force and torque on every body with mass (nmass particles of such bodies, listed
  * in b.bmass); dynamic: then advances every dynamic body by one step under them and gravity */
-void launch_bnd_forces(cudaStream_t s, const Const& c, const Bufs& b, int nbodies, int nmass, bool dynamic, int bs);
+void launch_bnd_forces(cudaStream_t s, const Const& c, const Bufs& b, int nbodies, int nmass, bool dynamic, int bs,
+                       int num_sms);
 void launch_stats(cudaStream_t s, const Const& c, const Bufs& b);
 void launch_scene_stats(cudaStream_t s, const Const& c, const Bufs& b, double* out, int nscenes);
 
