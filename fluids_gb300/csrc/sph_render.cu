@@ -119,17 +119,11 @@ __global__ void k_depth_order(View v, int n, const float4* __restrict__ pos, uin
     vals[i] = i;
 }
 
-__global__ void k_splat_keys(View v, int n, const float4* __restrict__ pos, const int32_t* __restrict__ order,
-                             unsigned long long* __restrict__ key) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int i = order[t];
-    float e[4], wx, wy, size;
-    if (!sprite(v, pos[i], e, wx, wy, size)) return;
-    /* a pixel already nearer than this sprite can get is skipped before any fragment arithmetic:
-       keys only decrease, so a stale read (even an L1 copy older than other CTAs' atomics)
-       only costs the full test */
-    const unsigned floor_bits = __float_as_uint(depth_floor(v, e));
+/* All pixels of a sprite by one thread.  A pixel already nearer than the sprite can get (floor_bits)
+ * is skipped before any fragment arithmetic: keys only decrease, so a stale read (even an L1 copy
+ * older than other CTAs' atomics) only costs the full test. */
+__device__ __forceinline__ void splat_sprite(const View& v, const float e[4], float wx, float wy, float size,
+                                             unsigned floor_bits, int i, unsigned long long* __restrict__ key) {
     const int x0 = max(0, (int)floorf(wx - 0.5f * size)), x1 = min(v.w - 1, (int)ceilf(wx + 0.5f * size));
     const int y0 = max(0, (int)floorf(wy - 0.5f * size)), y1 = min(v.h - 1, (int)ceilf(wy + 0.5f * size));
     constexpr int kAhead = 8;   /* key loads in flight per thread */
@@ -151,6 +145,16 @@ __global__ void k_splat_keys(View v, int n, const float4* __restrict__ pos, cons
             }
         }
     }
+}
+
+__global__ void k_splat_keys(View v, int n, const float4* __restrict__ pos, const int32_t* __restrict__ order,
+                             unsigned long long* __restrict__ key) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int i = order[t];
+    float e[4], wx, wy, size;
+    if (!sprite(v, pos[i], e, wx, wy, size)) return;
+    splat_sprite(v, e, wx, wy, size, __float_as_uint(depth_floor(v, e)), i, key);
 }
 
 /* Depth bounds of square tiles of pixels (side 1 << shift), so that the sprites behind the
@@ -204,19 +208,43 @@ __global__ void __launch_bounds__(256) k_cover(View v, int n, const float4* __re
     }
 }
 
-/* The particles test their tiles, and the few (particle, tile) pairs that pass -- about one in a
- * hundred, nearly all in the blocks of the surface and the silhouette -- go to a list (a block
- * reserves its part at once), so that k_splat_pairs spreads them over the GPU.  A pair past the
- * list's end is splatted by its own thread, and so are those of sprites of more than 32 tiles. */
-__device__ __forceinline__ void splat_pixel(const View& v, const float e[4], float wx, float wy, float size, int i,
-                                            int px, int py, unsigned long long* __restrict__ key) {
-    if (px >= v.w || py >= v.h) return;
-    unsigned long long* const at = key + (size_t)py * v.w + px;
-    const unsigned long long cur = __ldca(at);   /* L1 copy: stale is still safe */
-    float nd, lin;
-    if (!fragment(v, e, wx, wy, size, px, py, nd, lin)) return;
-    const unsigned long long k = ((unsigned long long)__float_as_uint(lin) << 32) | (unsigned)i;
-    if (k < cur) atomicMin(at, k);
+/* A tile of a sprite by 16 lanes (lane: 0..15), a pixel each at a time. */
+__device__ __forceinline__ void splat_tile(const View& v, const float e[4], float wx, float wy, float size,
+                                           unsigned floor_bits, int i, int tx, int ty, int shift, int lane,
+                                           unsigned long long* __restrict__ key) {
+    const int side = 1 << shift;
+    for (int q = lane; q < side * side; q += 16) {
+        const int px = (tx << shift) + (q & (side - 1)), py = (ty << shift) + (q >> shift);
+        if (px >= v.w || py >= v.h) continue;
+        unsigned long long* const at = key + (size_t)py * v.w + px;
+        const unsigned long long cur = __ldca(at);
+        if ((unsigned)(cur >> 32) < floor_bits) continue;
+        float nd, lin;
+        if (!fragment(v, e, wx, wy, size, px, py, nd, lin)) continue;
+        const unsigned long long k = ((unsigned long long)__float_as_uint(lin) << 32) | (unsigned)i;
+        if (k < cur) atomicMin(at, k);
+    }
+}
+/* The tiles that a sprite's square touches: [x0, x1] x [y0, y1], empty when x1 < x0 or y1 < y0. */
+__device__ __forceinline__ void sprite_tiles(const View& v, float wx, float wy, float size, int shift, int& x0, int& y0,
+                                             int& x1, int& y1) {
+    x0 = max(0, (int)floorf(wx - 0.5f * size)) >> shift;
+    y0 = max(0, (int)floorf(wy - 0.5f * size)) >> shift;
+    x1 = min(v.w - 1, (int)ceilf(wx + 0.5f * size)) >> shift;
+    y1 = min(v.h - 1, (int)ceilf(wy + 0.5f * size)) >> shift;
+}
+/* Whether a sprite may show in a tile: its nearest fragment there, at the pixel centre nearest to
+ * the sprite's, is not behind the tile's bound. */
+__device__ __forceinline__ bool tile_shows(const View& v, const float e[4], float wx, float wy, float inv,
+                                           unsigned floor_bits, unsigned bound, int tx, int ty, int shift) {
+    if (floor_bits > bound) return false;
+    const float last = (float)((1 << shift) - 1);
+    const float xa = (float)(tx << shift) + 0.5f, ya = (float)(ty << shift) + 0.5f;
+    const float dx = inv * fmaxf(0.0f, fmaxf(xa - wx, wx - (xa + last)));
+    const float dy = inv * fmaxf(0.0f, fmaxf(ya - wy, wy - (ya + last)));
+    const float mag = (dx * dx + dy * dy) * 0.999f;
+    if (mag > 1.0f) return false;   /* every pixel of it lies outside the disc */
+    return __float_as_uint(depth_floor(v, e, sqrtf(1.0f - mag))) <= bound;
 }
 
 /* The farthest bound of each 4 x 4 tiles: most hidden sprites are told by one to four of these. */
@@ -231,53 +259,48 @@ __global__ void __launch_bounds__(256) k_tile_max(int tw, int th, const unsigned
     coarse[k] = m;
 }
 
+/* The particles test their tiles.  Behind a closed surface few (particle, tile) pairs pass -- about
+ * one in a hundred, nearly all in the blocks of the surface and the silhouette -- and go to a list
+ * (a block reserves its part at once), so that k_splat_pairs spreads them over the GPU.  A sprite
+ * whose entries lie past the list's end is splatted by its own thread; one of more than 32 tiles is
+ * one entry, kWhole. */
+constexpr int kWhole = -1;
 __global__ void __launch_bounds__(256) k_splat_cull(View v, int n, const float4* __restrict__ pos, int shift, int tw,
                                                     const unsigned* __restrict__ tile, int cw,
                                                     const unsigned* __restrict__ coarse,
                                                     unsigned long long* __restrict__ key, int2* __restrict__ list,
                                                     unsigned cap, unsigned* __restrict__ count) {
     __shared__ unsigned s_sum[8], s_base;
+    constexpr unsigned kAll = 0xffffffffu;
     const int t = threadIdx.x, i = blockIdx.x * 256 + t, lane = t & 31, warp = t >> 5;
-    const int side = 1 << shift;
     float e[4], wx = 0.f, wy = 0.f, size = 1.f;
-    unsigned passed = 0;   /* the tiles that pass, in row order, of the first 32 */
-    int tx0 = 0, ty0 = 0, nx = 0, ny = 0;
+    unsigned passed = 0, floor_bits = 0;   /* the tiles that pass, in row order */
+    int x0 = 0, y0 = 0, x1 = -1, y1 = -1;
+    bool whole = false;
     if (i < n && sprite(v, pos[i], e, wx, wy, size)) {
-        const unsigned floor_bits = __float_as_uint(depth_floor(v, e));
+        floor_bits = __float_as_uint(depth_floor(v, e));
         const float inv = 2.0f / size;
-        tx0 = max(0, (int)floorf(wx - 0.5f * size)) >> shift;
-        ty0 = max(0, (int)floorf(wy - 0.5f * size)) >> shift;
-        nx = (min(v.w - 1, (int)ceilf(wx + 0.5f * size)) >> shift) - tx0 + 1;
-        ny = (min(v.h - 1, (int)ceilf(wy + 0.5f * size)) >> shift) - ty0 + 1;
+        sprite_tiles(v, wx, wy, size, shift, x0, y0, x1, y1);
+        const int nx = x1 - x0 + 1, ny = y1 - y0 + 1;
+        whole = nx > 0 && ny > 0 && (nx > 32 || ny > 32 || nx * ny > 32);
         bool hidden = true;
-        for (int cy = ty0 >> 2; cy <= (ty0 + ny - 1) >> 2; ++cy)
-            for (int cx = tx0 >> 2; cx <= (tx0 + nx - 1) >> 2; ++cx)
-                hidden = hidden && floor_bits > __ldg(&coarse[(size_t)cy * cw + cx]);
-        if (hidden) ny = 0;
-        int q = 0;
-        for (int ty = ty0; ty < ty0 + ny; ++ty)
-            for (int tx = tx0; tx < tx0 + nx; ++tx, ++q) {
-                const unsigned bound = __ldg(&tile[(size_t)ty * tw + tx]);
-                if (floor_bits > bound) continue;
-                /* the nearest fragment in this tile: at its pixel centre nearest to the sprite's */
-                const float xa = (float)(tx << shift) + 0.5f, ya = (float)(ty << shift) + 0.5f;
-                const float dx = inv * fmaxf(0.0f, fmaxf(xa - wx, wx - (xa + (float)(side - 1))));
-                const float dy = inv * fmaxf(0.0f, fmaxf(ya - wy, wy - (ya + (float)(side - 1))));
-                const float mag = (dx * dx + dy * dy) * 0.999f;
-                if (mag > 1.0f) continue;   /* every pixel of it lies outside the disc */
-                if (__float_as_uint(depth_floor(v, e, sqrtf(1.0f - mag))) > bound) continue;
-                if (q < 32) passed |= 1u << q;
-                else
-                    for (int k = 0; k < side * side; ++k)
-                        splat_pixel(v, e, wx, wy, size, i, (tx << shift) + (k & (side - 1)), (ty << shift) + (k >> shift),
-                                    key);
-            }
+        if (!whole)
+            for (int cy = y0 >> 2; cy <= y1 >> 2; ++cy)
+                for (int cx = x0 >> 2; cx <= x1 >> 2; ++cx)
+                    hidden = hidden && floor_bits > __ldg(&coarse[(size_t)cy * cw + cx]);
+        if (!hidden) {
+            int q = 0;
+            for (int ty = y0; ty <= y1; ++ty)
+                for (int tx = x0; tx <= x1; ++tx, ++q)
+                    if (tile_shows(v, e, wx, wy, inv, floor_bits, __ldg(&tile[(size_t)ty * tw + tx]), tx, ty, shift))
+                        passed |= 1u << q;
+        }
     }
-    const unsigned mine = (unsigned)__popc(passed);
+    const unsigned mine = whole ? 1u : (unsigned)__popc(passed);
     unsigned sum = mine;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const unsigned o = __shfl_up_sync(0xffffffffu, sum, d);
+        const unsigned o = __shfl_up_sync(kAll, sum, d);
         if (lane >= d) sum += o;
     }
     if (lane == 31) s_sum[warp] = sum;
@@ -292,30 +315,61 @@ __global__ void __launch_bounds__(256) k_splat_cull(View v, int n, const float4*
         s_base = all ? atomicAdd(count, all) : 0u;
     }
     __syncthreads();
-    unsigned at = s_base + s_sum[warp] + sum - mine;
-    for (; passed; passed &= passed - 1u, ++at) {
-        const int q = __ffs((int)passed) - 1, tx = tx0 + q % nx, ty = ty0 + q / nx;
-        if (at < cap) list[at] = make_int2(i, ty * tw + tx);
-        else
-            for (int k = 0; k < side * side; ++k)
-                splat_pixel(v, e, wx, wy, size, i, (tx << shift) + (k & (side - 1)), (ty << shift) + (k >> shift), key);
+    if (mine != 0u) {
+        const unsigned at = s_base + s_sum[warp] + sum - mine;
+        if (whole) {
+            if (at < cap) list[at] = make_int2(i, kWhole);
+        } else {
+            unsigned k = at;
+            for (unsigned m = passed; m && k < cap; m &= m - 1u, ++k) {
+                const int q = __ffs((int)m) - 1, nx = x1 - x0 + 1;
+                list[k] = make_int2(i, (y0 + q / nx) * tw + x0 + q % nx);
+            }
+        }
+        if (at + mine > cap) splat_sprite(v, e, wx, wy, size, floor_bits, i, key);
     }
 }
 
-/* The listed pairs, 16 lanes each. */
+/* The list's entries, 16 lanes each.  A whole sprite's lanes test a coarse bound each, then the
+ * tiles of those that pass. */
 __global__ void __launch_bounds__(256) k_splat_pairs(View v, const float4* __restrict__ pos, int shift, int tw,
+                                                     const unsigned* __restrict__ tile, int cw,
+                                                     const unsigned* __restrict__ coarse,
                                                      unsigned long long* __restrict__ key,
                                                      const int2* __restrict__ list, unsigned cap,
                                                      const unsigned* __restrict__ count) {
     const unsigned m = min(*count, cap);
-    const int side = 1 << shift;
+    const int lane = threadIdx.x & 15, first = threadIdx.x & 16;
+    const unsigned group = 0xffffu << first;
     for (unsigned k = (blockIdx.x * 256 + threadIdx.x) >> 4; k < m; k += gridDim.x * 16) {
         const int2 w = __ldg(&list[k]);
         float e[4], wx, wy, size;
-        if (!sprite(v, __ldg(&pos[w.x]), e, wx, wy, size)) continue;
-        const int ty = w.y / tw, tx = w.y - ty * tw;
-        for (int q = threadIdx.x & 15; q < side * side; q += 16)
-            splat_pixel(v, e, wx, wy, size, w.x, (tx << shift) + (q & (side - 1)), (ty << shift) + (q >> shift), key);
+        if (!sprite(v, __ldg(&pos[w.x]), e, wx, wy, size)) continue;   /* the same in the 16 lanes */
+        if (w.y != kWhole) {   /* the floor of a tile that passed would cost more than it saves */
+            const int ty = w.y / tw;
+            splat_tile(v, e, wx, wy, size, 0u, w.x, w.y - ty * tw, ty, shift, lane, key);
+            continue;
+        }
+        const unsigned floor_bits = __float_as_uint(depth_floor(v, e));
+        int x0, y0, x1, y1;
+        sprite_tiles(v, wx, wy, size, shift, x0, y0, x1, y1);
+        const float inv = 2.0f / size;
+        const int cx0 = x0 >> 2, cy0 = y0 >> 2, cnx = (x1 >> 2) - cx0 + 1, cells = cnx * ((y1 >> 2) - cy0 + 1);
+        for (int c0 = 0; c0 < cells; c0 += 16) {
+            const int c = c0 + lane;
+            const bool open = c < cells && floor_bits <= __ldg(&coarse[(size_t)(cy0 + c / cnx) * cw + cx0 + c % cnx]);
+            for (unsigned mc = __ballot_sync(group, open) >> first; mc; mc &= mc - 1u) {
+                const int cc = c0 + __ffs((int)mc) - 1;
+                const int bx = 4 * (cx0 + cc % cnx), by = 4 * (cy0 + cc / cnx), tx = bx + (lane & 3), ty = by + (lane >> 2);
+                const bool show =
+                    tx >= x0 && tx <= x1 && ty >= y0 && ty <= y1 &&
+                    tile_shows(v, e, wx, wy, inv, floor_bits, __ldg(&tile[(size_t)ty * tw + tx]), tx, ty, shift);
+                for (unsigned mt = __ballot_sync(group, show) >> first; mt; mt &= mt - 1u) {
+                    const int b = __ffs((int)mt) - 1;
+                    splat_tile(v, e, wx, wy, size, floor_bits, w.x, bx + (b & 3), by + (b >> 2), shift, lane, key);
+                }
+            }
+        }
     }
 }
 
@@ -679,14 +733,23 @@ inline bool image_ok(int w, int h) {
 extern "C" {
 
 /* The tiles of k_cover for a view: their side's shift, or -1 when the sprites, at the distance
- * of the scene's origin, are too small to cover tiles (below 6 pixels) or the projection is
- * not a symmetric one.  4 pixels to a side below 24-pixel sprites, 8 below 48, else 16. */
-static int tile_shift(const sph_view* view) {
+ * of the scene's origin, are too small to cover tiles (below 6 pixels), the projection is not a
+ * symmetric one, or the fluid's surface would not close: sprites less than 1.5 times as wide as the
+ * particles' spacing on the screen let many layers through, nearly every pair passes, and then
+ * the front-to-back order does more than the tiles.  Up to kAnyPairs particles the order's sort
+ * costs more than the pairs.  4 pixels to a side below 24-pixel sprites, 8 below 48, else 16.
+ * Measured on GB300 (depth stage of 3840 x 2160, us, ordered and with tiles): 300,000 particles of 0.7
+ * spacings 152 / 243 (6-pixel sprites) and 420 / 643 (17), of 2.9 459 / 152 (25); 2,000,000 of 1.35
+ * 335 / 460 (6), of 5.4 1592 / 388 (25); 19,683 of 0.3 331 / 285 (17), of 1.2 373 / 141 (25). */
+constexpr int kAnyPairs = 1 << 17;
+static int tile_shift(const sph_ctx* x, const sph_view* view) {
     const float *m = view->projection, *t = view->modelview + 12;
     if (m[8] != 0.f || m[9] != 0.f || m[12] != 0.f || m[13] != 0.f) return -1;
     const float dist = std::sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
     const float size = view->point_radius * (view->point_scale / dist);
     if (!(size >= 6.0f)) return -1;
+    const float spacing = 2.0f * x->p.particle_radius * 0.5f * (float)view->height * std::fabs(m[5]) / dist;
+    if (x->N > kAnyPairs && size < 64.0f && !(size >= 1.5f * spacing)) return -1;
     return size < 24.0f ? 2 : (size < 48.0f ? 3 : 4);
 }
 
@@ -774,7 +837,7 @@ int sph_render_depth(sph_ctx* x, const sph_view* view, float* d_depth) {
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
     const dim3 b2(16, 16);
-    const int shift = tile_shift(view);
+    const int shift = tile_shift(x, view);
     if (shift > 0) {
         const int tw = (v.w + (1 << shift) - 1) >> shift, th = (v.h + (1 << shift) - 1) >> shift;
         const int cw = (tw + 3) / 4, ch = (th + 3) / 4;
@@ -784,7 +847,8 @@ int sph_render_depth(sph_ctx* x, const sph_view* view, float* d_depth) {
         sph::k_tile_max<<<(cw * ch + bs - 1) / bs, bs, 0, s>>>(tw, th, tile, cw, ch, coarse);
         sph::k_splat_cull<<<(n + bs - 1) / bs, bs, 0, s>>>(v, n, x->b.pos, shift, tw, tile, cw, coarse, key, list, cap,
                                                            tile + ntiles);
-        sph::k_splat_pairs<<<4 * x->num_sms, bs, 0, s>>>(v, x->b.pos, shift, tw, key, list, cap, tile + ntiles);
+        sph::k_splat_pairs<<<4 * x->num_sms, bs, 0, s>>>(v, x->b.pos, shift, tw, tile, cw, coarse, key, list, cap,
+                                                         tile + ntiles);
     } else {
         const int32_t* sorted;
         if ((rc = splat_order(x, v, sorted)) != SPH_OK) return rc;
