@@ -936,6 +936,7 @@ struct SortCache {
     uint32_t* kalt = nullptr;
     int32_t* valt = nullptr;
     unsigned* flags = nullptr;
+    void* third = nullptr;        /* keys and values for sorts of three passes; from the first of them on */
     size_t n_cap = 0;
     int device = -1;
     cudaEvent_t done = nullptr;   /* the last sort's end: the next one, on any stream, waits for it */
@@ -1732,16 +1733,18 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
     if (g_sort.device != dev || g_sort.n_cap < (size_t)n || g_sort.ws_bytes < need) {
         if (g_sort.ws && g_sort.device == dev) {
             cudaFree(g_sort.ws); cudaFree(g_sort.kalt); cudaFree(g_sort.valt); cudaFree(g_sort.flags);
+            cudaFree(g_sort.third);
         }
         if (g_sort.done && g_sort.device == dev) cudaEventDestroy(g_sort.done);
         g_sort.done = nullptr;
         g_sort.ws = nullptr; g_sort.kalt = nullptr; g_sort.valt = nullptr; g_sort.flags = nullptr;
+        g_sort.third = nullptr;
         g_sort.ws_bytes = 0; g_sort.n_cap = 0;
         g_sort.device = dev;
         size_t ncap = (size_t)n;
         size_t wsb = sph::sort_workspace_bytes(n, 32);
-        if (cudaMalloc(&g_sort.ws, wsb) != cudaSuccess || cudaMalloc(&g_sort.kalt, 8 * ncap) != cudaSuccess ||
-            cudaMalloc(&g_sort.valt, 8 * ncap) != cudaSuccess || cudaMalloc(&g_sort.flags, 16) != cudaSuccess) {
+        if (cudaMalloc(&g_sort.ws, wsb) != cudaSuccess || cudaMalloc(&g_sort.kalt, 4 * ncap) != cudaSuccess ||
+            cudaMalloc(&g_sort.valt, 4 * ncap) != cudaSuccess || cudaMalloc(&g_sort.flags, 16) != cudaSuccess) {
             cudaGetLastError();
             return fail(nullptr, SPH_E_NOMEM, "sph_sort_pairs: scratch allocation failed");
         }
@@ -1762,15 +1765,32 @@ int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void*
     cudaStreamIsCapturing(s, &cap);
     const bool order = g_sort.done && cap == cudaStreamCaptureStatusNone;
     if (order) cudaStreamWaitEvent(s, g_sort.done, 0);
-    /* the last pass writes the caller's arrays; three passes go through both copies, a single
-     * one through a copy and back */
+    /* pass p reads the one pair of arrays and writes the other, so an odd number of them ends in
+     * the copies; three passes end in the caller's arrays by way of a third pair, where there is
+     * memory for it */
     const int passes = sph::sort_passes(key_bits);
-    uint32_t *ka = g_sort.kalt, *kb = ka + g_sort.n_cap;
-    int32_t *va = g_sort.valt, *vb = va + g_sort.n_cap;
+    uint32_t* ka = g_sort.kalt;
+    int32_t* va = g_sort.valt;
     sph::SortBufs sb{d_keys, d_vals, {ka, d_keys, ka, d_keys}, {va, d_vals, va, d_vals}};
-    if (passes == 3) sb = sph::SortBufs{d_keys, d_vals, {ka, kb, d_keys, nullptr}, {va, vb, d_vals, nullptr}};
+    bool copy = (passes & 1) != 0;
+    if (passes == 3 && !g_sort.third && cap == cudaStreamCaptureStatusNone) {
+        /* allowed beside a capture of another thread's */
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaMalloc(&g_sort.third, 8 * g_sort.n_cap) != cudaSuccess) {
+            cudaGetLastError();
+            g_sort.third = nullptr;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    if (passes == 3 && g_sort.third) {
+        uint32_t* kb = static_cast<uint32_t*>(g_sort.third);
+        int32_t* vb = reinterpret_cast<int32_t*>(kb + g_sort.n_cap);
+        sb = sph::SortBufs{d_keys, d_vals, {ka, kb, d_keys, nullptr}, {va, vb, d_vals, nullptr}};
+        copy = false;
+    }
     sph::sort_pairs_passes(s, sb, n, nullptr, key_bits, g_sort.ws, g_sort.flags, sms);
-    if (passes == 1) {
+    if (copy) {
         cudaMemcpyAsync(d_keys, ka, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(d_vals, va, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
     }

@@ -437,8 +437,9 @@ int sph_render_frame(sph_ctx* ctx, const sph_view* view, int method, int filter_
 
 /* clsort<cl_uint, cl_int> (opencl/algorithms/clsort.h:13-35): stable ascending sort of n
  * (key, value) pairs in place in device memory, on the low key_bits bits (1..32) of the
- * key.  Scratch memory is allocated on first use and cached per device; calls on different
- * streams are ordered on the GPU one after the other (not while a stream is being captured:
+ * key.  Scratch memory is allocated on first use and cached per device: 8 bytes a pair of the
+ * largest sort so far and, once a sort of 17 to 24 key bits has run outside a capture, 8 more, with
+ * 1 KB for every 4,096 pairs and 8 bits of key.  Calls on different streams are ordered on the GPU one after the other (not while a stream is being captured:
  * captured calls must not overlap another call on the GPU). */
 int sph_sort_pairs(uint32_t* d_keys, int32_t* d_vals, int n, int key_bits, void* cuda_stream);
 

@@ -40,6 +40,55 @@ for n in (50_001, 300_007, 700_001):
 print("sorted")
 """
 
+# the scratch of a sort whose passes need one copy of the pairs, then of one that uses two
+MEMORY = """
+import torch
+from fluids_gb300 import capi
+n = 1 << 26
+k = torch.randint(0, 1 << 24, (n,), dtype=torch.int32, device="cuda")
+v = torch.arange(n, dtype=torch.int32, device="cuda")
+capi.sort_pairs_device(k.data_ptr(), v.data_ptr(), 1000, 32)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+used = []
+for bits in (32, 24):
+    capi.sort_pairs_device(k.data_ptr(), v.data_ptr(), n, bits)
+    torch.cuda.synchronize()
+    used.append(free - torch.cuda.mem_get_info()[0])
+status = 4 * 256 * 4 * (n // 4096)
+slack = 16 << 20
+assert used[0] <= 8 * n + status + slack, used
+assert used[1] <= 16 * n + status + slack, used
+print("held", used)
+"""
+
+# captured three-pass sorts on scratch that a four-pass sort laid out
+CAPTURED = """
+import numpy as np, torch
+from fluids_gb300 import capi
+rng = np.random.default_rng(2)
+n = 700_001
+dk = torch.zeros(n, dtype=torch.int32, device="cuda")
+dv = torch.zeros(n, dtype=torch.int32, device="cuda")
+capi.sort_pairs_device(dk.data_ptr(), dv.data_ptr(), n, 32)
+torch.cuda.synchronize()
+sizes, graphs = (5_000, 40_001, 300_007, n), []
+for m in sizes:
+    graphs.append(torch.cuda.CUDAGraph())
+    with torch.cuda.graph(graphs[-1]):
+        capi.sort_pairs_device(dk.data_ptr(), dv.data_ptr(), m, 24, torch.cuda.current_stream().cuda_stream)
+for m, g in list(zip(sizes, graphs)) * 2:
+    keys = rng.integers(0, 1 << 24, size=m, dtype=np.int64).astype(np.uint32)
+    dk[:m].copy_(torch.from_numpy(keys.view(np.int32)))
+    dv[:m].copy_(torch.arange(m, dtype=torch.int32))
+    g.replay()
+    torch.cuda.synchronize()
+    order = np.argsort(keys, kind="stable")
+    assert np.array_equal(dv[:m].cpu().numpy(), order.astype(np.int32)), m
+    assert np.array_equal(dk[:m].cpu().numpy().view(np.uint32), keys[order]), m
+print("replayed")
+"""
+
 
 def _run(code):
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
@@ -49,6 +98,14 @@ def _run(code):
 
 def test_growing_scratch_beside_a_busy_default_stream(gpu_lib):
     assert "sorted" in _run(BUSY_DEFAULT)
+
+
+def test_scratch_held(gpu_lib):
+    assert "held" in _run(MEMORY)
+
+
+def test_three_passes_captured_without_a_third_pair(gpu_lib):
+    assert "replayed" in _run(CAPTURED)
 
 
 @pytest.mark.parametrize("n", [65_537, 300_001, 524_288])
