@@ -757,10 +757,10 @@ static int tile_shift(const sph_ctx* x, const sph_view* view) {
  * all of its tiles, in a crowd one in a hundred pairs does. */
 static size_t splat_list_cap(int n) { return std::min(32 * (size_t)n, 2 * (size_t)n + 524288); }
 
-/* Checks the view, allocates the depth-test keys, the list of pairs, the tile bounds and the
- * pair count (behind the ntiles bounds, before the coarse ones), and clears keys, bounds and
+/* Checks the view, allocates the depth-test keys, the list of pairs (with_list), the tile bounds and
+ * the pair count (behind the ntiles bounds, before the coarse ones), and clears keys, bounds and
  * count. */
-static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigned long long*& key, unsigned*& tile,
+static int splat_prepare(sph_ctx* x, const sph_view* view, bool with_list, sph::View& v, unsigned long long*& key, unsigned*& tile,
                          int2*& list, size_t& ntiles) {
     if (!sph::image_ok(view->width, view->height))
         return sph_ctx_fail(x, SPH_E_INVALID, "render: width and height must be 1..65536 (at most 2^28 pixels)");
@@ -770,7 +770,8 @@ static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigne
     const size_t npix = (size_t)view->width * view->height;
     ntiles = (size_t)((view->width + 3) / 4) * ((view->height + 3) / 4);   /* the most there are */
     const size_t ncoarse = (size_t)((view->width + 15) / 16) * ((view->height + 15) / 16);
-    const size_t need = 8 * npix + 4 * (ntiles + 2 + ncoarse) + 8 * splat_list_cap(x->N);
+    const size_t entries = with_list ? splat_list_cap(x->N) : 0;
+    const size_t need = 8 * npix + 4 * (ntiles + 2 + ncoarse) + 8 * entries;
     if (x->render_bytes < need) {
         cudaStreamSynchronize(x->stream);
         cudaFree(x->render_buf);
@@ -790,7 +791,7 @@ static int splat_prepare(sph_ctx* x, const sph_view* view, sph::View& v, unsigne
     v.h = view->height;
     key = reinterpret_cast<unsigned long long*>(x->render_buf);
     list = reinterpret_cast<int2*>(key + npix);
-    tile = reinterpret_cast<unsigned*>(list + splat_list_cap(x->N));
+    tile = reinterpret_cast<unsigned*>(list + entries);
     sph::k_splat_clear<<<(unsigned)((npix + 255) / 256), 256, 0, x->stream>>>(npix, key, ntiles, tile);
     return SPH_OK;
 }
@@ -832,12 +833,12 @@ int sph_render_depth(sph_ctx* x, const sph_view* view, float* d_depth) {
     unsigned* tile;
     int2* list;
     size_t ntiles;
-    int rc = splat_prepare(x, view, v, key, tile, list, ntiles);
+    const int shift = tile_shift(x, view);
+    int rc = splat_prepare(x, view, shift > 0, v, key, tile, list, ntiles);
     if (rc != SPH_OK) return rc;
     const cudaStream_t s = x->stream;
     const int bs = 256, n = x->N;
     const dim3 b2(16, 16);
-    const int shift = tile_shift(x, view);
     if (shift > 0) {
         const int tw = (v.w + (1 << shift) - 1) >> shift, th = (v.h + (1 << shift) - 1) >> shift;
         const int cw = (tw + 3) / 4, ch = (th + 3) / 4;
@@ -874,7 +875,7 @@ int sph_render_particles(sph_ctx* x, const sph_view* view, const sph_light* ligh
     int2* list;
     size_t ntiles;
     const int32_t* sorted;
-    int rc = splat_prepare(x, view, v, key, tile, list, ntiles);
+    int rc = splat_prepare(x, view, false, v, key, tile, list, ntiles);
     if (rc == SPH_OK) rc = splat_order(x, v, sorted);
     if (rc != SPH_OK) return rc;
     const cudaStream_t s = x->stream;

@@ -381,7 +381,8 @@ typedef struct sph_view {
  * pixel the NDC depth of the nearest sprite fragment (GL_LESS on the normalised depth, the
  * lower particle index winning a tie) and 0 where no sprite covers it.  No background
  * depth texture: fragments beyond the far plane are dropped.  Runs on the context stream;
- * holds about 8.3 bytes per pixel, 16 per particle and up to 4 MB more of scratch in the context. */
+ * the context keeps about 8.3 bytes per pixel of scratch and, by the view, a list of at most 16
+ * bytes per particle and 4 MB, or the particles' order with 16 bytes each. */
 int sph_render_depth(sph_ctx* ctx, const sph_view* view, float* d_depth);
 /* One pass of kernels/bilateral.cl (BilateralFilter::filter, filters/bilateralfilter.cpp:
  * 28-41): d_in and d_out must differ. */
@@ -420,7 +421,8 @@ typedef struct sph_light {
  * (the fragment shader writes none; the lower index wins a tie), lit by up to 8 directional
  * lights: (0, 0, 0, 1) + sum of diffuse * (89, 152, 255, 256) / 256 * max(0, n . -dir),
  * n from the point coordinate; clamped to [0, 1] as a fixed-point framebuffer stores it;
- * (0, 0, 0, 1) where no sprite is.  Into d_rgba (float4 per pixel), on the context stream. */
+ * (0, 0, 0, 1) where no sprite is.  Into d_rgba (float4 per pixel), on the context stream, with
+ * the scratch of sph_render_depth's ordered views. */
 int sph_render_particles(sph_ctx* ctx, const sph_view* view, const sph_light* lights, int nlights, float* d_rgba);
 /* GraphicsSettings::render_method (settings/settings.cpp:47-57). */
 enum sph_render_method { SPH_RENDER_PARTICLES = 0, SPH_RENDER_SCREEN_SPACE = 1 };
