@@ -258,7 +258,8 @@ __device__ __forceinline__ void pci_pressure_force_one(const Const& c, const Buf
         float total[3];
         ordered_walk<W>(i, c.n, b.nlist, w < W ? len : 0, i, s_fac, total, [&](int j) { return b.pci_pc[j]; },
                         [&](float4 pj, bool in, float2 (&f)[3]) {
-            const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            /* past the end: zeros, also for a particle that is not a number, whose list is empty */
+            const float dx = in ? pi.x - pj.x : 0.f, dy = in ? pi.y - pj.y : 0.f, dz = in ? pi.z - pj.z : 0.f;
             const float r2 = dx * dx + dy * dy + dz * dz;
             const float il0 = rsqrtf(r2), l0 = r2 * il0;
             const bool ok = l0 >= 1e-5f;

@@ -236,9 +236,10 @@ __global__ void __launch_bounds__(256) k_normals(Const c0, Neigh<LIST, EXACT> fl
             const float dx = __fsub_rn(pi.x, q.x), dy = __fsub_rn(pi.y, q.y), dz = __fsub_rn(pi.z, q.z);
             const float t = HH - (dx * dx + dy * dy + dz * dz);
             const float k = in ? (t * t) * __frcp_rn(q.w) : 0.f;
-            f[0] = make_float2(dx, k);
-            f[1] = make_float2(dy, k);
-            f[2] = make_float2(dz, k);
+            /* past the end: zeros, also for a particle that is not a number, whose list is empty */
+            f[0] = make_float2(in ? dx : 0.f, k);
+            f[1] = make_float2(in ? dy : 0.f, k);
+            f[2] = make_float2(in ? dz : 0.f, k);
         });
         if (w != 0) return;
         nx = total[0];
