@@ -4,10 +4,10 @@ The threads per block of the step's kernels (sph_set_block_size) are chosen by t
 few steps of the live context at each candidate and keeping the fastest; for a batched
 context the candidates are the shapes of its tiled launches -- threads per block
 and CTAs per SM (sph_set_tile_shape) of the grid whose warps take the 32-particle scene
-tiles.  The choice is
-stored in a JSON file keyed by GPU name, method, mode, batched or not, and the particle
-count rounded to a power of two, so later contexts of the same kind reuse it without
-timing.  The launch shape never changes results (tests/test_autotune.py), only speed.
+tiles (small batches take no tiles, see include/sph_capi.h: their candidates differ in the
+block size of the binning alone).  The choice is stored in a JSON file keyed by GPU name,
+method, mode, batched or not, and the particle count rounded to a power of two, so later
+contexts of the same kind reuse it without timing.  The launch shape never changes results (tests/test_autotune.py), only speed.
 
     from fluids_gb300 import autotune
     choice = autotune.tune(ctx, method=0, mode=1, batched=False)
