@@ -130,3 +130,28 @@ def test_barrier_words_left_by_a_timed_out_sort(gpu_lib, n):
     assert flags[0].item() == 0
     got = {t.data_ptr(): t for t in (v0, v1)}[vr.value]
     assert np.array_equal(got.cpu().numpy(), np.argsort(keys, kind="stable").astype(np.int32))
+
+
+@pytest.mark.parametrize("sizes", [(3_000, 4_000), (30_000, 20_001), (65_536, 40_000), (300_007, 150_001),
+                                   (700_001, 5_000)])
+def test_two_streams_share_the_scratch(gpu_lib, sizes):
+    """Sorts on two non-blocking streams, queued without waiting: each waits on the GPU for the one
+    before it, although a small sort's launch may be set up early."""
+    rng = np.random.default_rng(sizes[0])
+    streams = [torch.cuda.Stream() for _ in sizes]
+    keys = [rng.integers(0, 1 << 24, size=n, dtype=np.int64).astype(np.uint32) for n in sizes]
+    first = [torch.from_numpy(k.view(np.int32)).cuda() for k in keys]
+    rounds = [[(a.clone(), torch.arange(len(a), dtype=torch.int32, device="cuda")) for a in first] for _ in range(12)]
+    big = max(range(2), key=lambda i: sizes[i])
+    k0, v0 = first[big].clone(), torch.arange(sizes[big], dtype=torch.int32, device="cuda")
+    capi.sort_pairs_device(k0.data_ptr(), v0.data_ptr(), sizes[big], 24)   # the scratch
+    torch.cuda.synchronize()
+    for pairs in rounds:
+        for (dk, dv), s in zip(pairs, streams):
+            capi.sort_pairs_device(dk.data_ptr(), dv.data_ptr(), len(dk), 24, s.cuda_stream)
+    torch.cuda.synchronize()
+    for pairs in rounds:
+        for (dk, dv), k in zip(pairs, keys):
+            order = np.argsort(k, kind="stable")
+            assert np.array_equal(dv.cpu().numpy(), order.astype(np.int32))
+            assert np.array_equal(dk.cpu().numpy().view(np.uint32), k[order])
