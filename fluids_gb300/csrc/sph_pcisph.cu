@@ -91,7 +91,7 @@ __device__ __forceinline__ void pci_integrate_one(const Const& c, const Bufs& b,
 }
 
 /* update_pressure for one particle: predicted density from the fixed lists at x*.  The
- * list is walked two entries deep with the next two entries loaded during the current two
+ * list is walked SPH_PCI_WALK_DEPTH entries deep, with the next ones' indices loaded during their
  * visits (the sum keeps list order).  x* is written by this kernel, so it is read with plain loads.
  * The updated pressure's p / rho^2 (the initial density, as compute_pressure_force uses it)
  * goes to pci_pc, beside the position, for the force phase: the same IEEE quotient the force

@@ -293,9 +293,10 @@ __device__ __forceinline__ void cluster_barrier() {
  * cooperative or (CLUSTER) one cluster, a tile per CTA: for a small sort the launches of the
  * memset, the histogram and the passes are its time.  Measured on GB300, cooperative, against
  * those launches (24-bit keys, us): 2,387 pairs 20 / 41, 40,000 32 / 45, 150,000 38 / 49, 300,000
- * 44 / 52, 500,000 56 / 59, 600,000 (32-bit keys) 76 / 75.  Per pass each CTA ranks its tile, publishes its digit counts, and after a barrier of all CTAs adds the
- * counts of the tiles before it (and of all tiles, for the buckets), which it reads row by
- * row, so there is no separate histogram and no look-back; a second barrier ends the pass. */
+ * 44 / 52, 500,000 56 / 59, 600,000 (32-bit keys) 76 / 75.  Per pass each CTA ranks its tile,
+ * publishes its digit counts, and after a barrier of all CTAs adds the counts of the tiles before it
+ * (and of all tiles, for the buckets), which it reads row by row, so there is no separate histogram
+ * and no look-back; a second barrier ends the pass. */
 constexpr int kOneThreads = 512;
 constexpr int kOneWarps = kOneThreads / 32;
 constexpr int kOneTile = kOneThreads * 4;
