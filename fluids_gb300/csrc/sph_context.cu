@@ -287,6 +287,7 @@ void carve(sph_ctx* x, Carver& cv) {
     }
     /* scene tiles: at most one per 32 particles of a scene plus one per scene */
     b.tiles = cv.take<sph::SceneTile>(x->scene_in.empty() ? 1 : n / sph::kTileParticles + x->scene_in.size() + 1);
+    b.tile_next = cv.take<unsigned>(1);
 }
 
 /* The scene tile table of a batched context: each scene's particle range cut into tiles of
@@ -295,6 +296,7 @@ void carve(sph_ctx* x, Carver& cv) {
 int upload_tiles(sph_ctx* x) {
     x->c.ntiles = 0;
     x->c.tile_blocks = 0;
+    x->c.tile_next = nullptr;
     if (x->scene_in.empty() || x->N <= 0 || !x->b.tiles) return SPH_OK;
     x->h_tiles.clear();
     for (size_t sc = 0; sc < x->scene_in.size(); ++sc) {
@@ -305,9 +307,10 @@ int upload_tiles(sph_ctx* x) {
     }
     if (x->h_tiles.empty()) return SPH_OK;
     x->c.ntiles = (int)x->h_tiles.size();
-    const long long warps_needed = (x->c.ntiles + x->bs / 32 - 1) / (x->bs / 32);
+    const long long blocks_needed = (x->c.ntiles + x->bs / 32 - 1) / (x->bs / 32);
     const long long set = (long long)x->num_sms * x->tile_ctas;
-    x->c.tile_blocks = (int)(0 < set && set < warps_needed ? set : warps_needed);
+    x->c.tile_blocks = (int)(0 < set && set < blocks_needed ? set : blocks_needed);
+    x->c.tile_next = x->c.tile_blocks < blocks_needed ? x->b.tile_next : nullptr;
     SPH_CUDA(x, cudaStreamSynchronize(x->stream));
     SPH_CUDA(x, cudaMemcpy(const_cast<sph::SceneTile*>(x->b.tiles), x->h_tiles.data(),
                            sizeof(sph::SceneTile) * x->h_tiles.size(), cudaMemcpyHostToDevice));

@@ -41,6 +41,7 @@ struct Const {
     int monaghan;        /* COMPAT with the Monaghan kernels (sph_params::kernels) */
     int ntiles;          /* batched: entries of the scene tile table (SceneTile) */
     int tile_blocks;     /* batched: CTAs of a launch over the tiles */
+    unsigned* tile_next; /* batched: the counter that these CTAs take more tiles from; null: a warp per tile */
     int block0, blocks;  /* single-scene passes launched in parts: blocks [block0, block0 + blocks)
                             of the whole pass (0, 0: the whole pass in one launch) */
     int first, last;     /* the particles [first, last) of a launch with several lanes a particle */
@@ -94,11 +95,13 @@ struct SceneTile {
  * scene tile per warp (its particles one per lane; the lanes beyond its count are idle, so f
  * must not use warp-collective operations), with the grid constants of the tile's scene; f
  * takes the other constants of the scene by late_scene where it needs them, so that they are
- * not held in registers along its neighbour walk.  The grid is one warp per tile, or the
- * CTAs per SM that the caller set, which then stride over the tiles.  Measured on GB300 (40
- * scenes, 662,935 particles; one CTA chunk of tiles at a time from a counter before): list
- * pass 200 -> 186 us, forces 116 -> 108, normals 54 -> 51, a step 457 -> 420, also through
- * the three memsets of the counters. */
+ * not held in registers along its neighbour walk.  The grid is one warp per tile: measured on
+ * GB300 (40 scenes, 662,935 particles; one CTA chunk of tiles at a time from a counter before),
+ * list pass 200 -> 186 us, forces 116 -> 108, normals 54 -> 51, a step 457 -> 420.  With the CTAs
+ * per SM that the caller set, a CTA takes its first tiles by its index and further ones, a tile
+ * per warp, from a counter, which its last taker clears: strided over the tiles instead, the warps
+ * of an SM drift apart and the CTAs end unevenly (256 scenes, 4.9 million particles, 256 threads x
+ * 8: 2217 us a step with a counter before, 2603 strided, 2113 so; x 1: 7816, 9127, 7917). */
 /* W > 1: W adjacent threads per particle, all of them running f to its end (it sums over
  * them); threads past the last particle run it for the last one, which f tells by
  * lane_of_particle.  The scene is the particle's by scene_of, and f, which walks the lists
@@ -113,15 +116,30 @@ __device__ __forceinline__ void for_each_particle(const Const& c0, const SceneTi
         f(c0, 0LL, q, BATCH && scene_of ? scenes + __ldg(&scene_of[q]) : scenes);
     } else if constexpr (BATCH) {
         const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+        int chunk = blockIdx.x;
 #pragma unroll 1
-        for (int t = blockIdx.x * warps + (threadIdx.x >> 5); t < c0.ntiles; t += gridDim.x * warps) {
-            const SceneTile tl = tiles[t];
-            if (lane < tl.count) {
-                Const c = c0;
-                const SceneDev& sd = scenes[tl.scene];
-                apply_scene_grid(c, sd);
-                f(c, sd.cell_base, tl.first + lane, &sd);
+        for (;;) {
+            const int t = chunk * warps + (threadIdx.x >> 5);
+            if (t < c0.ntiles) {
+                const SceneTile tl = tiles[t];
+                if (lane < tl.count) {
+                    Const c = c0;
+                    const SceneDev& sd = scenes[tl.scene];
+                    apply_scene_grid(c, sd);
+                    f(c, sd.cell_base, tl.first + lane, &sd);
+                }
             }
+            if (c0.tile_next == nullptr) break;
+            __shared__ int s_chunk;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const int chunks = (c0.ntiles + warps - 1) / warps, k = (int)atomicAdd(c0.tile_next, 1u);
+                if (k == chunks - 1) *c0.tile_next = 0u;   /* the launch's last one */
+                s_chunk = (int)gridDim.x + k;
+            }
+            __syncthreads();
+            chunk = s_chunk;
+            if (chunk * warps >= c0.ntiles) break;
         }
     } else {
         const int i = (c0.block0 + (int)blockIdx.x) * (int)blockDim.x + (int)threadIdx.x;

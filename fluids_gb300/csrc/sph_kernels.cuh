@@ -57,6 +57,7 @@ struct Bufs {
     const SceneDev* scenes;
     const int32_t* scene_of;
     const SceneTile* tiles;                /* batched: per-scene tiles of 32 particles (Const::ntiles) */
+    unsigned* tile_next;                   /* batched: the tile counter (Const::tile_next), zero between launches */
     /* status */
     unsigned* flags;
     int32_t* pci_iters;

@@ -527,6 +527,13 @@ static inline int grid_for(const Const& c, int bs) {
     return c.blocks > 0 ? c.blocks : nblk(c.n, bs);
 }
 
+/* A pass over the particles or, batched, the tiles: the few CTAs of a set tile shape are not launched
+ * early, which would leave two on one SM. */
+template <bool BATCH, class K, class... A>
+static void launch_pass(cudaStream_t s, K kernel, int grid, int bs, A&&... args) {
+    launch_early(!BATCH && grid <= kEarlyBlocks, s, kernel, grid, bs, 0, std::forward<A>(args)...);
+}
+
 template <bool LIST, bool EXACT>
 static Neigh<LIST, EXACT> fluid_src(const Bufs& b) {
     return Neigh<LIST, EXACT>{b.tab, b.nlist, b.nlen, b.pos_s};
@@ -565,7 +572,7 @@ void launch_wc_density(cudaStream_t s, const Const& c, const Bufs& b, bool lists
 
 template <bool COMPAT, bool BATCH>
 static void lists_density_launch(cudaStream_t s, const Const& c, const Bufs& b, int bs) {
-    launch_chained(s, k_lists_density<COMPAT, BATCH>, grid_for<BATCH>(c, bs), bs, 0, c, b.pos_s, b.tab, b.bpos_s,
+    launch_pass<BATCH>(s, k_lists_density<COMPAT, BATCH>, grid_for<BATCH>(c, bs), bs, c, b.pos_s, b.tab, b.bpos_s,
                    b.btab, b.bphi_s, b.nlist, b.nlen, b.sblist, b.sblen, b.density, b.pressure, b.aux, b.scenes,
                    b.tiles, nullptr, nullptr, b.bnear, b.noff, b.prho, nullptr, nullptr);
 }
@@ -720,11 +727,11 @@ static void forces_launch(cudaStream_t s, const Const& c, const Bufs& b, bool fu
     }
     if constexpr (LIST) {
         if (pack && st && fuse && !write_acc) {
-            launch_chained(s, k_wc_forces<COMPAT, LIST, true, false, true, BATCH, true>, g, bs, 0, c, fs, bsrc, b);
+            launch_pass<BATCH>(s, k_wc_forces<COMPAT, LIST, true, false, true, BATCH, true>, g, bs, c, fs, bsrc, b);
             return;
         }
     }
-#define SPH_WCF(F, W, S) launch_chained(s, k_wc_forces<COMPAT, LIST, F, W, S, BATCH>, g, bs, 0, c, fs, bsrc, b)
+#define SPH_WCF(F, W, S) launch_pass<BATCH>(s, k_wc_forces<COMPAT, LIST, F, W, S, BATCH>, g, bs, c, fs, bsrc, b)
     if (fuse) {
         if (write_acc) { if (st) SPH_WCF(true, true, true); else SPH_WCF(true, true, false); }
         else { if (st) SPH_WCF(true, false, true); else SPH_WCF(true, false, false); }

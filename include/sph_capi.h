@@ -309,8 +309,8 @@ int sph_set_block_size(sph_ctx* ctx, int block_size);
  * launches over per-scene tiles -- each scene's particle range cut into tiles of 32
  * particles, a tile never straddling two scenes -- with one tile per warp, which reads the
  * scene's constants once.  The shape of the grid is block_size threads (sph_set_block_size)
- * times SMs x ctas_per_sm CTAs, whose warps stride over the tiles (0 = as many CTAs as give
- * every tile its warp).  With S SMs, that is the list pass above 768 S particles in the batch
+ * times SMs x ctas_per_sm CTAs, which take their tiles from a counter (0 = as many CTAs as
+ * give every tile its warp).  With S SMs, that is the list pass above 768 S particles in the batch
  * (512 S without boundary particles) and the others above 512 S (116,736 and 77,824 on 152 SMs);
  * smaller batches take several lanes a particle in blocks of their own, whatever the shape.
  * The shape never changes results; fluids_gb300/autotune.py picks it.
