@@ -527,11 +527,12 @@ static inline int grid_for(const Const& c, int bs) {
     return c.blocks > 0 ? c.blocks : nblk(c.n, bs);
 }
 
-/* A pass over the particles or, batched, the tiles: the few CTAs of a set tile shape are not launched
- * early, which would leave two on one SM. */
+/* A pass over the particles or, batched, the tiles.  Not launched early: the few CTAs of a set tile
+ * shape, which would leave two on one SM, and the parts of a divided pass (Const::blocks), which
+ * would start on the SMs that the part before leaves first. */
 template <bool BATCH, class K, class... A>
-static void launch_pass(cudaStream_t s, K kernel, int grid, int bs, A&&... args) {
-    launch_early(!BATCH && grid <= kEarlyBlocks, s, kernel, grid, bs, 0, std::forward<A>(args)...);
+static void launch_pass(cudaStream_t s, K kernel, int grid, int bs, const Const& c, A&&... args) {
+    launch_early(!BATCH && c.blocks == 0 && grid <= kEarlyBlocks, s, kernel, grid, bs, 0, c, std::forward<A>(args)...);
 }
 
 template <bool LIST, bool EXACT>
