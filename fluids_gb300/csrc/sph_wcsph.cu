@@ -390,7 +390,14 @@ __global__ void __launch_bounds__(256, SPH_FORCES_MIN_BLOCKS)
         /* loaded ahead of the guard so that the list loop can issue them early */
         float4 aj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
         if constexpr (PACK) {
-            load_pair(&b.nrec[2 * (size_t)j], vj, nj);
+            if constexpr (COMPAT) {
+                /* most pairs of the kernel text's densities are refused: loads that can wait for
+                 * the guard (1,000,000 particles 125 us, 143 by load_pair) */
+                vj = __ldg(&b.nrec[2 * (size_t)j]);
+                nj = __ldg(&b.nrec[2 * (size_t)j + 1]);
+            } else {
+                load_pair(&b.nrec[2 * (size_t)j], vj, nj);
+            }
             aj = make_float4(vj.w, nj.w, 1.0f, 0.f);   /* (C_j, R_j, -, -); the guard uses R_j > 0 */
         } else {
             aj = __ldg(&b.aux[j]);
