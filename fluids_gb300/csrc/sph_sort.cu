@@ -470,8 +470,11 @@ void sort_launches(cudaStream_t s, const SortBufs& b, int n, int passes, uint32_
     }
 }
 
+/* k_sort_one's grid barrier in a sort's workspace (behind the histogram, among the counters). */
+static unsigned* sort_barrier(void* ws) { return static_cast<unsigned*>(ws) + 4 * 256 + 32; }
+
 /* The sort of (b.kin, b.vin) by passes whose outputs b names.  ws: sort_workspace_bytes, of any
- * content.  gate: null, or a flag word an earlier kernel of the stream wrote;
+ * content, gated with its sort_barrier at zero.  gate: null, or a flag word an earlier kernel of the stream wrote;
  * every kernel of the sort leaves at once while it is 0. */
 void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned* gate, int key_bits, void* ws,
                        unsigned* flags, int num_sms) {
@@ -483,7 +486,7 @@ void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned*
     const int one = n <= kOneSolo ? 1 : (n + kOneTile - 1) / kOneTile;
     if (one <= kOneTiles && one <= 2 * num_sms) {
         SortBufs bb = b;
-        unsigned* bar = counters + 32;
+        unsigned* bar = sort_barrier(ws);
         uint32_t* counts = status;
         int nn = n, np = passes;
         void* args[] = {&bb, &nn, &np, &counts, &bar, &flags, &gate};
@@ -497,8 +500,9 @@ void sort_pairs_passes(cudaStream_t s, const SortBufs& b, int n, const unsigned*
         }
         void* fn = n <= kOneSolo ? (void*)k_sort_one<8> : (void*)k_sort_one<4>;
         /* a barrier whose wait ran out leaves arrivals behind, and the next launch's barriers
-         * would open too early: its words start at zero in each launch */
-        cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s);
+         * would open too early: its words start at zero in each launch (gated: cleared by
+         * k_inc_place, as a memset between it and the sort cost 3 to 5 us a step) */
+        if (!gate) cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s);
         if (cudaLaunchCooperativeKernel(fn, dim3(one), dim3(kOneThreads), args, 0, s) == cudaSuccess) return;
         cudaGetLastError();   /* then by several launches */
     }
@@ -676,11 +680,13 @@ __global__ void __launch_bounds__(kThreads) k_inc_place(const int2* __restrict__
                                                         uint32_t* __restrict__ bcnt, int4* __restrict__ store,
                                                         unsigned* __restrict__ over, unsigned* __restrict__ done,
                                                         const uint32_t* __restrict__ tcnt,
-                                                        uint32_t* __restrict__ tpre, uint32_t* __restrict__ boff) {
+                                                        uint32_t* __restrict__ tpre, uint32_t* __restrict__ boff,
+                                                        unsigned* __restrict__ bar) {
     extern __shared__ uint32_t s_first[];   /* min(tiles, kIncSmemTiles) entries */
     __shared__ uint32_t s_scan[kWarps];
     __shared__ bool s_last;
     chain_next();
+    if (blockIdx.x == 0 && threadIdx.x < 2) bar[threadIdx.x] = 0u;   /* the gated sort's grid barrier */
     if (*valid == 0u) return;   /* no previous result: the full sort runs */
     const int m = (int)*lcount;
     if (m > n / 6) {
@@ -975,7 +981,7 @@ void sort_pairs_incremental(cudaStream_t s, const uint32_t* keys, int n, int key
     /* at most a sixth of the particles is placed, a thread each */
     const int pblocks = max(1, min(4 * num_sms, (n / 6 + kThreads - 1) / kThreads));
     launch_chained(s, k_inc_place, pblocks, kThreads, fsm, list, lcount, prev, first, sub, n, L.tiles, valid, bcnt,
-                   store, over, done, tcnt, tpre, boff);
+                   store, over, done, tcnt, tpre, boff, sort_barrier(sort_ws));
     /* the gated full sort of (keys, identity) on the side stream, beside the merge (one of
      * the two writes the result); prev is its scratch and its last pass writes kout / vout */
     const bool fork_side = side != nullptr && fork != nullptr && join != nullptr;

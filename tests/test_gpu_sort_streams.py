@@ -132,6 +132,38 @@ def test_barrier_words_left_by_a_timed_out_sort(gpu_lib, n):
     assert np.array_equal(got.cpu().numpy(), np.argsort(keys, kind="stable").astype(np.int32))
 
 
+@pytest.mark.parametrize("n", [32_769, 200_001, 524_288])
+def test_barrier_words_left_before_a_gated_sort(gpu_lib, n):
+    """The same for the full sort that the step's sort opens when it has no previous order
+    (sph::sort_pairs_incremental), and then its update of that order."""
+    lib = capi.lib()
+    f = getattr(lib, "_ZN3sph22sort_pairs_incrementalEP11CUstream_stPKjiiPjPiPvS6_S4_iS1_P10CUevent_stS8_b")
+    f.restype = None
+    size = getattr(lib, "_ZN3sph24sort_inc_workspace_bytesEi")
+    size.restype = C.c_size_t
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 1 << 21, size=n, dtype=np.int64).astype(np.uint32)
+    inc = torch.zeros(size(C.c_int(n)), dtype=torch.uint8, device="cuda")
+    ws = torch.full((4 * 256 + 64 + 1024 * 256,), 37, dtype=torch.int32, device="cuda")
+    flags = torch.zeros(4, dtype=torch.int32, device="cuda")
+    ko, vo = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for k in range(3):   # no previous order; a few keys moved; most of them moved, so a full sort again
+        moved = rng.uniform(size=n) < (0.0, 0.01, 0.9)[k]
+        keys = np.where(moved, rng.integers(0, 1 << 21, size=n), keys).astype(np.uint32)
+        dk = torch.from_numpy(keys.view(np.int32)).cuda()
+        ws[4 * 256 + 32:4 * 256 + 34] = 37
+        torch.cuda.synchronize()
+        f(C.c_void_p(0), C.c_void_p(dk.data_ptr()), C.c_int(n), C.c_int(21), C.c_void_p(ko.data_ptr()),
+          C.c_void_p(vo.data_ptr()), C.c_void_p(inc.data_ptr()), C.c_void_p(ws.data_ptr()), C.c_void_p(flags.data_ptr()),
+          C.c_int(sms), C.c_void_p(0), C.c_void_p(0), C.c_void_p(0), C.c_bool(False))
+        torch.cuda.synchronize()
+        order = np.argsort(keys, kind="stable")
+        assert flags[0].item() == 0
+        assert np.array_equal(vo.cpu().numpy(), order.astype(np.int32)), k
+        keys = keys[order]   # the step hands the next call its particles in this order
+
+
 @pytest.mark.parametrize("sizes", [(3_000, 4_000), (30_000, 20_001), (65_536, 40_000), (300_007, 150_001),
                                    (700_001, 5_000)])
 def test_two_streams_share_the_scratch(gpu_lib, sizes):
