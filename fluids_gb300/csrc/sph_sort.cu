@@ -68,15 +68,13 @@ __device__ __forceinline__ unsigned same_digit(uint32_t d) {
     }
     return peers;
 }
-/* same_digit for a warp whose digits may be few (nearly sorted keys of any caller): by match_any
- * where an earlier round of the warp's keys, told by `few`, held at most kFewDigits of them.
- * Measured on GB300 (us; ballots alone, then with the choice at 4, 8 and 12 digits): 4,194,304 nearly
- * sorted pairs of 16 bits 115, 99, 96, 96; of seven keys 112, 112, 94, 94; random ones 139 in all. */
+/* Keys of a caller may be nearly sorted too: a warp looks at its first round of them by ballots, and
+ * matches the others by match_any when it held at most kFewDigits digits.  Measured on GB300 (us;
+ * ballots alone, then with the choice at 4, 8 and 12 digits): 4,194,304 nearly sorted pairs of 16
+ * bits 115, 99, 96, 96; of seven keys 112, 112, 94, 94; random ones 139 in all.  Taken for the rest
+ * of the keys at once, not key by key: 1,062,234 random pairs of 24 bits 80.6 without the choice, 82.5
+ * key by key, 81.4 so, and 4,194,304 nearly sorted ones of 16 bits 90 and 84. */
 constexpr int kFewDigits = 8;
-template <bool FEW>
-__device__ __forceinline__ unsigned same_digit(uint32_t d, bool few) {
-    return FEW || few ? __match_any_sync(0xffffffffu, d) : same_digit<false>(d);
-}
 /* Whether the warp's round with these peers had few digits. */
 __device__ __forceinline__ bool few_digits(unsigned peers, unsigned lt_mask) {
     return __popc(__ballot_sync(0xffffffffu, (peers & lt_mask) == 0u)) <= kFewDigits;
@@ -131,17 +129,30 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
             const long long i = base + (long long)u * kThreads + threadIdx.x;
             k[u] = i < n ? __ldg(&keys[i]) : 0u;
         }
-        unsigned few = 0u;   /* the passes of few digits */
+        unsigned active[kHistItems];
 #pragma unroll
-        for (int u = 0; u < kHistItems; ++u) {
-            const long long i = base + (long long)u * kThreads + threadIdx.x;
-            const bool valid = i < n;
-            const unsigned active = __ballot_sync(0xffffffffu, valid);
-            for (int p = 0; p < passes; ++p) {
-                const uint32_t d = (k[u] >> (8 * p)) & 255u;
-                const unsigned all = same_digit<FEW>(d, (few >> p) & 1u), peers = all & active;
-                if (!FEW && u == 0 && few_digits(all, lt_mask)) few |= 1u << p;
-                if (valid && lane == __ffs(peers) - 1) atomicAdd(&s_hist[p][d], (uint32_t)__popc(peers));
+        for (int u = 0; u < kHistItems; ++u)
+            active[u] = __ballot_sync(0xffffffffu, base + (long long)u * kThreads + threadIdx.x < n);
+        for (int p = 0; p < passes; ++p) {
+            auto add = [&](int u, uint32_t d, unsigned peers) {
+                peers &= active[u];
+                if (((active[u] >> lane) & 1u) && (peers & lt_mask) == 0u) atomicAdd(&s_hist[p][d], (uint32_t)__popc(peers));
+            };
+            const uint32_t d0 = (k[0] >> (8 * p)) & 255u;
+            const unsigned p0 = same_digit<FEW>(d0);
+            add(0, d0, p0);
+            if (FEW || few_digits(p0, lt_mask)) {
+#pragma unroll
+                for (int u = 1; u < kHistItems; ++u) {
+                    const uint32_t d = (k[u] >> (8 * p)) & 255u;
+                    add(u, d, same_digit<true>(d));
+                }
+            } else {
+#pragma unroll
+                for (int u = 1; u < kHistItems; ++u) {
+                    const uint32_t d = (k[u] >> (8 * p)) & 255u;
+                    add(u, d, same_digit<false>(d));
+                }
             }
         }
     }
@@ -154,8 +165,8 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist(const uint32_t* __restri
 
 /* Three blocks an SM (80 registers, no spills): the look-back's words in flight took it to 128
  * registers and two blocks, and sorts of 16,000,000 nearly sorted pairs (16 bits) from 284 us to
- * 304 against 265 now; 1,062,234 random pairs (32 bits) 104 us either way.  Four blocks gain another
- * 5 % there and lose 3 to 8 % below 1,500,000 pairs. */
+ * 347; 244 now, with the choice of the digit match.  Four blocks gain another 5 % there and lose 3
+ * to 8 % below 1,500,000 pairs. */
 template <bool FEW>
 __global__ void __launch_bounds__(kThreads, 3) k_onesweep(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
                                                        uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int n,
@@ -195,17 +206,29 @@ __global__ void __launch_bounds__(kThreads, 3) k_onesweep(const uint32_t* __rest
         key[k] = valid ? __ldg(&kin[idx]) : 0xffffffffu;   /* tail keys sort last and are not written */
         val[k] = valid ? (vin ? __ldg(&vin[idx]) : (int32_t)idx) : 0;   /* no vin: the identity */
     }
-    bool few = false;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint32_t d = (key[k] >> shift) & 255u;
-        const unsigned peers = same_digit<FEW>(d, few);
-        if (!FEW && k == 0) few = few_digits(peers, lt_mask);
+    auto rank_one = [&](int k, uint32_t d, unsigned peers) {
         const uint32_t before = s_whist[warp][d];
         __syncwarp();
         if ((peers & lt_mask) == 0u) s_whist[warp][d] = before + (uint32_t)__popc(peers);
         __syncwarp();
         rank[k] = before + (uint32_t)__popc(peers & lt_mask);
+    };
+    const uint32_t d0 = (key[0] >> shift) & 255u;
+    const unsigned p0 = same_digit<FEW>(d0);
+    const bool few = FEW || few_digits(p0, lt_mask);
+    rank_one(0, d0, p0);
+    if (few) {
+#pragma unroll
+        for (int k = 1; k < kItems; ++k) {
+            const uint32_t d = (key[k] >> shift) & 255u;
+            rank_one(k, d, same_digit<true>(d));
+        }
+    } else {
+#pragma unroll
+        for (int k = 1; k < kItems; ++k) {
+            const uint32_t d = (key[k] >> shift) & 255u;
+            rank_one(k, d, same_digit<false>(d));
+        }
     }
     __syncthreads();
 
